@@ -72,8 +72,9 @@ struct TileCursor {
   }
 };
 
-// One thread's N logits of a tile (bit i of mword is the label of logit i): dS = sigmoid(s) - label packed as bf16 pairs (low half = even column) and, with
-// LOSS, the BCE-with-logits terms added to lacc.  FULL: all N columns are valid entries of Y.
+// One thread's 32 logits of a tile (bit i of mword is the label of logit i): dS = sigmoid(s) - label packed as bf16 pairs
+// (low half = even column) and, with LOSS, the BCE-with-logits terms added to lacc.  FULL: all columns are valid entries
+// of Y; otherwise the first y_valid are.
 // SCORE selects how the logit follows from the dot product a = x.y of the tensor cores:
 //   0  s = a
 //   1  s = a + xb + yb[col]                     (per-query scalar terms of the Clifford models)
@@ -82,62 +83,101 @@ struct TileCursor {
 //      d s / d x = (y - x) / distance.
 // dsum accumulates the values handed to the second GEMM (SCORE != 0 only).
 //
-// The epilogue is bound by instruction issue (sixteen warps share four schedulers), so everything is derived from one
-// hyperbolic tangent of the non-positive half argument, t = tanh(-|s| / 2) in (-1, 0]:
-//   sigmoid(|s|) = u = 0.5 - 0.5 t  in [0.5, 1)        (no cancellation)
-//   tanh(s / 2)  = t with its sign flipped where s >= 0 (one logic op on the sign bits)
-//   dS = sigmoid(s) - label = 0.5 tanh(s / 2) + c      with c = 0.5 - label (one of two constants, picked by the mask)
-//   BCE(s, label) = softplus(s) - label s = c s + 0.5 |s| - ln 2 * lg2(u)
-// and the three sums  sum c s,  sum |s|,  sum lg2(u)  are kept apart (lacc[0..2]) and combined once per segment.  The
-// last one is the logarithm of a product: the N <= 32 factors u of a chunk (each in [0.5, 1), so the product stays above
-// 2^-32) are multiplied up and ONE logarithm is taken per chunk.  That leaves one special-function operation (the
-// tanh) and about ten other instructions per logit; the special-function unit (16 results per clock and SM) would
-// otherwise need as many cycles per tile as the two GEMMs do.
-template <int N, bool LOSS, bool MASK, bool FULL, int SCORE>
-__device__ __forceinline__ void epilogue_chunk(const uint32_t (&r)[N], uint32_t mword, float base, float label_pos,
-                                               int y_valid, uint32_t (&packed)[N / 2], float (&lacc)[3], float xb,
+// Everything is derived from one hyperbolic tangent per logit, t = tanh(s / 2):
+//   dS = sigmoid(s) - label = 0.5 t + c              with c = 0.5 - label (one of two constants)
+//   sigmoid(|s|) = 0.5 (1 + |t|)  in [0.5, 1)        (no cancellation)
+//   BCE(s, label) = softplus(s) - label s = c s + 0.5 |s| - ln 2 * (lg2(1 + |t|) - 1)
+// and the three sums  sum c s,  sum |s|,  sum lg2(sigmoid(|s|))  are kept apart (lacc[0..2]) and combined once per segment.
+// The last one is the logarithm of a product: the 32 factors 1 + |t| (each in [1, 2), so the product stays below 2^32)
+// are multiplied up and ONE logarithm is taken per call.
+//
+// The epilogue is bound by instruction issue (all its warps share four schedulers), so it works on pairs of logits with
+// the packed fp32 operations (two results per issued instruction), and the label of a logit costs nothing where no lane
+// of the warp has a positive among its 32 columns: positives are a few per thousand logits, so most warps take that
+// path (`any` is uniform in the warp).  5.5 issued instructions per logit with the loss and 2.5 without, against 15 and 8
+// of the scalar form with a select per logit; one of them is the special-function tanh (16 results per clock and SM).
+template <bool LOSS, bool LABELS, bool FULL, int SCORE>
+__device__ __forceinline__ void epilogue_pairs(const uint32_t (&r)[32], uint32_t mword, float c_base, float delta,
+                                               int y_valid, uint32_t (&packed)[16], float (&lacc)[3], float xb,
                                                const float* __restrict__ yb, float margin, float& dsum) {
-  const float c_base = 0.5f - base, c_pos = 0.5f - label_pos;
-  float uprod = 1.f;
+  const uint64_t half2 = pack2(0.5f, 0.5f), c2 = pack2(c_base, c_base), zero2 = pack2(0.f, 0.f);
+  uint64_t s_sum = zero2, prod = pack2(1.f, 1.f), d_sum = zero2;
+  float abs0 = 0.f, abs1 = 0.f, pos_sum = 0.f;
 #pragma unroll
-  for (int i = 0; i < N; i += 2) {
-    float ds2[2];
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      float s = __uint_as_float(r[i + u]);
-      float gscale = 1.f;
-      if constexpr (SCORE == 1) s += xb + yb[i + u];
-      if constexpr (SCORE == 2) {
-        const float d2 = fmaxf(fmaf(-2.f, s, xb + yb[i + u]), 1e-12f);
-        gscale = rsqrtf(d2);
-        s = fmaf(-d2, gscale, margin);
-      }
-      float c = c_base;
-      if constexpr (MASK) c = ((mword >> (i + u)) & 1u) ? c_pos : c_base;
-      const bool valid = FULL || (i + u < y_valid);
-      float th;  // tanh(s / 2)
-      if constexpr (LOSS) {
-        const float tn = fast_tanh(-0.5f * fabsf(s));
-        th = __uint_as_float(__float_as_uint(tn) ^ (~__float_as_uint(s) & 0x80000000u));
-        const float us = fmaf(-0.5f, tn, 0.5f);   // sigmoid(|s|)
-        if (valid) {
-          lacc[0] = fmaf(c, s, lacc[0]);
-          lacc[1] += fabsf(s);
-          uprod *= us;
-        }
-      } else {
-        th = fast_tanh(0.5f * s);
-      }
-      float d = fmaf(0.5f, th, c);
-      if constexpr (SCORE == 2) d *= gscale;
-      if (!valid) d = 0.f;
-      if constexpr (SCORE != 0) dsum += d;
-      ds2[u] = d;
+  for (int i = 0; i < 32; i += 2) {
+    float s0 = __uint_as_float(r[i]), s1 = __uint_as_float(r[i + 1]);
+    float g0 = 1.f, g1 = 1.f;
+    if constexpr (SCORE == 1) { s0 += xb + yb[i]; s1 += xb + yb[i + 1]; }
+    if constexpr (SCORE == 2) {
+      const float a0 = fmaxf(fmaf(-2.f, s0, xb + yb[i]), 1e-12f), a1 = fmaxf(fmaf(-2.f, s1, xb + yb[i + 1]), 1e-12f);
+      g0 = rsqrtf(a0);
+      g1 = rsqrtf(a1);
+      s0 = fmaf(-a0, g0, margin);
+      s1 = fmaf(-a1, g1, margin);
     }
-    __nv_bfloat162 v = __floats2bfloat162_rn(ds2[0], ds2[1]);  // .x (low 16 bits) = even K element
+    if constexpr (!FULL) {   // a padded column counts as s = 0: t = 0, a factor of one, nothing added to the sums
+      s0 = i < y_valid ? s0 : 0.f;
+      s1 = i + 1 < y_valid ? s1 : 0.f;
+    }
+    const uint64_t s2 = pack2(s0, s1);
+    float h0, h1;
+    unpack2(mul2(s2, half2), h0, h1);
+    const float t0 = fast_tanh(h0), t1 = fast_tanh(h1);
+    uint64_t d2 = fma2(pack2(t0, t1), half2, c2);
+    if constexpr (LOSS) {
+      s_sum = add2(s_sum, s2);
+      abs0 += fabsf(s0);
+      abs1 += fabsf(s1);
+      prod = mul2(prod, pack2(1.f + fabsf(t0), 1.f + fabsf(t1)));
+    }
+    float d0, d1;
+    unpack2(d2, d0, d1);
+    if constexpr (LABELS) {
+      const bool p0 = (mword >> i) & 1u, p1 = (mword >> (i + 1)) & 1u;
+      if (p0) d0 -= delta;
+      if (p1) d1 -= delta;
+      if constexpr (LOSS) {
+        if (p0) pos_sum += s0;
+        if (p1) pos_sum += s1;
+      }
+    }
+    if constexpr (SCORE == 2) { d0 *= g0; d1 *= g1; }
+    if constexpr (!FULL) {
+      d0 = i < y_valid ? d0 : 0.f;
+      d1 = i + 1 < y_valid ? d1 : 0.f;
+    }
+    if constexpr (SCORE != 0) d_sum = add2(d_sum, pack2(d0, d1));
+    __nv_bfloat162 v = __floats2bfloat162_rn(d0, d1);  // .x (low 16 bits) = even K element
     packed[i >> 1] = *reinterpret_cast<uint32_t*>(&v);
   }
-  if constexpr (LOSS) lacc[2] += fast_lg2(uprod);
+  if constexpr (LOSS) {
+    float a, b;
+    unpack2(s_sum, a, b);
+    lacc[0] = fmaf(c_base, a + b, lacc[0]);
+    if constexpr (LABELS) lacc[0] = fmaf(-delta, pos_sum, lacc[0]);
+    lacc[1] += abs0 + abs1;
+    unpack2(prod, a, b);
+    lacc[2] += fast_lg2(a * b) - (FULL ? 32.f : static_cast<float>(max(0, min(y_valid, 32))));
+  }
+  if constexpr (SCORE != 0) {
+    float a, b;
+    unpack2(d_sum, a, b);
+    dsum += a + b;
+  }
+}
+
+template <bool LOSS, bool MASK, int SCORE>
+__device__ __forceinline__ void epilogue_chunk(const uint32_t (&r)[32], uint32_t mword, float base, float delta,
+                                               int y_valid, uint32_t (&packed)[16], float (&lacc)[3], float xb,
+                                               const float* __restrict__ yb, float margin, float& dsum) {
+  const float c_base = 0.5f - base;
+  const bool any = MASK && __any_sync(0xffffffffu, mword != 0u);
+  if (y_valid >= 32) {
+    if (!any) epilogue_pairs<LOSS, false, true, SCORE>(r, mword, c_base, delta, 32, packed, lacc, xb, yb, margin, dsum);
+    else epilogue_pairs<LOSS, MASK, true, SCORE>(r, mword, c_base, delta, 32, packed, lacc, xb, yb, margin, dsum);
+  } else {
+    epilogue_pairs<LOSS, MASK, false, SCORE>(r, mword, c_base, delta, y_valid, packed, lacc, xb, yb, margin, dsum);
+  }
 }
 
 }  // namespace dice

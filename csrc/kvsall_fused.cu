@@ -264,7 +264,6 @@ kvsall_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     float loss_acc = 0.f;
     uint32_t g = 0, seg = 0;
     bool ok = true;
-    const float label_pos = p.base + p.pos_delta;
 
     for (long long w = w_begin; w < w_end && ok && !*s_abort;) {
       int x, y0, run;
@@ -319,13 +318,8 @@ kvsall_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         tmem_ld32(s_addr, r);
         tc_wait_ld();
         uint32_t packed[16];
-        if (y_valid >= 32) {
-          epilogue_chunk<32, LOSS, MASK, true, SCORE>(r, mword, p.base, label_pos, y_valid, packed, seg_l, xb, yb,
-                                                  p.margin, seg_dsum);
-        } else {
-          epilogue_chunk<32, LOSS, MASK, false, SCORE>(r, mword, p.base, label_pos, y_valid, packed, seg_l, xb, yb,
-                                                   p.margin, seg_dsum);
-        }
+        epilogue_chunk<LOSS, MASK, SCORE>(r, mword, p.base, p.pos_delta, y_valid, packed, seg_l, xb, yb, p.margin,
+                                          seg_dsum);
         tmem_st16(s_addr, packed);
         tc_wait_st();
         tc_fence_before();
