@@ -14,14 +14,13 @@
 // correction (see elementwise.cu), because BCE(s, y) = softplus(s) − y·s splits into a dense label-free term and a
 // term over the known tails only.
 //
-// Structure of a CTA (576 threads, one CTA per SM, persistent over a contiguous range of (x-tile, y-tile) pairs):
+// Structure of a CTA (one CTA per SM, persistent over a contiguous range of (x-tile, y-tile) pairs; tile sizes in Cfg):
 //   warp 0       TMA producer: X tile once per segment, Y tiles through a ring of stages
 //   warp 1       tcgen05.mma issuer (one elected lane); owns the TMEM allocation
-//   warps 2..17  epilogue: tcgen05.ld S → sigmoid / loss → tcgen05.st dS (bf16, packed) → final drain of out
-// TMEM columns: [0, D) out accumulator, [256, 384) and [384, 512) the double-buffered S tiles; dS overwrites
-// columns of the S buffer it was computed from (the warp's own 32 columns, so no other warp's unread data is
-// touched).  Sixteen epilogue warps (four per scheduler) keep the special-function unit busy: with eight the
-// epilogue of the loss variant took 1.7x the time of the two GEMMs of a tile.
+//   warps 2..    epilogue: tcgen05.ld S → sigmoid / loss → tcgen05.st dS (bf16, packed) → final drain of out
+// TMEM columns: [0, D) out accumulator, behind it the S buffers; dS overwrites columns of the S buffer it was computed
+// from (the warp's own 32 columns, so no other warp's unread data is touched).  Three or four epilogue warps per
+// scheduler keep the special-function unit busy.
 // Every mbarrier wait is bounded; on a time-out the kernel records a status code, drains its TMA copies, frees
 // TMEM and returns.
 #include "dice_b200.h"
@@ -37,42 +36,58 @@
 namespace dice {
 
 constexpr int BLOCK_X = 128;
-constexpr int BLOCK_Y = 128;
-constexpr int SLAB_BYTES = 128 * 128;  // 128 rows x 64 bf16 (one 128-byte swizzle span per row)
-constexpr int NUM_EPI_WARPS = 16;   // four per TMEM lane quarter, each owning 32 of a tile's 128 S columns
-constexpr int NUM_THREADS = 64 + 32 * NUM_EPI_WARPS;
 
+// Tile sizes per embedding width.  A Y tile is held from its first GEMM through the epilogue to its second GEMM, and the
+// tensor pipe takes  G1(t), G2(t-1), G1(t+1), G2(t) ...  so three Y stages have to be on chip before the refill of a
+// stage (1100 - 1600 cycles from L2) is off the critical path.  At D = 256 three stages of 128 rows do not fit beside the
+// 64 KB X tile; three of 96 rows do.  The first GEMM is bound by shared-memory reads (128 B per clock: 56 cycles per
+// 128x96x16 step against 64 for 128x128x16), so the narrower tile costs 17 % of that GEMM and saves the wait.
+// For D <= 128 the accumulator leaves room in tensor memory for three S buffers.
 template <int D>
 struct Cfg {
-  static constexpr int NSLAB = D / 64;
-  static constexpr int TILE_BYTES = NSLAB * SLAB_BYTES;
-  static constexpr int NSTAGE = (D == 256) ? 2 : 4;
-  static constexpr int SMEM_BYTES = TILE_BYTES * (1 + NSTAGE) + 1024 /*align*/ + 512 /*barriers*/;
+  static constexpr int NSLAB = D / 64;                 // 64-column slabs (one 128-byte swizzle span per row)
+  static constexpr int BY = (D == 256) ? 96 : 128;     // rows of a Y tile = columns of S
+  static constexpr int NCG = BY / 32;                  // column groups of 32: one per epilogue warp of a lane quarter
+  static constexpr int EPI_WARPS = 4 * NCG;
+  static constexpr int THREADS = 64 + 32 * EPI_WARPS;
+  static constexpr int NBUF = (D == 256) ? 2 : 3;      // S buffers in tensor memory
+  static constexpr int S_COL = (D == 256) ? 256 : 128; // first tensor-memory column of the S buffers
+  static constexpr int NSTAGE = (D == 256) ? 3 : (D == 128) ? 5 : 6;
+  static constexpr int XSLAB = BLOCK_X * 128;
+  static constexpr int YSLAB = BY * 128;
+  static constexpr int X_BYTES = NSLAB * XSLAB;
+  static constexpr int Y_BYTES = NSLAB * YSLAB;
+  static constexpr int SMEM_BYTES = X_BYTES + NSTAGE * Y_BYTES + 1024 /*align*/ + 512 /*barriers*/;
+  static_assert(S_COL + NBUF * BY <= 512 && S_COL >= D, "tensor memory layout");
+  static_assert(SMEM_BYTES <= 227 * 1024, "shared memory layout");
+  static_assert(YSLAB % 1024 == 0, "swizzle atoms are 1024-byte aligned");
 };
 
 template <int D, bool LOSS, bool MASK, int SCORE>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+__global__ void __launch_bounds__(Cfg<D>::THREADS, 1)
 kvsall_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_y,
                     const KvsAllParams p) {
   using C = Cfg<D>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sX = smem;
-  uint8_t* sY = smem + C::TILE_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::TILE_BYTES * (1 + C::NSTAGE));
+  uint8_t* sY = smem + C::X_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::X_BYTES + C::NSTAGE * C::Y_BYTES);
   uint64_t* x_full = bars + 0;
   uint64_t* x_empty = bars + 1;
   uint64_t* dx_full = bars + 2;
   uint64_t* dx_empty = bars + 3;
-  uint64_t* s_full = bars + 4;       // [2]
-  uint64_t* ds_full = bars + 6;      // [2]
-  uint64_t* y_empty = bars + 8;      // [NSTAGE]
-  uint64_t* y_full = bars + 12;      // [NSTAGE][4]: one per 64-column slab, so the S GEMM starts on the first slab
-  uint32_t* tmem_base_smem = reinterpret_cast<uint32_t*>(bars + 28);
-  volatile int* s_abort = reinterpret_cast<volatile int*>(bars + 29);
-  volatile int* s_last = reinterpret_cast<volatile int*>(bars + 30);   // this CTA completed the x tile (fused optimiser)
-  uint64_t* opt_issued = bars + 31;   // all epilogue warps have issued the reductions of a segment
-  uint64_t* opt_decided = bars + 32;  // s_last of the segment is valid
+  uint64_t* opt_issued = bars + 4;    // all epilogue warps have issued the reductions of a segment
+  uint64_t* opt_decided = bars + 5;   // s_last of the segment is valid
+  uint64_t* s_full = bars + 6;        // [NBUF]
+  uint64_t* ds_full = s_full + C::NBUF;      // [NBUF]
+  uint64_t* y_empty = ds_full + C::NBUF;     // [NSTAGE]
+  uint64_t* y_full = y_empty + C::NSTAGE;    // [NSTAGE]
+  uint64_t* words = y_full + C::NSTAGE;
+  uint32_t* tmem_base_smem = reinterpret_cast<uint32_t*>(words);
+  volatile int* s_abort = reinterpret_cast<volatile int*>(words + 1);   // [0] abort flag, [1] always zero
+  volatile int* s_last = reinterpret_cast<volatile int*>(words + 2);    // this CTA completed the x tile (fused optimiser)
+  static_assert(8 * (9 + 2 * C::NBUF + 2 * C::NSTAGE) <= 512, "barrier area");
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -86,18 +101,18 @@ kvsall_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     mbar_init(x_full, 1);
     mbar_init(x_empty, 1);
     mbar_init(dx_full, 1);
-    mbar_init(dx_empty, NUM_EPI_WARPS);
-    for (int i = 0; i < 2; ++i) {
+    mbar_init(dx_empty, C::EPI_WARPS);
+    for (int i = 0; i < C::NBUF; ++i) {
       mbar_init(s_full + i, 1);
-      mbar_init(ds_full + i, NUM_EPI_WARPS);
+      mbar_init(ds_full + i, C::EPI_WARPS);
     }
     for (int i = 0; i < C::NSTAGE; ++i) {
       mbar_init(y_empty + i, 1);
-      for (int sl = 0; sl < C::NSLAB; ++sl) mbar_init(y_full + i * 4 + sl, 1);
+      mbar_init(y_full + i, 1);
     }
-    mbar_init(opt_issued, NUM_EPI_WARPS);
+    mbar_init(opt_issued, C::EPI_WARPS);
     mbar_init(opt_decided, 1);
-    *reinterpret_cast<volatile uint64_t*>(bars + 29) = 0;  // abort flag and an always-zero word next to it
+    *reinterpret_cast<volatile uint64_t*>(words + 1) = 0;  // abort flag and an always-zero word next to it
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -116,7 +131,7 @@ kvsall_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
   griddep_wait();
   griddep_launch();
   const uint32_t tmem_out = tmem_base;              // D columns
-  const uint32_t tmem_s0 = tmem_base + 256;         // two S buffers of 128 columns
+  const uint32_t tmem_s0 = tmem_base + C::S_COL;    // NBUF S buffers of BY columns
 
   auto fail = [&](int code) {
     atomicCAS(p.status, 0, code);
@@ -137,19 +152,18 @@ kvsall_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         p.map.locate(w, x, y0, run);
         const int n = static_cast<int>(min(static_cast<long long>(run), w_end - w));
         if (!mbar_wait_bounded(x_empty, (seg & 1) ^ 1, s_abort)) { fail(ST_TIMEOUT_PRODUCER); break; }
-        mbar_arrive_expect_tx(x_full, C::TILE_BYTES);
-        for (int s = 0; s < C::NSLAB; ++s) tma_load_2d(sX + s * SLAB_BYTES, &tmap_x, s * 64, x * BLOCK_X, x_full);
+        mbar_arrive_expect_tx(x_full, C::X_BYTES);
+        for (int s = 0; s < C::NSLAB; ++s) tma_load_2d(sX + s * C::XSLAB, &tmap_x, s * 64, x * BLOCK_X, x_full);
         ++x_loads;
         bool ok = true;
         for (int t = 0; t < n; ++t, ++ycount) {
           const uint32_t st = ycount % C::NSTAGE;
           if (!mbar_wait_bounded(y_empty + st, ((ycount / C::NSTAGE) & 1) ^ 1, s_abort)) { ok = false; break; }
           stamp(ycount, 0);
-          uint8_t* dst = sY + st * C::TILE_BYTES;
-          for (int s = 0; s < C::NSLAB; ++s) {
-            mbar_arrive_expect_tx(y_full + st * 4 + s, SLAB_BYTES);
-            tma_load_2d(dst + s * SLAB_BYTES, &tmap_y, s * 64, (y0 + t) * BLOCK_Y, y_full + st * 4 + s);
-          }
+          uint8_t* dst = sY + st * C::Y_BYTES;
+          mbar_arrive_expect_tx(y_full + st, C::Y_BYTES);
+          for (int s = 0; s < C::NSLAB; ++s)
+            tma_load_2d(dst + s * C::YSLAB, &tmap_y, s * 64, (y0 + t) * C::BY, y_full + st);
         }
         if (!ok) { fail(ST_TIMEOUT_PRODUCER); break; }
         w += n;
@@ -161,9 +175,7 @@ kvsall_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         if (x_loads > 0) drained &= mbar_wait_bounded(x_full, (x_loads - 1) & 1, s_abort + 1 /*always 0*/, 1u << 20);
         for (uint32_t i = 0; i < C::NSTAGE && i < ycount; ++i) {
           const uint32_t last = ycount - 1 - i;  // the most recent use of each stage
-          for (int sl = 0; sl < C::NSLAB; ++sl)
-            drained &= mbar_wait_bounded(y_full + (last % C::NSTAGE) * 4 + sl, (last / C::NSTAGE) & 1, s_abort + 1,
-                                         1u << 20);
+          drained &= mbar_wait_bounded(y_full + last % C::NSTAGE, (last / C::NSTAGE) & 1, s_abort + 1, 1u << 20);
         }
         if (!drained) atomicExch(p.status, ST_TIMEOUT_DRAIN);
       }
@@ -171,50 +183,48 @@ kvsall_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
   } else if (warp == 1) {
     // =========================================================================== MMA issuer
     // The two GEMMs of consecutive tiles are issued in whichever order their inputs become ready: the second GEMM
-    // of tile g (needs dS from the epilogue) ahead of the first GEMM of tile g + 2 (needs the Y stage that the
-    // former releases), so that the tensor pipe has work while that stage is being refilled.
+    // of tile g (needs dS from the epilogue) ahead of the first GEMM of tile g + NBUF (whose S buffer it releases).
+    // The tensor pipe queues only a few MMAs, so a probe of an mbarrier between two of them leaves a bubble of about 90
+    // cycles (measured: 1650 cycles per 96-row tile without probes inside a GEMM, 2300 with one per 64-column slab).  All
+    // probes therefore sit between GEMMs, back to back so that their latencies overlap, and a tile has one load barrier.
     if (lane == 0) {
-      constexpr uint32_t IDESC_G1 = make_idesc_bf16(BLOCK_X, BLOCK_Y, 0, 0);  // S = X · Yᵀ, both K-major
+      constexpr uint32_t IDESC_G1 = make_idesc_bf16(BLOCK_X, C::BY, 0, 0);  // S = X · Yᵀ, both K-major
       constexpr uint32_t IDESC_G2 = make_idesc_bf16(BLOCK_X, D, 0, 1);        // out += dS · Y, Y read MN-major
       // descriptors are built once; per MMA only the 14-bit start-address field (16-byte units) is advanced
       const uint64_t xdesc = make_sw128_desc(smem_u32(sX), 16, 1024);
       const uint64_t ydesc_g1 = make_sw128_desc(smem_u32(sY), 16, 1024);
-      const uint64_t ydesc_g2 = make_sw128_desc(smem_u32(sY), SLAB_BYTES, 1024);
+      const uint64_t ydesc_g2 = make_sw128_desc(smem_u32(sY), C::YSLAB, 1024);
 
-      auto issue_g1 = [&](uint32_t gi) -> bool {
+      auto issue_g1 = [&](uint32_t gi) {
         const uint32_t st = gi % C::NSTAGE;
-        const uint32_t par = (gi / C::NSTAGE) & 1;
         stamp(gi, 1);
         tc_fence_after();
-        const uint64_t yd = ydesc_g1 + st * (C::TILE_BYTES >> 4);
-        const uint32_t d_tmem = tmem_s0 + (gi & 1) * BLOCK_Y;
+        const uint64_t yd = ydesc_g1 + st * (C::Y_BYTES >> 4);
+        const uint32_t b = gi % C::NBUF;
+        const uint32_t d_tmem = tmem_s0 + b * C::BY;
 #pragma unroll
         for (int sl = 0; sl < C::NSLAB; ++sl) {
-          if (sl > 0) {  // slab 0 was probed by the caller
-            if (!mbar_wait_bounded(y_full + st * 4 + sl, par, s_abort)) return false;
-            tc_fence_after();
-          }
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk) {
-            const uint32_t off16 = sl * (SLAB_BYTES >> 4) + kk * 2;  // 16 bf16 = 32 bytes inside the swizzle span
-            if (sl == 0 && kk == 0) mma_ss(d_tmem, xdesc + off16, yd + off16, IDESC_G1, 0u);
-            else mma_ss(d_tmem, xdesc + off16, yd + off16, IDESC_G1, 1u);
+            const uint32_t xo = sl * (C::XSLAB >> 4) + kk * 2;  // 16 bf16 = 32 bytes inside the swizzle span
+            const uint32_t yo = sl * (C::YSLAB >> 4) + kk * 2;
+            if (sl == 0 && kk == 0) mma_ss(d_tmem, xdesc + xo, yd + yo, IDESC_G1, 0u);
+            else mma_ss(d_tmem, xdesc + xo, yd + yo, IDESC_G1, 1u);
           }
         }
-        tc_commit(s_full + (gi & 1));
-        return true;
+        tc_commit(s_full + b);
       };
       auto issue_g2 = [&](uint32_t gi, bool first, bool last) {
         const uint32_t st = gi % C::NSTAGE;
         stamp(gi, 2);
         tc_fence_after();
-        const uint64_t yd = ydesc_g2 + st * (C::TILE_BYTES >> 4);
-        const uint32_t a_base = tmem_s0 + (gi & 1) * BLOCK_Y;
+        const uint64_t yd = ydesc_g2 + st * (C::Y_BYTES >> 4);
+        const uint32_t a_base = tmem_s0 + (gi % C::NBUF) * C::BY;
 #pragma unroll
-        for (int k = 0; k < BLOCK_Y / 16; ++k) {
+        for (int k = 0; k < C::BY / 16; ++k) {
           // dS: the 32 K elements of column group c are packed into columns [32 c, 32 c + 16) of the S buffer
           const uint32_t a_tmem = a_base + 32 * (k >> 1) + 8 * (k & 1);
-          // Y tile as [K = 128 rows, N = D]: N blocks of 64 are one slab apart, groups of 8 K-rows 1024 B apart;
+          // Y tile as [K = BY rows, N = D]: N blocks of 64 are one slab apart, groups of 8 K-rows 1024 B apart;
           // 16 K-rows = 2048 bytes
           if (k == 0) mma_ts(tmem_out, a_tmem, yd, IDESC_G2, first ? 0u : 1u);
           else mma_ts(tmem_out, a_tmem, yd + k * 128, IDESC_G2, 1u);
@@ -230,16 +240,17 @@ kvsall_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
       bool ok = true;
       while (!c2.done() && ok && !*s_abort) {
         bool progressed = false;
-        if (g2 < g1 && mbar_test_wait(ds_full + (g2 & 1), (g2 >> 1) & 1) &&
-            (!c2.first() || mbar_test_wait(dx_empty, (c2.seg & 1) ^ 1))) {
+        // readiness only ever goes from false to true until this thread consumes it
+        const bool ds_ready = mbar_test_wait(ds_full + g2 % C::NBUF, (g2 / C::NBUF) & 1);
+        const bool y_ready = mbar_test_wait(y_full + g1 % C::NSTAGE, (g1 / C::NSTAGE) & 1);
+        if (g2 < g1 && ds_ready && (!c2.first() || mbar_test_wait(dx_empty, (c2.seg & 1) ^ 1))) {
           issue_g2(g2, c2.first(), c2.last());
           ++g2;
           c2.advance();
           progressed = true;
         }
-        if (!progressed && !c1.done() && g1 - g2 < 2 && (!c1.first() || mbar_test_wait(x_full, c1.seg & 1)) &&
-            mbar_test_wait(y_full + (g1 % C::NSTAGE) * 4, (g1 / C::NSTAGE) & 1)) {
-          if (!issue_g1(g1)) { ok = false; break; }
+        if (!c1.done() && g1 - g2 < C::NBUF && y_ready && (!c1.first() || mbar_test_wait(x_full, c1.seg & 1))) {
+          issue_g1(g1);
           if (c1.last()) tc_commit(x_empty);  // last S GEMM of the segment: the X buffer may be refilled
           ++g1;
           c1.advance();
@@ -258,7 +269,7 @@ kvsall_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
   } else {
     // =========================================================================== epilogue warps
     const int quarter = warp & 3;              // TMEM lane group this warp may access
-    const int cg = (warp - 2) >> 2;            // which 32 of the 128 S columns
+    const int cg = (warp - 2) >> 2;            // which 32 of the S columns
     const uint32_t lane_sel = static_cast<uint32_t>(quarter * 32) << 16;
     const int row = quarter * 32 + lane;
     float loss_acc = 0.f;
@@ -279,26 +290,31 @@ kvsall_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
       }
 
       // label words are fetched one tile ahead: the strided global load would otherwise sit on the critical path
+      // (a tile may reach past the row's last word: those columns are padding)
       const uint32_t* mrow = nullptr;
+      int mword_at = y0 * C::NCG + cg;
       uint32_t mnext = 0u;
       if constexpr (MASK) {
         if (valid_x) {
-          mrow = p.mask + static_cast<size_t>(x_global) * p.mask_stride + y0 * 4 + cg;
-          mnext = mrow[0];
+          mrow = p.mask + static_cast<size_t>(x_global) * p.mask_stride;
+          if (mword_at < p.mask_stride) mnext = mrow[mword_at];
         }
       }
       for (int t = 0; t < n; ++t, ++g) {
-        const uint32_t b = g & 1;
+        const uint32_t b = g % C::NBUF;
         const uint32_t mword = mnext;
         if constexpr (MASK) {
-          if (valid_x && t + 1 < n) mnext = mrow[(t + 1) * 4];
+          mword_at += C::NCG;
+          mnext = 0u;
+          if (valid_x && t + 1 < n && mword_at < p.mask_stride) mnext = mrow[mword_at];
         }
         // the 32 per-column scalars of this chunk: the same addresses in every lane (a broadcast from L1), fetched
         // before the wait for S
+        const int y_valid = p.y_rows - (y0 + t) * C::BY - cg * 32;  // columns >= y_valid of this chunk are padding
         float yb[SCORE != 0 ? 32 : 1];
         if constexpr (SCORE != 0) {
-          if (p.y_bias != nullptr) {
-            const float4* src = reinterpret_cast<const float4*>(p.y_bias + static_cast<size_t>(y0 + t) * BLOCK_Y + cg * 32);
+          if (p.y_bias != nullptr && y_valid > 0) {   // y_bias is readable up to the next multiple of 128 rows
+            const float4* src = reinterpret_cast<const float4*>(p.y_bias + static_cast<size_t>(y0 + t) * C::BY + cg * 32);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               const float4 v = __ldg(src + i);
@@ -309,11 +325,10 @@ kvsall_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
             for (int i = 0; i < 32; ++i) yb[i] = 0.f;
           }
         }
-        if (!mbar_wait_bounded(s_full + b, (g >> 1) & 1, s_abort)) { ok = false; break; }
+        if (!mbar_wait_bounded(s_full + b, (g / C::NBUF) & 1, s_abort)) { ok = false; break; }
         if (warp == 2 && lane == 0) stamp(g, 3);
         tc_fence_after();
-        const int y_valid = p.y_rows - (y0 + t) * BLOCK_Y - cg * 32;  // columns >= y_valid of this chunk are padding
-        const uint32_t s_addr = tmem_s0 + b * BLOCK_Y + lane_sel + cg * 32;
+        const uint32_t s_addr = tmem_s0 + b * C::BY + lane_sel + cg * 32;
         uint32_t r[32];
         tmem_ld32(s_addr, r);
         tc_wait_ld();
@@ -333,36 +348,26 @@ kvsall_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         if (valid_x && p.x_dsum != nullptr) atomicAdd(p.x_dsum + x_global, seg_dsum * p.scale);
       }
 
-      // drain the accumulated out tile of this segment: this warp owns D / 4 of its columns
+      // drain the accumulated out tile of this segment: chunks of CW columns are dealt to the column groups
       if (!mbar_wait_bounded(dx_full, seg & 1, s_abort)) { ok = false; break; }
       tc_fence_after();
       float* out_row = p.out;
       if (valid_x) out_row = p.out + static_cast<size_t>(x_global) * D;
-      constexpr int DC = D / 4;
-      if constexpr (DC >= 32) {
+      constexpr int CW = D >= 128 ? 32 : 16;
 #pragma unroll
-        for (int c = 0; c < DC / 32; ++c) {
-          const int col0 = cg * DC + c * 32;
-          uint32_t r[32];
-          tmem_ld32(tmem_out + lane_sel + col0, r);
+      for (int c0 = 0; c0 < D / CW; c0 += C::NCG) {
+        const int col0 = (c0 + cg) * CW;
+        if (col0 < D) {
+          uint32_t r[CW];
+          if constexpr (CW == 32) tmem_ld32(tmem_out + lane_sel + col0, r);
+          else tmem_ld16(tmem_out + lane_sel + col0, r);
           tc_wait_ld();
           if (valid_x) {
 #pragma unroll
-            for (int i = 0; i < 32; i += 4)
+            for (int i = 0; i < CW; i += 4)
               red_add_v4(out_row + col0 + i, __uint_as_float(r[i]) * p.scale, __uint_as_float(r[i + 1]) * p.scale,
                          __uint_as_float(r[i + 2]) * p.scale, __uint_as_float(r[i + 3]) * p.scale);
           }
-        }
-      } else {
-        const int col0 = cg * DC;
-        uint32_t r[16];
-        tmem_ld16(tmem_out + lane_sel + col0, r);
-        tc_wait_ld();
-        if (valid_x) {
-#pragma unroll
-          for (int i = 0; i < 16; i += 4)
-            red_add_v4(out_row + col0 + i, __uint_as_float(r[i]) * p.scale, __uint_as_float(r[i + 1]) * p.scale,
-                       __uint_as_float(r[i + 2]) * p.scale, __uint_as_float(r[i + 3]) * p.scale);
         }
       }
       tc_fence_before();
@@ -370,7 +375,7 @@ kvsall_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
       if (warp == 2 && lane == 0) stamp(g - 1, 5);
       if (lane == 0) mbar_arrive(dx_empty);
       if (p.opt.param != nullptr) {
-        // the y tiles of this segment are counted once all sixteen warps' reductions are on their way to L2; whoever
+        // the y tiles of this segment are counted once all epilogue warps' reductions are on their way to L2; whoever
         // brings the count of the x tile to ny_tiles holds the last partial sum and applies the update.  The hand-shake
         // between the warps uses mbarriers with bounded waits, like every other wait of this kernel.
         __threadfence();
@@ -397,7 +402,7 @@ kvsall_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
           uint2* __restrict__ ps = reinterpret_cast<uint2*>(p.opt.shadow) + base4;
           const int kind = p.opt.kind;
           const OptStepConsts c = opt_step_consts(kind, *p.opt.step + 1, p.opt.beta1, p.opt.beta2);
-          for (int i = threadIdx.x - 64; i < rows * (D / 4); i += 32 * NUM_EPI_WARPS) {
+          for (int i = threadIdx.x - 64; i < rows * (D / 4); i += 32 * C::EPI_WARPS) {
             float4 wv = pw[i];
             const float4 gv = __ldcg(pg + i);   // the sums were formed in L2 by other SMs' reductions
             float4 m = make_float4(0.f, 0.f, 0.f, 0.f), v = m;
@@ -452,7 +457,7 @@ static int launch(const CUtensorMap& tx, const CUtensorMap& ty, const KvsAllPara
       return -3;
     configured[dev] = true;
   }
-  return launch_pdl(kern, dim3(num_ctas), dim3(NUM_THREADS), Cfg<D>::SMEM_BYTES, stream, tx, ty, p) == cudaSuccess ? 0 : -4;
+  return launch_pdl(kern, dim3(num_ctas), dim3(Cfg<D>::THREADS), Cfg<D>::SMEM_BYTES, stream, tx, ty, p) == cudaSuccess ? 0 : -4;
 }
 
 }  // namespace dice
@@ -482,7 +487,8 @@ extern "C" int dice_kvsall_fused(const void* x, int x_rows, const void* y, int y
   CUtensorMap tx, ty;
   int rc = make_tmap_bf16(&tx, x, x_rows, D);
   if (rc) return rc;
-  rc = make_tmap_bf16(&ty, y, y_rows, D);
+  const int by = D == 256 ? Cfg<256>::BY : D == 128 ? Cfg<128>::BY : Cfg<64>::BY;
+  rc = make_tmap_bf16(&ty, y, y_rows, D, by);
   if (rc) return rc;
   KvsAllParams p;
   p.out = out;
@@ -491,8 +497,8 @@ extern "C" int dice_kvsall_fused(const void* x, int x_rows, const void* y, int y
   p.x_rows = x_rows;
   p.y_rows = y_rows;
   p.nx_tiles = (x_rows + BLOCK_X - 1) / BLOCK_X;
-  p.ny_tiles = (y_rows + BLOCK_Y - 1) / BLOCK_Y;
-  p.map = TileMap::make(p.nx_tiles, p.ny_tiles, BLOCK_Y * D * 2, 48ll << 20);
+  p.ny_tiles = (y_rows + by - 1) / by;
+  p.map = TileMap::make(p.nx_tiles, p.ny_tiles, by * D * 2, 48ll << 20);
   p.base = base;
   p.scale = scale;
   p.mask = mask;
