@@ -147,6 +147,18 @@ int dice_candidate_bce(const float* q, const long long* cand, long long cand_str
                        const float* labels, const float* const* ent, float* const* g_ent, float* dq, float* scores,
                        double* loss, float scale, int kind, float margin, float eps, int N, int D, int W,
                        unsigned char* const* touched, long long num_entities, int* status, void* stream);
+int dice_sampled_grad(int model, int normalize, int draw, const long long* h, const long long* r, long long idx_stride,
+                      const long long* cand, long long cand_stride, const float* labels, const long long* pos, int N, int C,
+                      unsigned long long seed, unsigned long long offset, const long long* step, float label_pos,
+                      float label_neg, const float* ent, float* g_ent, unsigned char* touched, int* list_head, void* nodes,
+                      float* fixed, long long num_entities, const float* rel, float* g_rel, long long num_relations,
+                      const float* coeff, float* g_coeff, double* loss, float scale, float margin, float eps, int D,
+                      int* status, void* stream);
+int dice_sampled_update(int kind, int sparse, float* E, float* gE, float* mE, float* vE, unsigned char* touched,
+                        int* list_head, const void* nodes, const float* fixed, long long rows, int D, int C, int translation,
+                        float* R, float* gR, float* mR, float* vR, long long nR, float* coeff, float* gC, float* mC,
+                        float* vC, long long nC, float lr, float beta1, float beta2, float eps, float weight_decay,
+                        double* loss, float* loss_out, long long* step, unsigned int* done, void* stream);
 
 // ---------------------------------------------------------------------------------------- optimisers, step bookkeeping
 int dice_optimizer_step(int kind, float* param, float* grad, float* m, float* v, void* shadow, const long long* step,

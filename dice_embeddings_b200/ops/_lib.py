@@ -127,6 +127,8 @@ class _Sigs:
     dice_uniform_int = [_p, _l, _l, ctypes.c_ulonglong, ctypes.c_ulonglong, _p, _l, _l, _p]
     dice_neg_sample = [_p, _i, _i, _l, ctypes.c_ulonglong, ctypes.c_ulonglong, _p, _i, _f, _f, _p, _p, _p, _p, _p, _p]
     dice_candidate_bce = [_p, _p, _l, _l, _i, _p, _p, _p, _p, _p, _p, _f, _i, _f, _f, _i, _i, _i, _p, _l, _p, _p]
+    dice_sampled_grad = [_i, _i, _i, _p, _p, _l, _p, _l, _p, _p, _i, _i, ctypes.c_ulonglong, ctypes.c_ulonglong, _p, _f, _f, _p, _p, _p, _p, _p, _p, _l, _p, _p, _l, _p, _p, _p, _f, _f, _f, _i, _p, _p]
+    dice_sampled_update = [_i, _i, _p, _p, _p, _p, _p, _p, _p, _p, _l, _i, _i, _i, _p, _p, _p, _p, _l, _p, _p, _p, _p, _l, _f, _f, _f, _f, _f, _p, _p, _p, _p, _p]
     dice_sparse_rows_optimizer = [_i, _p, _p, _p, _p, _p, _p, _l, _i, _p, _f, _f, _f, _f, _f, _p]
     dice_eval_rank = [_p, _i, _p, _i, _i, _p, _p, _p, _i, _i, _p, _i, _i, _p, _p, _p, _p, _i, _p, _p, _p, _p, _l, _p, _p]
     dice_eval_rank_cand_cap = [_i, _i, _i, _i, _i]

@@ -444,6 +444,78 @@ def sparse_rows_optimizer(kind: int, param, grad, m, v, shadow, touched: torch.T
           float(weight_decay), others=(grad, m, v, shadow, touched, step))
 
 
+SAMPLED_DRAW = {"given": 0, "corrupt": 1, "tails": 2}
+
+
+class SampledStep:
+    """Launch arguments of ``dice_sampled_grad`` + ``dice_sampled_update`` for one batch shape: the training step on
+    sampled candidates against one table (see ``csrc/sampled_step.cu``).
+
+    ``draw`` "given": ``x`` holds the queries' head and relation ids in its first two columns, ``cand`` (row stride
+    ``cand.stride(0)``) and ``labels [N, C]`` the candidates; "corrupt" / "tails": ``pos [N, 3]`` holds the positives and
+    the corruptions are drawn on the device.  ``head`` (int32 per entity row, filled with -1) switches on the chains of
+    drawn entities; it is only worth having while a row is drawn a few times per step at most (``MAX_CHAIN``)."""
+
+    #: expected draws per row up to which the chains are used: a chain is walked serially, one L2 round trip per link
+    MAX_CHAIN = 4
+
+    def __init__(self, code: int, normalize: bool, draw: str, N: int, C: int, E, gE, mE, vE, touched, head, R, gR, mR, vR,
+                 coeff, gC, mC, vC, opt_kind: int, sparse: bool, seed: int, label_pos: float, label_neg: float, scale: float,
+                 margin: float, eps: float, step, loss_acc, loss_out, status, num_entities: int):
+        dev = E.device
+        for n, t in (("E", E), ("gE", gE), ("mE", mE), ("vE", vE), ("R", R), ("gR", gR), ("mR", mR), ("vR", vR),
+                     ("loss_out", loss_out)):
+            _req(t, torch.float32, n)
+        _req(touched, torch.uint8, "touched")
+        _req(step, torch.int64, "step")
+        _req(loss_acc, torch.float64, "loss_acc")
+        _req(status, torch.int32, "status")
+        D = E.shape[1]
+        assert E.shape == gE.shape == mE.shape == vE.shape and touched.numel() >= E.shape[0]
+        assert R.shape == gR.shape == mR.shape == vR.shape and R.shape[1] == D
+        assert draw in SAMPLED_DRAW and num_entities <= E.shape[0]
+        chained = head is not None and draw != "given" and N * (C - 1) <= self.MAX_CHAIN * num_entities and N * C < 2 ** 31
+        self.nodes = torch.empty(N * C, 2, dtype=torch.int32, device=dev) if chained else None
+        self.fixed = torch.empty(N, D, dtype=torch.float32, device=dev) if chained else None
+        if chained:
+            _req(head, torch.int32, "head")
+            assert head.numel() >= E.shape[0]
+        self.head = head if chained else None
+        self.done = torch.zeros(1, dtype=torch.int32, device=dev)
+        self.a = (int(code), int(bool(normalize)), SAMPLED_DRAW[draw], int(N), int(C))
+        self.E, self.step, self.status = E, step, status
+        self._keep = (gE, mE, vE, touched, head, R, gR, mR, vR, coeff, gC, mC, vC, loss_acc, loss_out)
+        trainable = coeff is not None and gC is not None
+        self._grad_tail = (_ptr(step), float(label_pos), float(label_neg), _ptr(E), _ptr(gE), _ptr(touched), _ptr(self.head),
+                           _ptr(self.nodes), _ptr(self.fixed), int(num_entities), _ptr(R), _ptr(gR), int(R.shape[0]),
+                           _ptr(coeff), _ptr(gC) if trainable else None, _ptr(loss_acc), float(scale), float(margin),
+                           float(eps), int(D), _ptr(status))
+        self.seed = int(seed) & (2 ** 64 - 1)
+        c_args = (_ptr(coeff), _ptr(gC), _ptr(mC), _ptr(vC), coeff.numel()) if trainable else (None, None, None, None, 0)
+        self._upd_head = (int(opt_kind), int(sparse), _ptr(E), _ptr(gE), _ptr(mE), _ptr(vE), _ptr(touched), _ptr(self.head),
+                          _ptr(self.nodes), _ptr(self.fixed), int(E.shape[0]), int(D), int(C), int(code == 5), _ptr(R),
+                          _ptr(gR), _ptr(mR), _ptr(vR), R.numel(), *c_args)
+        self._upd_tail = (_ptr(loss_acc), _ptr(loss_out), _ptr(step), _ptr(self.done))
+
+    def launch(self, lr: float, beta1: float, beta2: float, eps: float, weight_decay: float, x=None, cand=None, labels=None,
+               pos=None) -> None:
+        code, normalize, draw, N, C = self.a
+        if draw == 0:
+            assert x.dtype == torch.int64 and cand.dtype == torch.int64 and x.stride(1) == 1
+            assert x.shape[0] == N and cand.shape == (N, C) and (C == 1 or cand.stride(1) == 1)
+            _req(labels, torch.float32, "labels")
+            assert labels.numel() == N * C
+            src = (_ptr(x), x.data_ptr() + 8, x.stride(0), _ptr(cand), cand.stride(0), _ptr(labels), None)
+        else:
+            _req(pos, torch.int64, "pos")
+            assert pos.shape == (N, 3)
+            src = (None, None, 0, None, 0, None, _ptr(pos))
+        _call("dice_sampled_grad", self.E, code, normalize, draw, *src, N, C, self.seed, 0, *self._grad_tail,
+              others=(x, cand, labels, pos))
+        _call("dice_sampled_update", self.E, *self._upd_head, float(lr), float(beta1), float(beta2), float(eps),
+              float(weight_decay), *self._upd_tail)
+
+
 def eval_rank(x: torch.Tensor, y: torch.Tensor, target: Optional[torch.Tensor], target_idx: Optional[torch.Tensor],
               greater: Optional[torch.Tensor], status: torch.Tensor, col_bias: Optional[torch.Tensor] = None,
               y_offset: int = 0, y_stride: int = 1, k: int = 0, cand_score: Optional[torch.Tensor] = None,

@@ -2,11 +2,9 @@
 
 One step is the launch sequence
 
-1. ``neg_sample``        (NegSample only) corrupted triples + labels from the counter-based device generator
-2. ``lookup_compose``    gather ``E[h]``, ``R[r]`` and compose the query vectors in fp32
-3. ``candidate_bce``     score each query against its own candidates, BCE-with-logits, ``dq`` and candidate-row grads
-4. ``compose_backward``  chain rule of the composition into ``dE`` / ``dR``
-5. ``optimizer_step`` ×k and ``finish_step``
+1. ``sampled_grad``      the corruptions (NegSample) drawn by the counter-based generator, gather of ``E[h]`` and ``R[r]``,
+                         composition, scores against the candidates, BCE-with-logits, all gradients
+2. ``sampled_update``    optimiser over the entities, the relations and the coefficient; loss and step counter
 
 replayed from a CUDA graph.  The reference runs the same step as ``forward_triples`` / ``forward_k_vs_sample`` +
 ``BCEWithLogitsLoss`` + autograd + ``torch.optim`` (``dicee/models/base_model.py:25-46, 331-344``), with the
@@ -101,51 +99,41 @@ class FusedSampledEngine:
         self.loss_acc = torch.zeros(1, dtype=torch.float64, device=dev)
         self.loss_out = torch.zeros(1, dtype=torch.float32, device=dev)
         self.status = torch.zeros(1, dtype=torch.int32, device=dev)
-        self.ent_tab = K.pointer_table([self.E], dev)
-        self.gent_tab = K.pointer_table([self.gE], dev)
+        self.touched = torch.zeros(self.NE, dtype=torch.uint8, device=dev)
+        self.list_head = torch.full((self.NE,), -1, dtype=torch.int32, device=dev)
         self._bufs = {}
         self._graphs = {}
 
     # ------------------------------------------------------------------ buffers
     def _buffers(self, key):
-        """``key = (queries N, candidates C, positives B or 0)``."""
+        """``key = (groups N, candidates C, draw)``."""
         if key not in self._bufs:
-            N, C, B = key
+            N, C, draw = key
             dev = self.device
-            b = SimpleNamespace()
-            b.h, b.r = (torch.zeros(N, dtype=torch.int64, device=dev) for _ in range(2))
-            b.cand = torch.zeros(N, C, dtype=torch.int64, device=dev)
-            b.labels = torch.zeros(N, C, dtype=torch.float32, device=dev)
-            b.q = torch.zeros(N, self.D, dtype=torch.float32, device=dev)
-            b.dq = torch.zeros(N, self.D, dtype=torch.float32, device=dev)
-            b.pos = torch.zeros(max(B, 1), 3, dtype=torch.int64, device=dev)
+            b = SimpleNamespace(x=None, cand=None, labels=None, pos=None)
+            if draw == "corrupt":
+                b.pos = torch.zeros(N, 3, dtype=torch.int64, device=dev)
+            else:
+                triples = self.st == "NegSample"     # one candidate per query, in the third column
+                b.x = torch.zeros(N, 3 if triples else 2, dtype=torch.int64, device=dev)
+                b.cand = b.x[:, 2:3] if triples else torch.zeros(N, C, dtype=torch.int64, device=dev)
+                b.labels = torch.zeros(N, C, dtype=torch.float32, device=dev)
+            c = (self.coeff, self.gC, self.mC, self.vC) if self.coeff is not None else (None,) * 4
+            if not self.coeff_trainable:
+                c = (c[0], None, None, None)
+            b.step = K.SampledStep(self.code, self.normalize, draw, N, C, self.E, self.gE, self.mE, self.vE, self.touched,
+                                   self.list_head, self.R, self.gR, self.mR, self.vR, *c, self.opt_kind, False, self.seed,
+                                   1.0 - self.label_smoothing, self.label_smoothing, 1.0 / (float(N) * float(C)),
+                                   self.margin, self.dist_eps, self.step_count, self.loss_acc, self.loss_out, self.status,
+                                   self.NE)
             self._bufs[key] = b
         return self._bufs[key]
 
-    def _launch_all(self, b, key) -> None:
-        N, C, B = key
-        if B:  # draw the corruptions on the device
-            K.neg_sample(b.pos, self.neg_ratio, self.NE, self.seed, 0, b.labels, hrt=(b.h, b.r, b.cand),
-                         label_pos=1.0 - self.label_smoothing, label_neg=self.label_smoothing, step=self.step_count)
-        scale = 1.0 / float(N * C)
-        K.lookup_compose(self.code, self.normalize, b.h, b.r, self.ent_tab, 1, self.NE, self.R, self.coeff, None, 0,
-                         0, b.q, N, self.D, self.status)
-        K.candidate_bce(b.q, b.cand, C, 1, C, b.labels, self.ent_tab, 1, self.gent_tab, b.dq, None, self.loss_acc,
-                        scale, self.kind, self.margin, self.dist_eps)
-        K.compose_backward(self.code, self.normalize, b.h, b.r, self.ent_tab, 1, self.R, self.coeff, b.dq,
-                           self.gent_tab, self.gR, self.gC if self.coeff_trainable else None, N, self.D)
-        b1, b2 = self.betas
-        K.optimizer_step(self.opt_kind, self.E, self.gE, self.mE, self.vE, None, self.step_count, self.lr, b1, b2,
-                         self.eps, self.weight_decay)
-        K.optimizer_step(self.opt_kind, self.R, self.gR, self.mR, self.vR, None, self.step_count, self.lr, b1, b2,
-                         self.eps, self.weight_decay)
-        if self.coeff_trainable:
-            K.optimizer_step(self.opt_kind, self.coeff, self.gC, self.mC, self.vC, None, self.step_count, self.lr,
-                             b1, b2, self.eps, self.weight_decay)
-        K.finish_step(self.loss_acc, self.loss_out, 1.0, self.step_count)
+    def _launch_all(self, b) -> None:
+        b.step.launch(self.lr, *self.betas, self.eps, self.weight_decay, x=b.x, cand=b.cand, labels=b.labels, pos=b.pos)
 
     def launches_per_step(self, with_sampling: bool = True) -> int:
-        return 6 + (1 if with_sampling and self.st == "NegSample" else 0) + (1 if self.coeff_trainable else 0)
+        return 2
 
     def _tensors(self):
         t = [self.E, self.R, self.mE, self.vE, self.mR, self.vR, self.gE, self.gR, self.step_count, self.loss_acc]
@@ -159,14 +147,14 @@ class FusedSampledEngine:
             self.use_graph = False
             self._graphs.clear()
         if not self.use_graph:
-            self._launch_all(b, key)
+            self._launch_all(b)
             return
         if gkey not in self._graphs:
             s = torch.cuda.Stream(device=self.device)
             s.wait_stream(torch.cuda.current_stream(self.device))
             state = [(x, x.clone()) for x in self._tensors()]
             with torch.cuda.stream(s):
-                self._launch_all(b, key)
+                self._launch_all(b)
             torch.cuda.current_stream(self.device).wait_stream(s)
             torch.cuda.synchronize(self.device)
             K.check_status(self.status, "during sampled-step warm-up")
@@ -174,7 +162,7 @@ class FusedSampledEngine:
                 x.copy_(c)
             g = torch.cuda.CUDAGraph()
             with torch.cuda.graph(g):
-                self._launch_all(b, key)
+                self._launch_all(b)
             self._graphs[gkey] = g
         self._graphs[gkey].replay()
 
@@ -186,27 +174,22 @@ class FusedSampledEngine:
           corruptions drawn by the device generator;
         * 1vsSample / KvsSample: ``(x [B, 2], candidate ids [B, C], labels [B, C])``.
         """
-        if self.st == "NegSample":
-            if len(batch) == 1 or batch[1] is None:
-                pos = batch[0]
-                B = pos.shape[0]
-                key = (B * (1 + self.neg_ratio), 1, B)
-                b = self._buffers(key)
-                b.pos.copy_(pos)
-            else:
-                x, y = batch[0], batch[1]
-                key = (x.shape[0], 1, 0)
-                b = self._buffers(key)
-                b.h.copy_(x[:, 0])
-                b.r.copy_(x[:, 1])
-                b.cand.copy_(x[:, 2:3])
-                b.labels.copy_(y.reshape(-1, 1))
+        if self.st == "NegSample" and (len(batch) == 1 or batch[1] is None):
+            pos = batch[0]
+            key = (pos.shape[0], 1 + self.neg_ratio, "corrupt")
+            b = self._buffers(key)
+            b.pos.copy_(pos)
+        elif self.st == "NegSample":
+            x, y = batch[0], batch[1]
+            key = (x.shape[0], 1, "given")
+            b = self._buffers(key)
+            b.x.copy_(x)
+            b.labels.copy_(y.reshape(-1, 1))
         else:
             x, idx, y = batch[0], batch[1], batch[2]
-            key = (x.shape[0], idx.shape[1], 0)
+            key = (x.shape[0], idx.shape[1], "given")
             b = self._buffers(key)
-            b.h.copy_(x[:, 0])
-            b.r.copy_(x[:, 1])
+            b.x.copy_(x)
             b.cand.copy_(idx)
             b.labels.copy_(y)
         self._run(b, key)

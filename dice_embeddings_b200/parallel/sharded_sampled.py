@@ -20,7 +20,10 @@ the same shape, all in the symmetric heap) and its own slice of the batch.  One 
         optimizer_step (relations, ...)  reads all ranks' gradient buffers by peer loads: all-reduce folded into the update
         finish_step                      global mean loss
 
-so the index dispatch / row gather / gradient combine of an embedding-parallel step never goes through a collective
+With one rank the table is local and the step is the two launches of ``csrc/sampled_step.cu``: drawn entities never get a
+gradient row in memory, their triples are chained per row and added up inside the row's update.
+
+So the index dispatch / row gather / gradient combine of an embedding-parallel step never goes through a collective
 library call, and rows that were not sampled cost nothing.  The reference trains these techniques with dense
 ``torch.optim`` updates of the whole table on every replica (``dicee/models/base_model.py:86-118``).
 """
@@ -107,6 +110,8 @@ class ShardedSampledEngine:
         self.tab = SimpleNamespace(E=heap.table("E"), gE=heap.table("gE"), touched=heap.table("touched"),
                                    gR=heap.table("gR"), gC=heap.table("gC"), loss=heap.table("loss"),
                                    sig=heap.table("sig"))
+        if W == 1:
+            self.list_head = torch.full((self.rows_pad,), -1, dtype=torch.int32, device=dev)
         self._bufs = {}
         self._graphs = {}
         self._eager_done = set()
@@ -120,6 +125,9 @@ class ShardedSampledEngine:
             dev = self.device
             b = SimpleNamespace()
             b.pos = torch.zeros(max(B, 1), 3, dtype=torch.int64, device=dev)
+            if self.W == 1:
+                self._bufs[key] = self._local_buffers(b, key)
+                return b
             b.h, b.r = (torch.zeros(N, dtype=torch.int64, device=dev) for _ in range(2))
             b.cand = torch.zeros(N, C, dtype=torch.int64, device=dev)
             b.labels = torch.zeros(N, C, dtype=torch.float32, device=dev)
@@ -131,12 +139,36 @@ class ShardedSampledEngine:
             self._bufs[key] = b
         return self._bufs[key]
 
+    def _local_buffers(self, b, key):
+        """One rank: the arguments of the two-launch step."""
+        N, C, B = key
+        draw = {"flat": "corrupt", "tails": "tails", "given": "given"}[self.layout]
+        if draw == "corrupt":
+            N, C = B, N // B            # B (1 + k) single triples are B groups of 1 + k
+        b.x = b.cand = b.labels = None
+        if draw == "given":
+            b.x = torch.zeros(N, 2, dtype=torch.int64, device=self.device)
+            b.cand = torch.zeros(N, C, dtype=torch.int64, device=self.device)
+            b.labels = torch.zeros(N, C, dtype=torch.float32, device=self.device)
+        c = (None,) * 4 if self.coeff is None else (self.coeff, self.gC[:1], self.mC, self.vC)
+        if not self.coeff_trainable:
+            c = (c[0], None, None, None)
+        b.step = K.SampledStep(self.code, self.normalize, draw, N, C, self.E, self.gE, self.mE, self.vE, self.touched,
+                               self.list_head, self.R, self.gR, self.mR, self.vR, *c, self.opt_kind, True, self.seed,
+                               1.0 - self.label_smoothing, self.label_smoothing, 1.0 / (float(N) * float(C)), self.margin,
+                               self.dist_eps, self.step_count, self.loss_acc[:1], self.loss_out, self.status, self.NE)
+        return b
+
     def _barrier(self) -> None:
         K.p2p_barrier(self.tab.sig, self.rank, self.W, self.barrier_count, self.status)
 
     def _launch_all(self, b, key) -> None:
         N, C, B = key
         W, D = self.W, self.D
+        if W == 1:
+            b.step.launch(self.lr, *self.betas, self.eps, self.weight_decay, x=b.x, cand=b.cand, labels=b.labels,
+                          pos=None if self.layout == "given" else b.pos)
+            return
         scale = 1.0 / (float(N) * float(C) * float(W))
         self._barrier()                                          # S0
         self.gR.zero_()
@@ -170,6 +202,8 @@ class ShardedSampledEngine:
         K.finish_step(self.loss_acc, self.loss_out, 1.0, self.step_count, acc_table=self.tab.loss, n_acc=W)
 
     def launches_per_step(self) -> int:
+        if self.W == 1:
+            return 2
         return 2 + 6 + (1 if self.layout in ("flat", "tails") else 0) + (1 if self.coeff_trainable else 0)
 
     def _run(self, b, key) -> None:
@@ -205,8 +239,11 @@ class ShardedSampledEngine:
             x, idx, y = batch[0], batch[1], batch[2]
             key = (x.shape[0], idx.shape[1], 0)
             b = self._buffers(key)
-            b.h.copy_(x[:, 0])
-            b.r.copy_(x[:, 1])
+            if self.W == 1:
+                b.x.copy_(x)
+            else:
+                b.h.copy_(x[:, 0])
+                b.r.copy_(x[:, 1])
             b.cand.copy_(idx)
             b.labels.copy_(y)
         self._run(b, key)

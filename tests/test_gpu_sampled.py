@@ -157,3 +157,91 @@ def test_uniform_int_into_column_block():
     flat = torch.empty(300 * 8, dtype=torch.int64, device=DEV)
     K.uniform_int(flat, 50, seed=3)
     assert torch.equal(flat.view(300, 8), cand[:, 1:])
+
+
+# The drawn corruptions of the two-launch step: widths at the edges of the lane layouts (one, two and four floats per lane,
+# several chunks), table sizes with and without chains (4 draws per row is the limit), groups split over several warps.
+@pytest.mark.parametrize("name,D,NE,B,k", [
+    ("DistMult", 4, 50, 33, 1), ("DistMult", 36, 4000, 700, 5), ("DistMult", 132, 4000, 700, 5), ("DistMult", 512, 900, 64, 3),
+    ("ComplEx", 64, 4000, 333, 40), ("ComplEx", 72, 3000, 50, 100), ("ComplEx", 256, 100, 200, 9), ("ComplEx", 264, 3000, 65, 7),
+    ("QMult", 64, 2000, 256, 3), ("QMult", 144, 2000, 100, 17), ("OMult", 256, 2000, 100, 9), ("OMult", 288, 2000, 31, 9),
+    ("Keci", 96, 2000, 500, 10), ("Keci", 512, 2000, 100, 10), ("TransE", 100, 2000, 300, 6), ("TransE", 384, 60, 300, 6)])
+def test_drawn_corruptions_match_autograd(name, D, NE, B, k):
+    """fp32 sums of at most a few hundred terms in another order: 1e-4 of the largest gradient leaves a factor of 10."""
+    gen = torch.Generator(device=DEV).manual_seed(D + NE)
+    coins = set()
+    for step in range(8):
+        ref, fused = _pair(name, D, NE=NE)
+        pos = torch.stack((torch.randint(0, NE, (B,), device=DEV, generator=gen),
+                           torch.randint(0, 12, (B,), device=DEV, generator=gen),
+                           torch.randint(0, NE, (B,), device=DEV, generator=gen)), 1)
+        x = torch.zeros(B * (1 + k), 3, dtype=torch.int64, device=DEV)
+        y = torch.zeros(B * (1 + k), device=DEV)
+        K.neg_sample(pos, k, NE, 5, step, y, x=x, label_pos=0.9, label_neg=0.1)
+        coin = bool((x[B:, 0] != pos[:, 0].repeat(k)).any())
+        if coin in coins:
+            continue
+        coins.add(coin)
+        ref = ref.double()
+        loss_ref = torch.nn.functional.binary_cross_entropy_with_logits(ref(x), y.double())
+        loss_ref.backward()
+        eng = FusedSampledEngine(fused, "NegSample", lr=1.0, device=DEV, neg_ratio=k, label_smoothing=0.1, seed=5,
+                                 use_graph=step % 2 == 0)
+        eng.step_count.fill_(step)
+        start = {n: p.detach().double().clone() for n, p in fused.named_parameters()}
+        loss = eng.step((pos,))
+        eng.sync_to_model()
+        assert abs(float(loss) - float(loss_ref)) < 1e-5 * abs(float(loss_ref))
+        for (n, p_ref), (_, p) in zip(ref.named_parameters(), fused.named_parameters()):
+            if p_ref.grad is None:
+                continue
+            g = start[n] - p.detach().double()
+            # the update w - lr g rounds w to 2^-24 of its size on top
+            tol = 1e-4 * p_ref.grad.abs().max() + 2.0 ** -23 * start[n].abs().max()
+            assert (g - p_ref.grad).abs().max() < tol, (n, coin)
+        assert int(eng.touched.sum()) == 0 and int((eng.list_head != -1).sum()) == 0 and float(eng.gE.abs().sum()) == 0.0
+        assert int(eng.step_count) == step + 1
+    assert len(coins) == 2
+
+
+@pytest.mark.parametrize("name,D,NE,B,k", [("TransE", 128, 5000, 300, 9), ("ComplEx", 64, 777, 40, 33), ("QMult", 256, 90, 64, 50)])
+def test_sparse_update_of_drawn_tails(name, D, NE, B, k):
+    """Row-wise sparse Adam over drawn tails: same rows, same values as the flagged-row optimiser on autograd's gradient."""
+    ref, fused = _pair(name, D, NE=NE)
+    gen = torch.Generator(device=DEV).manual_seed(3)
+    pos = torch.stack((torch.randint(0, NE, (B,), device=DEV, generator=gen), torch.randint(0, 12, (B,), device=DEV, generator=gen),
+                       torch.randint(0, NE, (B,), device=DEV, generator=gen)), 1)
+    cand = torch.zeros(B, 1 + k, dtype=torch.int64, device=DEV)
+    cand[:, 0] = pos[:, 2]
+    step = torch.full((1,), 7, dtype=torch.int64, device=DEV)
+    K.uniform_int(cand[:, 1:], NE, 11, 0, step=step)
+    x = torch.stack((pos[:, :1].expand(-1, 1 + k), pos[:, 1:2].expand(-1, 1 + k), cand), 2).reshape(-1, 3)
+    y = torch.full((B, 1 + k), 0.1, device=DEV)
+    y[:, 0] = 0.9
+    loss_ref = torch.nn.functional.binary_cross_entropy_with_logits(ref(x), y.reshape(-1))
+    loss_ref.backward()
+    E, R = fused.entity_embeddings.weight.data, fused.relation_embeddings.weight.data
+    z = torch.zeros_like
+    mE = 1e-3 * torch.randn(E.shape, device=DEV, generator=gen)
+    vE = 1e-6 * (1 + torch.rand(E.shape, device=DEV, generator=gen))
+    touched, head = torch.zeros(NE, dtype=torch.uint8, device=DEV), torch.full((NE,), -1, dtype=torch.int32, device=DEV)
+    loss_acc, loss_out = torch.zeros(1, dtype=torch.float64, device=DEV), torch.zeros(1, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    want_p, want_m, want_v = E.clone(), mE.clone(), vE.clone()
+    flags = torch.zeros(NE, dtype=torch.uint8, device=DEV)
+    flags[cand.reshape(-1)] = 1
+    flags[pos[:, 0]] = 1
+    K.sparse_rows_optimizer(0, want_p, ref.entity_embeddings.weight.grad.clone(), want_m, want_v, None, flags, step, 0.01, 0.9,
+                            0.999, 1e-8, 0.0)
+    s = K.SampledStep(K.MODEL_CODE[name], name == "QMult", "tails", B, 1 + k, E, z(E), mE, vE, touched, head, R, z(R), z(R), z(R),
+                      None, None, None, None, 0, True, 11, 0.9, 0.1, 1.0 / (B * (1 + k)), float(getattr(fused, "margin", 0.0)),
+                      float(getattr(fused, "_eps", 0.0)), step, loss_acc, loss_out, status, NE)
+    s.launch(0.01, 0.9, 0.999, 1e-8, 0.0, pos=pos)
+    torch.cuda.synchronize()
+    assert int(status) == 0 and int(step) == 8 and abs(float(loss_out) - float(loss_ref)) < 1e-5 * float(loss_ref)
+    # gradients agree to 1e-4 of the largest (sums in another order); moments and weights follow from them
+    g = float(ref.entity_embeddings.weight.grad.abs().max())
+    assert (mE - want_m).abs().max() < 1e-5 * g + 1e-9
+    assert (vE - want_v).abs().max() < 1e-6 * g * g + 1e-12
+    assert (E - want_p).abs().max() < 0.01 * (1e-5 * g + 1e-9) / 1e-3 * 10 + 1e-6
+    assert int(touched.sum()) == 0 and int((head != -1).sum()) == 0
