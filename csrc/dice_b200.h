@@ -57,6 +57,27 @@ int dice_kvsall_pair(const void* x, int x_rows, const void* y, int y_rows, int D
                      int mask_stride, float pos_delta, int loss_share, long long* trace, void* stream);
 
 // Filtered-rank counting / running top-k over X Yᵀ without storing it (see csrc/eval_rank.cu).
+int dice_rank_count(const void* x, const void* x_lo, int x_rows, const void* y, const void* y_lo, int y_rows, int D,
+                    const float* target, const int* target_idx, const float* col_bias, int y_offset, int y_stride,
+                    const unsigned int* mask, long long mask_stride, int* greater, const float* margin, int* band_rows,
+                    int* band_cols, unsigned long long* band_count, long long band_cap, int* status, int num_ctas, void* stream);
+int dice_rank_group_max(const void* x, int x_rows, const void* y, int y_rows, int D, const float* col_bias, float* gmax,
+                        int groups, int* status, int num_ctas, void* stream);
+int dice_rank_collect(const void* x, int x_rows, const void* y, int y_rows, int D, const float* col_bias, int y_offset,
+                      int y_stride, const float* floor, int cand_cap, int tie_cap, float* cand_score, int* cand_idx,
+                      int* cand_count, int* status, int num_ctas, void* stream);
+int dice_filter_mask(int n, const long long* ptr, const int* cols, const long long* ab, long long ab_stride, long long num_b,
+                     const long long* keys, long long num_keys, const long long* offsets, const long long* values,
+                     unsigned int* mask, long long mask_stride, int y_rows, void* stream);
+int dice_split_rows(const float* src, long long src_stride, long long n, int d, int d_pad, void* hi, void* lo, float* copy,
+                    float* margin, float factor, void* stream);
+int dice_topk_floor(const float* gmax, int rows, int groups, int k, float* floor, int* cand_count, void* stream);
+int dice_topk_select(const float* score, const int* idx, const int* count, int rows, int cand_cap, int tie_cap, int k,
+                     float* out_s, long long* out_i, float* kth_score, int* overflow, void* stream);
+int dice_topk_scan_blocks(int B, int n);
+int dice_topk_scan(const void* q, int q_is_bf16, long long q_stride, int B, int d, const void* table, int n, int D, int k,
+                   const float* col_bias, int y_offset, int y_stride, float* part_s, int* part_i, unsigned int* done,
+                   float* out_s, long long* out_i, void* stream);
 int dice_eval_rank(const void* x, int x_rows, const void* y, int y_rows, int D, const float* target,
                    const int* target_idx, const float* col_bias, int y_offset, int y_stride, int* greater, int k,
                    int cand_cap, float* cand_score, int* cand_idx, int* cand_count, int* status, int num_ctas,

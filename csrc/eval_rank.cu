@@ -1,15 +1,15 @@
-// Fused link-prediction ranking / top-k kernel for sm_100a (tcgen05 + TMEM + TMA) and its sparse companion.
+// Link-prediction ranking: the running top-k form of the tensor-core kernel, gather-dots and the exact second pass.
 //
-// dice_eval_rank:   for queries X [x_rows, D] and entity rows Y [y_rows, D] (bf16, row-major) the tensor cores
-//                   produce S = X · Yᵀ tile by tile in TMEM; the epilogue never stores S.  It counts, per query row,
-//                   the entities whose score exceeds that row's target score (the dense part of
-//                   rank = 1 + #greater − #filtered greater) and, optionally, keeps a running top-k per row.
+// dice_eval_rank:   for queries X [x_rows, D] and entity rows Y [y_rows, D] (bf16, row-major) the tensor cores produce
+//                   S = X · Yᵀ tile by tile in TMEM; the epilogue never stores S.  With k > 0 (the kernel of this file) it
+//                   counts, per query row, the entities whose score exceeds that row's target score and keeps a running
+//                   top-k per row; every other form is a launch of the kernel in rank_tiles.cu.
 // dice_eval_sparse: gather-dots for the sparse part: the target score of each query and the number of *filtered*
 //                   entities (a CSR list per query) that beat it.
 //
-// The same CTA structure as the training kernel is used (warp 0 TMA producer, warp 1 MMA issuer, warps 2..9
-// epilogue, one persistent CTA per SM over a contiguous range of (x-tile, y-tile) pairs) but there is no second
-// GEMM, so all 512 TMEM columns hold four S buffers.  Every wait is bounded and reports through the status word.
+// CTA structure: warp 0 TMA producer, warp 1 MMA issuer, warps 2..9 epilogue, one persistent CTA per SM over a contiguous
+// range of (x-tile, y-tile) pairs; all 512 TMEM columns hold four S buffers.  Every wait is bounded and reports through the
+// status word.
 #include "dice_b200.h"
 #include "ptx_sm100.cuh"
 #include "tile_map.cuh"
@@ -38,7 +38,7 @@ struct EvalParams {
   int x_rows, y_rows, nx_tiles, ny_tiles;
   TileMap map;             // visiting order of the (x tile, y tile) pairs
   int y_offset, y_stride;  // global id of column c is y_offset + c * y_stride (contiguous or cyclic row shards)
-  // top-k (TOPK variants): every (segment, row, half) appends its k best to the row's candidate list
+  // top-k: every (segment, row, half) appends its k best to the row's candidate list
   int k;
   int cand_cap;            // capacity of a row's candidate list (entries)
   float* cand_score;       // [x_rows, cand_cap], pre-filled with -inf
@@ -46,13 +46,6 @@ struct EvalParams {
   int* cand_count;         // [x_rows], zero-initialised
   float* row_floor;        // [x_rows], pre-filled with -inf: best known lower bound of each row's k-th best score,
                            // published by finished segments so that later segments start with a tight threshold
-  // band mode (BAND variants): scores within +-margin[row] of the target are not decided here; their (row, entity)
-  // pairs are appended to a list for an exact second pass, only scores above target + margin are counted
-  const float* margin;     // [x_rows]
-  int* band_rows;          // [band_cap]
-  int* band_cols;          // [band_cap] global entity ids
-  unsigned long long* band_count;
-  long long band_cap;
 };
 
 template <int D>
@@ -68,14 +61,11 @@ __device__ __forceinline__ void atomic_max_float(float* addr, float v) {
   else atomicMin(reinterpret_cast<unsigned int*>(addr), __float_as_uint(v));
 }
 
-template <int D, int MODE>  // 0 count, 1 count + running top-k, 2 count with an undecided band, 3 collect above floor
+template <int D>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 eval_rank_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_y,
                  const EvalParams p) {
   using C = Cfg<D>;
-  constexpr bool TOPK = MODE == 1;
-  constexpr bool BAND = MODE == 2;
-  constexpr bool COLLECT = MODE == 3;  // every score >= row_floor[row] is appended to the row's candidate list
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sX = smem;
@@ -206,8 +196,8 @@ eval_rank_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     const int row = quarter * 32 + lane;
     uint32_t g = 0;
     bool ok = true;
-    float top_s[TOPK ? KMAX : 1];
-    int top_i[TOPK ? KMAX : 1];
+    float top_s[KMAX];
+    int top_i[KMAX];
 
     for (long long w = w_begin; w < w_end && ok && !*s_abort;) {
       int x, y0, run;
@@ -222,23 +212,12 @@ eval_rank_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         if (rel_id >= 0 && rel_id % p.y_stride == 0) tgt_col = rel_id / p.y_stride;
       }
       int cnt = 0;
-      float hi = tgt, lo = tgt;
-      if constexpr (BAND) {
-        const float mg = valid_x ? p.margin[x_global] : 0.f;
-        hi = tgt + mg;
-        lo = tgt - mg;
-      }
       // scores at or below `floor_s` cannot be among the row's k best: some finished segment already holds k better
       float floor_s = -CUDART_INF_F;
-      if constexpr (TOPK) {
-        if (valid_x && p.row_floor != nullptr) floor_s = p.row_floor[x_global];
-      }
-      if constexpr (COLLECT) floor_s = valid_x ? p.row_floor[x_global] : CUDART_INF_F;
+      if (valid_x && p.row_floor != nullptr) floor_s = p.row_floor[x_global];
       float thr = valid_x ? floor_s : CUDART_INF_F;
       int minpos = 0;
-      if constexpr (TOPK) {
-        for (int j = 0; j < p.k; ++j) { top_s[j] = -CUDART_INF_F; top_i[j] = -1; }
-      }
+      for (int j = 0; j < p.k; ++j) { top_s[j] = -CUDART_INF_F; top_i[j] = -1; }
 
       for (int t = 0; t < n; ++t, ++g) {
         const uint32_t b = g % NBUF;
@@ -254,25 +233,20 @@ eval_rank_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
           tmem_ld32(s_addr + col0, r);
           tc_wait_ld();
           const int rel = tgt_col - (tile_col0 + col0);  // position of the true entity inside this chunk, if any
-          uint32_t band = 0u;
           const bool plain = (col0 + 32 <= y_valid) && (p.col_bias == nullptr);
           if (plain) {
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
               const float s = __uint_as_float(r[i]);
-              cnt += (s > hi && i != rel) ? 1 : 0;
-              if constexpr (BAND) band |= ((s > lo && s <= hi && i != rel) ? 1u : 0u) << i;
-              if constexpr (COLLECT) band |= (s >= floor_s ? 1u : 0u) << i;
-              if constexpr (TOPK) {
-                if (s > thr) {
-                  top_s[minpos] = s;
-                  top_i[minpos] = p.y_offset + (tile_col0 + col0 + i) * p.y_stride;
-                  thr = top_s[0];
-                  minpos = 0;
-                  for (int j = 1; j < p.k; ++j)
-                    if (top_s[j] < thr) { thr = top_s[j]; minpos = j; }
-                  thr = fmaxf(thr, floor_s);
-                }
+              cnt += (s > tgt && i != rel) ? 1 : 0;
+              if (s > thr) {
+                top_s[minpos] = s;
+                top_i[minpos] = p.y_offset + (tile_col0 + col0 + i) * p.y_stride;
+                thr = top_s[0];
+                minpos = 0;
+                for (int j = 1; j < p.k; ++j)
+                  if (top_s[j] < thr) { thr = top_s[j]; minpos = j; }
+                thr = fmaxf(thr, floor_s);
               }
             }
           } else {
@@ -282,53 +256,15 @@ eval_rank_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
               float s = __uint_as_float(r[i]);
               if (p.col_bias != nullptr && in) s += p.col_bias[tile_col0 + col0 + i];
               if (!in) s = -CUDART_INF_F;
-              cnt += (s > hi && i != rel) ? 1 : 0;
-              if constexpr (BAND) band |= ((s > lo && s <= hi && i != rel) ? 1u : 0u) << i;
-              if constexpr (COLLECT) band |= (s >= floor_s ? 1u : 0u) << i;
-              if constexpr (TOPK) {
-                if (s > thr) {
-                  top_s[minpos] = s;
-                  top_i[minpos] = p.y_offset + (tile_col0 + col0 + i) * p.y_stride;
-                  thr = top_s[0];
-                  minpos = 0;
-                  for (int j = 1; j < p.k; ++j)
-                    if (top_s[j] < thr) { thr = top_s[j]; minpos = j; }
-                  thr = fmaxf(thr, floor_s);
-                }
-              }
-            }
-          }
-          if constexpr (COLLECT) {
-            while (band) {  // rare: the floor is the k-th best score of a sample of the table
-              const int i = __ffs(band) - 1;
-              band &= band - 1;
-              const int pos = atomicAdd(p.cand_count + x_global, 1);
-              if (pos < p.cand_cap) {
-                float s = __uint_as_float(r[0]);
-#pragma unroll
-                for (int u = 1; u < 32; ++u) s = (u == i) ? __uint_as_float(r[u]) : s;
-                if (p.col_bias != nullptr) s += p.col_bias[tile_col0 + col0 + i];
-                p.cand_score[static_cast<size_t>(x_global) * p.cand_cap + pos] = s;
-                p.cand_idx[static_cast<size_t>(x_global) * p.cand_cap + pos] =
-                    p.y_offset + (tile_col0 + col0 + i) * p.y_stride;
-              }
-            }
-          }
-          if constexpr (BAND) {
-            if (band != 0u) {  // undecided pairs of this thread's 32 columns go to the list of the exact pass
-              const int nb = __popc(band);
-              const unsigned long long base = atomicAdd(p.band_count, static_cast<unsigned long long>(nb));
-              if (static_cast<long long>(base) + nb <= p.band_cap) {
-                unsigned long long at = base;
-                while (band) {
-                  const int i = __ffs(band) - 1;
-                  band &= band - 1;
-                  p.band_rows[at] = x_global;
-                  p.band_cols[at] = p.y_offset + (tile_col0 + col0 + i) * p.y_stride;
-                  ++at;
-                }
-              } else {
-                atomicCAS(p.status, 0, ST_INBOX_OVERFLOW);
+              cnt += (s > tgt && i != rel) ? 1 : 0;
+              if (s > thr) {
+                top_s[minpos] = s;
+                top_i[minpos] = p.y_offset + (tile_col0 + col0 + i) * p.y_stride;
+                thr = top_s[0];
+                minpos = 0;
+                for (int j = 1; j < p.k; ++j)
+                  if (top_s[j] < thr) { thr = top_s[j]; minpos = j; }
+                thr = fmaxf(thr, floor_s);
               }
             }
           }
@@ -340,16 +276,14 @@ eval_rank_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
       if (!ok) break;
       if (valid_x) {
         if (p.greater != nullptr && cnt != 0) atomicAdd(p.greater + x_global, cnt);
-        if constexpr (TOPK) {
-          if (p.row_floor != nullptr && thr > floor_s) atomic_max_float(p.row_floor + x_global, thr);
-          const int pos = atomicAdd(p.cand_count + x_global, p.k);
-          if (pos + p.k <= p.cand_cap) {
-            float* cs = p.cand_score + static_cast<size_t>(x_global) * p.cand_cap + pos;
-            int* ci = p.cand_idx + static_cast<size_t>(x_global) * p.cand_cap + pos;
-            for (int j = 0; j < p.k; ++j) { cs[j] = top_s[j]; ci[j] = top_i[j]; }
-          } else {
-            atomicCAS(p.status, 0, ST_INBOX_OVERFLOW);
-          }
+        if (p.row_floor != nullptr && thr > floor_s) atomic_max_float(p.row_floor + x_global, thr);
+        const int pos = atomicAdd(p.cand_count + x_global, p.k);
+        if (pos + p.k <= p.cand_cap) {
+          float* cs = p.cand_score + static_cast<size_t>(x_global) * p.cand_cap + pos;
+          int* ci = p.cand_idx + static_cast<size_t>(x_global) * p.cand_cap + pos;
+          for (int j = 0; j < p.k; ++j) { cs[j] = top_s[j]; ci[j] = top_i[j]; }
+        } else {
+          atomicCAS(p.status, 0, ST_INBOX_OVERFLOW);
         }
       }
       w += n;
@@ -366,10 +300,10 @@ eval_rank_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
   }
 }
 
-template <int D, int MODE>
+template <int D>
 static int launch(const CUtensorMap& tx, const CUtensorMap& ty, const EvalParams& p, int num_ctas,
                   cudaStream_t stream) {
-  auto kern = eval_rank_kernel<D, MODE>;
+  auto kern = eval_rank_kernel<D>;
   static bool configured[64] = {false};   // the attribute is per device: one flag per device ordinal
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -3;
@@ -493,6 +427,16 @@ extern "C" int dice_eval_rank(const void* x, int x_rows, const void* y, int y_ro
   if (k < -1 || k > KMAX) return -7;   // k == -1: collect mode (every score >= row_floor goes to the candidate lists)
   if (k != 0 && (cand_score == nullptr || cand_idx == nullptr || cand_count == nullptr || cand_cap < k)) return -7;
   if (k == -1 && row_floor == nullptr) return -7;
+  if (margin != nullptr && (k > 0 || band_rows == nullptr || band_cols == nullptr || band_count == nullptr)) return -7;
+  if (k == -1)
+    return dice_rank_collect(x, x_rows, y, y_rows, D, col_bias, y_offset, y_stride, row_floor, cand_cap, 0, cand_score, cand_idx,
+                             cand_count, status, num_ctas, stream);
+  if (k == 0) {
+    if (D != 64 && D != 128 && D != 256) return -6;
+    if (target == nullptr || greater == nullptr) return 0;   // nothing can be counted
+    return dice_rank_count(x, nullptr, x_rows, y, nullptr, y_rows, D, target, target_idx, col_bias, y_offset, y_stride, nullptr, 0,
+                           greater, margin, band_rows, band_cols, band_count, band_cap, status, num_ctas, stream);
+  }
   CUtensorMap tx, ty;
   int rc = make_tmap_bf16(&tx, x, x_rows, D);
   if (rc) return rc;
@@ -517,12 +461,6 @@ extern "C" int dice_eval_rank(const void* x, int x_rows, const void* y, int y_ro
   p.cand_idx = cand_idx;
   p.cand_count = cand_count;
   p.row_floor = row_floor;
-  p.margin = margin;
-  p.band_rows = band_rows;
-  p.band_cols = band_cols;
-  p.band_count = band_count;
-  p.band_cap = band_cap;
-  if (margin != nullptr && (k > 0 || band_rows == nullptr || band_cols == nullptr || band_count == nullptr)) return -7;
   if (num_ctas <= 0) {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
@@ -532,17 +470,10 @@ extern "C" int dice_eval_rank(const void* x, int x_rows, const void* y, int y_ro
   const long long total = static_cast<long long>(p.nx_tiles) * p.ny_tiles;
   if (num_ctas > total) num_ctas = static_cast<int>(total);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int mode = k > 0 ? 1 : (k == -1 ? 3 : (margin != nullptr ? 2 : 0));
-#define DICE_EVAL_DISPATCH(DD)                                              \
-  case DD:                                                                  \
-    if (mode == 1) return launch<DD, 1>(tx, ty, p, num_ctas, s);            \
-    if (mode == 2) return launch<DD, 2>(tx, ty, p, num_ctas, s);            \
-    if (mode == 3) return launch<DD, 3>(tx, ty, p, num_ctas, s);            \
-    return launch<DD, 0>(tx, ty, p, num_ctas, s);
   switch (D) {
-    DICE_EVAL_DISPATCH(256)
-    DICE_EVAL_DISPATCH(128)
-    DICE_EVAL_DISPATCH(64)
+    case 256: return launch<256>(tx, ty, p, num_ctas, s);
+    case 128: return launch<128>(tx, ty, p, num_ctas, s);
+    case 64: return launch<64>(tx, ty, p, num_ctas, s);
     default: return -6;
   }
 }

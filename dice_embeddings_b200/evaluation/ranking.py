@@ -21,6 +21,9 @@ import torch
 from ..data.vocab import PairCSR
 
 ALL_HITS_RANGE = list(range(1, 11))
+#: largest mask of known answers per batch for which a CSR vocabulary is turned into bits without looking at its lists: below
+#: this the mask costs less than gathering the lists of the batch (4096 queries against 131 072 entities)
+MASK_BYTES = 64 << 20
 
 
 def metrics_from_ranks(ranks: torch.Tensor, divisor: Optional[float] = None,
@@ -98,9 +101,30 @@ def fused_tail_ranks(model, triples: torch.Tensor, er_vocab, batch_size: int = 4
     from ..ops.kernels import KernelError
     ranker = ranker or eval_rank.ranker_for_model(model)
     dev = ranker.device
+    n = triples.shape[0]
+    if n == 0:
+        return torch.zeros(0, dtype=torch.long)
+    triples = triples.to(dev)
+    # a vocabulary in CSR form is looked up on the device, as bits of a mask; the batches are only queued, and one copy at
+    # the end waits for all of them
+    if isinstance(er_vocab, PairCSR) and len(er_vocab) > 0 and ranker.group is None and ranker.y_stride == 1 \
+            and ranker.y_offset == 0 and min(batch_size, n) * ranker._mask_words() * 4 <= MASK_BYTES:
+        keys, offsets, values = er_vocab.tensors(dev)
+        ranks = torch.empty(n, dtype=torch.int64, device=dev)
+        for i in range(0, n, batch_size):
+            b = triples[i:i + batch_size]
+            q, _ = eval_rank.model_queries(model, b[:, :2])
+            ranks[i:i + batch_size] = ranker.ranks_of_pairs(q, b[:, 2], b, er_vocab.num_b, keys, offsets, values)
+        ranks = ranks.cpu()
+        try:
+            ranker.check()
+            return ranks
+        except KernelError:     # the band list of some batch ran full: batch by batch below
+            if not ranker.exact:
+                raise
     out = []
-    for i in range(0, triples.shape[0], batch_size):
-        b = triples[i:i + batch_size].to(dev)
+    for i in range(0, n, batch_size):
+        b = triples[i:i + batch_size]
         q, _ = eval_rank.model_queries(model, b[:, :2])
         ptr, cols = filter_csr(er_vocab, b[:, 0], b[:, 1])
         try:
@@ -116,7 +140,7 @@ def fused_tail_ranks(model, triples: torch.Tensor, er_vocab, batch_size: int = 4
             finally:
                 ranker.exact = True
         out.append(r)
-    return torch.cat(out) if out else torch.zeros(0, dtype=torch.long)
+    return torch.cat(out)
 
 
 @torch.no_grad()

@@ -130,6 +130,15 @@ class _Sigs:
     dice_sampled_grad = [_i, _i, _i, _p, _p, _l, _p, _l, _p, _p, _i, _i, ctypes.c_ulonglong, ctypes.c_ulonglong, _p, _f, _f, _p, _p, _p, _p, _p, _p, _l, _p, _p, _l, _p, _p, _p, _f, _f, _f, _i, _p, _p]
     dice_sampled_update = [_i, _i, _p, _p, _p, _p, _p, _p, _p, _p, _l, _i, _i, _i, _p, _p, _p, _p, _l, _p, _p, _p, _p, _l, _f, _f, _f, _f, _f, _p, _p, _p, _p, _p]
     dice_sparse_rows_optimizer = [_i, _p, _p, _p, _p, _p, _p, _l, _i, _p, _f, _f, _f, _f, _f, _p]
+    dice_rank_count = [_p, _p, _i, _p, _p, _i, _i, _p, _p, _p, _i, _i, _p, _l, _p, _p, _p, _p, _p, _l, _p, _i, _p]
+    dice_rank_group_max = [_p, _i, _p, _i, _i, _p, _p, _i, _p, _i, _p]
+    dice_rank_collect = [_p, _i, _p, _i, _i, _p, _i, _i, _p, _i, _i, _p, _p, _p, _p, _i, _p]
+    dice_filter_mask = [_i, _p, _p, _p, _l, _l, _p, _l, _p, _p, _p, _l, _i, _p]
+    dice_split_rows = [_p, _l, _l, _i, _i, _p, _p, _p, _p, _f, _p]
+    dice_topk_floor = [_p, _i, _i, _i, _p, _p, _p]
+    dice_topk_select = [_p, _p, _p, _i, _i, _i, _i, _p, _p, _p, _p, _p]
+    dice_topk_scan_blocks = [_i, _i]
+    dice_topk_scan = [_p, _i, _l, _i, _i, _p, _i, _i, _i, _p, _i, _i, _p, _p, _p, _p, _p, _p]
     dice_eval_rank = [_p, _i, _p, _i, _i, _p, _p, _p, _i, _i, _p, _i, _i, _p, _p, _p, _p, _i, _p, _p, _p, _p, _l, _p, _p]
     dice_eval_rank_cand_cap = [_i, _i, _i, _i, _i]
     dice_conv_gate_supported = [_i, _i, _i, _i]

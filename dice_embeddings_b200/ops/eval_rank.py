@@ -1,8 +1,9 @@
 """Filtered ranking and top-k over an entity table without materialising the score matrix.
 
 ``rank = 1 + #{j : s_j > s_target} − #{j ∈ known answers, j ≠ target : s_j > s_target}``: the dense count comes
-from the tcgen05 kernel ``dice_eval_rank`` (GEMM tiles in TMEM, counting epilogue), the target score and the
-filtered count from gather-dots (``dice_eval_sparse``).  With a process group every rank holds a row shard of the
+from the tcgen05 kernel ``dice_rank_count`` (GEMM tiles in TMEM, counting epilogue), which leaves out the known answers
+through a bit mask where that is cheaper; otherwise they are counted by gather-dots (``dice_eval_sparse``), like the target
+scores.  With a process group every rank holds a row shard of the
 table (contiguous or cyclic); target scores, counts and top-k candidates are merged across ranks by merge kernels that
 read the ranks' buffers in a symmetric heap through peer loads, ordered by the bounded device barrier: the hot loop
 holds no library collective and no host round trip.
@@ -47,32 +48,32 @@ class FusedRanker:
 
     def __init__(self, table: torch.Tensor, col_bias: Optional[torch.Tensor] = None, y_offset: int = 0,
                  y_stride: int = 1, group=None, exact: bool = False, band_capacity: int = 1 << 24):
-        """``exact``: ranks equal those of an fp32 scoring of the same operands.  The tensor cores still do the bulk
-        of the work on bf16-rounded operands; a score can differ from its fp32 value by at most
-        ``2^-8 · ‖q‖ · ‖e‖``, so only entities whose bf16 score lies within that margin of the target are undecided,
-        and exactly those (typically a fraction of a percent) are re-scored in fp32 by a second, sparse pass."""
+        """``exact``: ranks equal those of an fp32 scoring of the same operands.  The tensor cores still do the bulk of the
+        work, on operands split into two bf16 terms each; such a score differs from its fp32 value by at most
+        ``MARGIN[d] · ‖q‖ · ‖e‖``, so only entities within that margin of the target are undecided, and exactly those
+        (well below a tenth of a percent) are re-scored in fp32 by a second, sparse pass."""
         assert table.is_cuda, "the fused ranker runs on a CUDA device"
         self.d = table.shape[1]
         self.d_pad = pad_dim(self.d)
         if self.d_pad is None:
             raise ValueError(f"embedding width {self.d} exceeds the kernel's limit of {SUPPORTED_D[-1]}")
-        self.table = to_kernel_operand(table, self.d_pad)
         self.exact = bool(exact)
         if self.exact:
             t32 = table.detach().float()
-            if self.d != self.d_pad:
-                t32 = torch.nn.functional.pad(t32, (0, self.d_pad - self.d))
-            self.table_f32 = t32.contiguous()
+            self.table, self.table_lo, copy, _ = kernels.split_rows(t32, self.d_pad, want_copy=self.d != self.d_pad)
+            self.table_f32 = copy if copy is not None else t32.contiguous()
             self.row_norm_max = float(self.table_f32.norm(dim=1).max()) if table.shape[0] else 0.0
             self.band_rows = torch.empty(band_capacity, dtype=torch.int32, device=table.device)
             self.band_cols = torch.empty(band_capacity, dtype=torch.int32, device=table.device)
-            self.band_count = torch.zeros(1, dtype=torch.int64, device=table.device)
+        else:
+            self.table = to_kernel_operand(table, self.d_pad)
         self.col_bias = None if col_bias is None else col_bias.detach().float().contiguous()
         self.y_offset, self.y_stride, self.group = int(y_offset), int(y_stride), group
         self.device = table.device
         self._flags = torch.zeros(2, dtype=torch.int32, device=self.device)
         self.status = self._flags[0:1]      # kernel status word
         self.overflow = self._flags[1:2]    # set when a top-k candidate list ran full
+        self._scan_done = {}
         self.W, self.rank = 1, 0
         self._heap = None
         if group is not None:
@@ -126,13 +127,52 @@ class FusedRanker:
             raise kernels.KernelError("a top-k candidate list ran full: the table prefix used for the threshold was "
                                       "not representative; call topk again with a smaller batch")
 
+    #: relative error of a split score for each padded width: the terms left out of (hi + lo)(hi + lo) are at most
+    #: 3 · 2^-16, the accumulation of 3 d products and of the fp32 reference at most 4 d · 2^-23
+    MARGIN = {d: 3 * 2.0 ** -16 + 4 * d * 2.0 ** -23 for d in SUPPORTED_D}
+    #: largest bit mask of known answers (bytes); beyond it the known answers are scored one by one
+    MASK_LIMIT = 512 << 20
+
+    def _mask_words(self) -> int:
+        return (self.table.shape[0] + 127) // 128 * 4
+
+    def _mask_pays(self, B: int, entries: int) -> bool:
+        """A bit mask of the known answers costs clearing, setting and reading ``B · |E| / 8`` bytes; scoring them one by
+        one reads a row of the table for each.  Queries of a popular pair have thousands of known answers, and the warps
+        that walked them took 10 of the 21 ms of an evaluation of 20 466 queries against 14 541 entities; with 16 answers
+        per query against two million rows the lists cost 41 us and the mask would be 2 GB."""
+        mask = B * self._mask_words() * 4
+        row = self.d_pad * (4 if self.exact else 2)
+        return self.group is None and mask <= self.MASK_LIMIT and entries * row > 4 * mask
+
     @torch.no_grad()
     def ranks(self, q: torch.Tensor, target: torch.Tensor, filt_ptr: Optional[torch.Tensor] = None,
               filt_cols: Optional[torch.Tensor] = None) -> torch.Tensor:
         """Filtered ranks ``[B]`` (int64) of entity ``target[i]`` for query vector ``q[i]``.  The filter of query
         ``i`` is ``filt_cols[filt_ptr[i]:filt_ptr[i+1]]`` (global entity ids; the target itself is ignored)."""
         B = q.shape[0]
-        qk = to_kernel_operand(q, self.d_pad)
+        mask = None
+        if filt_ptr is not None:
+            filt_ptr = filt_ptr.to(torch.int64).contiguous()
+            filt_cols = filt_cols.to(torch.int32).contiguous()
+            if self.y_offset == 0 and self.y_stride == 1 and self._mask_pays(B, filt_cols.numel()):
+                mask = torch.zeros(B, self._mask_words(), dtype=torch.int32, device=self.device)
+                kernels.filter_mask(mask, self.table.shape[0], ptr=filt_ptr, cols=filt_cols)
+                filt_ptr = filt_cols = None
+        return self._ranks(q, target, filt_ptr, filt_cols, mask)
+
+    @torch.no_grad()
+    def ranks_of_pairs(self, q: torch.Tensor, target: torch.Tensor, ab: torch.Tensor, num_b: int, keys: torch.Tensor,
+                       offsets: torch.Tensor, values: torch.Tensor) -> torch.Tensor:
+        """:meth:`ranks` with the filter of query ``i`` given as the pair in the first two columns of ``ab[i]``, looked up on
+        the device in a CSR over sorted keys ``a * num_b + b`` (whole table on this device)."""
+        assert self.group is None and self.y_offset == 0 and self.y_stride == 1
+        mask = torch.zeros(q.shape[0], self._mask_words(), dtype=torch.int32, device=self.device)
+        kernels.filter_mask(mask, self.table.shape[0], ab=ab, num_b=num_b, keys=keys, offsets=offsets, values=values)
+        return self._ranks(q, target, None, None, mask)
+
+    def _ranks(self, q, target, filt_ptr, filt_cols, mask) -> torch.Tensor:
+        B = q.shape[0]
         tgt_idx = target.to(torch.int32).contiguous()
         sharded = self.group is not None
         if sharded:   # partial results live in the symmetric heap, where the merge kernels of every rank read them
@@ -143,33 +183,36 @@ class FusedRanker:
         else:
             tgt_part = tgt_score = torch.zeros(B, dtype=torch.float32, device=self.device)
             greater = torch.zeros(B, dtype=torch.int32, device=self.device)
-            filtered = torch.zeros(B, dtype=torch.int32, device=self.device)
-        if filt_ptr is not None:
-            filt_ptr = filt_ptr.to(torch.int64).contiguous()
-            filt_cols = filt_cols.to(torch.int32).contiguous()
+            filtered = torch.zeros(B, dtype=torch.int32, device=self.device) if filt_ptr is not None else None
+        kw = dict(col_bias=self.col_bias, y_offset=self.y_offset, y_stride=self.y_stride)
+        band = {}
         if self.exact:
-            return self._ranks_exact(q, qk, tgt_idx, tgt_part, tgt_score, greater, filtered, filt_ptr, filt_cols)
+            # target scores and filtered counts from the fp32 operands, dense counts from the split ones
+            q32 = q.detach().float()
+            qk, q_lo, copy, margin = kernels.split_rows(q32, self.d_pad, want_copy=self.d != self.d_pad,
+                                                        margin_factor=self.row_norm_max * self.MARGIN[self.d_pad])
+            qs, table = copy if copy is not None else q32.contiguous(), self.table_f32
+            band_count = torch.zeros(1, dtype=torch.int64, device=self.device)
+            band = dict(x_lo=q_lo, y_lo=self.table_lo, margin=margin, band_rows=self.band_rows, band_cols=self.band_cols,
+                        band_count=band_count)
+        else:
+            qk = to_kernel_operand(q, self.d_pad)
+            qs, table = qk, self.table
         if sharded:  # phase 1: owners score their targets, phase 2: everybody counts against the merged scores
-            kernels.eval_sparse(qk, self.table, tgt_idx, tgt_part, None, col_bias=self.col_bias,
-                                y_offset=self.y_offset, y_stride=self.y_stride)
+            kernels.eval_sparse(qs, table, tgt_idx, tgt_part, None, **kw)
             self._barrier()
             kernels.peer_sum_f32(self._tab["tgt"], self.W, tgt_score, B, self.status)
             greater.zero_()
             filtered.zero_()
             if filt_ptr is not None:
-                kernels.eval_sparse(qk, self.table, tgt_idx, None, filtered, filt_ptr, filt_cols,
-                                    col_bias=self.col_bias, target_in=tgt_score, y_offset=self.y_offset,
-                                    y_stride=self.y_stride)
+                kernels.eval_sparse(qs, table, tgt_idx, None, filtered, filt_ptr, filt_cols, target_in=tgt_score, **kw)
         else:
-            kernels.eval_sparse(qk, self.table, tgt_idx, tgt_score, filtered if filt_ptr is not None else None,
-                                filt_ptr, filt_cols, col_bias=self.col_bias)
-        kernels.eval_rank(qk, self.table, tgt_score, tgt_idx, greater, self.status, col_bias=self.col_bias,
-                          y_offset=self.y_offset, y_stride=self.y_stride)
-        return self._finish_ranks(greater, filtered, B)
-
-    def _finish_ranks(self, greater, filtered, B: int) -> torch.Tensor:
+            kernels.eval_sparse(qs, table, tgt_idx, tgt_score, filtered, filt_ptr, filt_cols, **kw)
+        kernels.rank_count(qk, self.table, tgt_score, tgt_idx, greater, self.status, mask=mask, **band, **kw)
+        if self.exact:
+            kernels.eval_band_exact(qs, table, self.band_rows, self.band_cols, band_count, tgt_score, greater, **kw)
         if self.group is None:
-            return (1 + greater - filtered).long()
+            return (greater.add_(1) if filtered is None else 1 + greater - filtered).long()
         out = torch.empty(B, dtype=torch.int64, device=self.device)
         self._barrier()                       # every rank's counts are complete
         kernels.merge_ranks(self._tab["greater"], self._tab["filtered"], self.W, out, B, self.status)
@@ -179,93 +222,63 @@ class FusedRanker:
     TWO_STAGE_ROWS = 131072
     SAMPLE_ROWS = 32768
 
-    def _running_topk(self, qk: torch.Tensor, table: torch.Tensor, kk: int, col_bias):
-        """Per-segment running top-k lists in the kernel + merge: right for small tables (every thread keeps its own
-        list, which costs a warm-up per segment)."""
-        B = qk.shape[0]
-        cap = kernels.eval_rank_cand_cap(B, table.shape[0], self.d_pad, kk)
-        cs = torch.full((B, cap), float("-inf"), dtype=torch.float32, device=self.device)
-        ci = torch.full((B, cap), -1, dtype=torch.int32, device=self.device)
-        cc = torch.zeros(B, dtype=torch.int32, device=self.device)
-        floor = torch.full((B,), float("-inf"), dtype=torch.float32, device=self.device)
-        kernels.eval_rank(qk, table, None, None, None, self.status, col_bias=col_bias, y_offset=self.y_offset,
-                          y_stride=self.y_stride, k=kk, cand_score=cs, cand_idx=ci, cand_count=cc, row_floor=floor)
-        sc, pos = torch.topk(cs, kk, dim=1)
-        return sc, torch.gather(ci, 1, pos).long()
+    #: queries per pass: bounds the group maxima (16 KB per query at 131 072 rows)
+    TOPK_QUERIES = 8192
 
-    def _topk_local(self, qk: torch.Tensor, kk: int):
-        n_local = self.table.shape[0]
+    def _done(self) -> torch.Tensor:
+        """Block counter of the scan: calls on one stream follow one another, so there is one per stream."""
+        if not torch.cuda.is_current_stream_capturing():
+            key = torch.cuda.current_stream(self.device).cuda_stream
+            if key in self._scan_done:
+                return self._scan_done[key]
+            if len(self._scan_done) < 64:
+                self._scan_done[key] = torch.zeros(1, dtype=torch.int32, device=self.device)
+                return self._scan_done[key]
+        return torch.zeros(1, dtype=torch.int32, device=self.device)
+
+    def _topk_local(self, q: torch.Tensor, kk: int):
+        n_local, B = self.table.shape[0], q.shape[0]
+        kw = dict(col_bias=self.col_bias, y_offset=self.y_offset, y_stride=self.y_stride)
+        # up to four queries: one launch that reads the table once on the ordinary cores.  Everything else goes through the
+        # tensor cores, where a tile costs the same for 1 query as for 128.
+        if kk and B and q.dtype in (torch.float32, torch.bfloat16) and q.stride(1) == 1 and kernels.topk_scan_blocks(B, n_local):
+            return kernels.topk_scan(q, self.table, kk, self._done(), **kw)
+        if B > self.TOPK_QUERIES:
+            parts = [self._topk_local(q[i:i + self.TOPK_QUERIES], kk) for i in range(0, B, self.TOPK_QUERIES)]
+            return torch.cat([p[0] for p in parts]), torch.cat([p[1] for p in parts])
+        if kk == 0 or B == 0:
+            return (torch.empty(B, kk, dtype=torch.float32, device=self.device),
+                    torch.empty(B, kk, dtype=torch.int64, device=self.device))
+        qk = to_kernel_operand(q, self.d_pad)
         if n_local <= self.TWO_STAGE_ROWS:
-            return self._running_topk(qk, self.table, kk, self.col_bias)
+            return kernels.topk_bounded(qk, self.table, kk, self.status, self.overflow, **kw)
         # stage 1: the k-th best score over a sample of the table is a lower bound of the k-th best overall.  The
         # sample takes every (n / S)-th row, so it is representative whatever the order of the rows (a prefix of a
         # table sorted by norm would not be); it is copied once per ranker.
         S = self.SAMPLE_ROWS
         if getattr(self, "_sample", None) is None:
             step = max(n_local // S, 1)
-            self._sample = self.table[::step][:S].contiguous()
             self._sample_bias = None if self.col_bias is None else self.col_bias[::step][:S].contiguous()
-        sc_s, _ = self._running_topk(qk, self._sample, kk, self._sample_bias)
-        floor = sc_s[:, kk - 1].contiguous()
-        # stage 2: one pass over the whole table that appends every score >= floor (few per row) to the row's list
-        B = qk.shape[0]
-        cap = int(8 * kk * (n_local / S) + 64)
-        cs = torch.full((B, cap), float("-inf"), dtype=torch.float32, device=self.device)
-        ci = torch.full((B, cap), -1, dtype=torch.int32, device=self.device)
-        cc = torch.zeros(B, dtype=torch.int32, device=self.device)
-        kernels.eval_rank(qk, self.table, None, None, None, self.status, col_bias=self.col_bias,
-                          y_offset=self.y_offset, y_stride=self.y_stride, k=-1, cand_score=cs, cand_idx=ci,
-                          cand_count=cc, row_floor=floor)
-        # a list that ran full (prefix not representative of the table, e.g. rows sorted by norm) is recorded on the
-        # device and reported by check(); nothing here waits for the GPU
-        self.overflow.logical_or_((cc > cap).any().view(1))
-        sc, pos = torch.topk(cs, kk, dim=1)
-        return sc, torch.gather(ci, 1, pos).long()
-
-    def _ranks_exact(self, q, qk, tgt_idx, tgt_part, tgt_score, greater, filtered, filt_ptr, filt_cols) -> torch.Tensor:
-        q32 = q.detach().float()
-        if self.d != self.d_pad:
-            q32 = torch.nn.functional.pad(q32, (0, self.d_pad - self.d))
-        q32 = q32.contiguous()
-        kw = dict(col_bias=self.col_bias, y_offset=self.y_offset, y_stride=self.y_stride)
-        sharded = self.group is not None
-        # exact target scores and exact filtered counts from the fp32 operands
-        kernels.eval_sparse(q32, self.table_f32, tgt_idx, tgt_part, None if sharded else
-                            (filtered if filt_ptr is not None else None), None if sharded else filt_ptr,
-                            None if sharded else filt_cols, **kw)
-        emax = self.row_norm_max
-        if sharded:
-            self._barrier()
-            kernels.peer_sum_f32(self._tab["tgt"], self.W, tgt_score, q.shape[0], self.status)
-            greater.zero_()
-            filtered.zero_()
-            if filt_ptr is not None:
-                kernels.eval_sparse(q32, self.table_f32, tgt_idx, None, filtered, filt_ptr, filt_cols,
-                                    target_in=tgt_score, **kw)
-        # |bf16 score - fp32 score| <= 2^-8 (1 + 2^-9) |q| |e|; a little head room for the fp32 accumulation orders
-        margin = (q32.norm(dim=1) * (emax * 2.0 ** -8 * 1.01) + 1e-30).contiguous()
-        self.band_count.zero_()
-        kernels.eval_rank(qk, self.table, tgt_score, tgt_idx, greater, self.status, margin=margin,
-                          band_rows=self.band_rows, band_cols=self.band_cols, band_count=self.band_count, **kw)
-        kernels.eval_band_exact(q32, self.table_f32, self.band_rows, self.band_cols, self.band_count, tgt_score,
-                                greater, **kw)
-        return self._finish_ranks(greater, filtered, q.shape[0])
+            self._sample = self.table[::step][:S].contiguous()
+        floor = kernels.topk_bounded(qk, self._sample, kk, self.status, self.overflow, col_bias=self._sample_bias, kth_only=True)
+        # stage 2: one pass over the whole table that collects what reaches the bound (few per row).  A list that ran full
+        # (sample not representative of the table) is recorded on the device and reported by check()
+        return kernels.topk_bounded(qk, self.table, kk, self.status, self.overflow, floor=floor,
+                                    cand_cap=int(8 * kk * (n_local / S) + 64), **kw)
 
     @torch.no_grad()
     def topk(self, q: torch.Tensor, k: int) -> Tuple[torch.Tensor, torch.Tensor]:
         """``(scores [B, k], entity ids [B, k])`` of the best entities per query, best first."""
-        B = q.shape[0]
         n_local = self.table.shape[0]
-        qk = to_kernel_operand(q, self.d_pad)
         if k > 32:  # beyond the in-kernel list: plain matmul in slices (rare; interactive use)
-            s = qk.float() @ self.table.float().t()
+            s = to_kernel_operand(q, self.d_pad).float() @ self.table.float().t()
             if self.col_bias is not None:
                 s = s + self.col_bias
             sc, ix = torch.topk(s, min(k, n_local), dim=1)
             ix = ix * self.y_stride + self.y_offset
         else:
             kk = min(k, n_local)
-            sc, ix = self._topk_local(qk, kk)
+            sc, ix = self._topk_local(q.detach(), kk)
         if self.group is not None:
             sc, ix = self._merge_topk(sc, ix, k)
         return sc, ix

@@ -556,6 +556,145 @@ def eval_rank(x: torch.Tensor, y: torch.Tensor, target: Optional[torch.Tensor], 
                   band_rows, band_cols, band_count, row_floor))
 
 
+def rank_count(x: torch.Tensor, y: torch.Tensor, target: torch.Tensor, target_idx: Optional[torch.Tensor],
+               greater: torch.Tensor, status: torch.Tensor, col_bias: Optional[torch.Tensor] = None, y_offset: int = 0,
+               y_stride: int = 1, mask: Optional[torch.Tensor] = None, x_lo: Optional[torch.Tensor] = None,
+               y_lo: Optional[torch.Tensor] = None, margin: Optional[torch.Tensor] = None,
+               band_rows: Optional[torch.Tensor] = None, band_cols: Optional[torch.Tensor] = None,
+               band_count: Optional[torch.Tensor] = None, num_ctas: int = 0) -> None:
+    """Counting form of the ranking kernel: like :func:`eval_rank` with ``k = 0``, plus a bit ``mask [x_rows, words]`` of
+    columns to leave out and, in the band form, the second bf16 terms ``x_lo`` / ``y_lo`` of the operands."""
+    for n, t in (("x", x), ("y", y), ("x_lo", x_lo), ("y_lo", y_lo)):
+        if t is not None:
+            _req(t, torch.bfloat16, n)
+    assert x.shape[1] == y.shape[1] and (x_lo is None or x_lo.shape == x.shape) and (y_lo is None or y_lo.shape == y.shape)
+    _req(target, torch.float32, "target")
+    _req(greater, torch.int32, "greater")
+    if target_idx is not None:
+        _req(target_idx, torch.int32, "target_idx")
+    if col_bias is not None:
+        _req(col_bias, torch.float32, "col_bias")
+    if mask is not None:
+        _req(mask, torch.int32, "mask")
+        assert mask.shape[0] >= x.shape[0] and mask.shape[1] * 32 >= y.shape[0]
+    if margin is not None:
+        _req(margin, torch.float32, "margin")
+    _call("dice_rank_count", x, _ptr(x), _ptr(x_lo), x.shape[0], _ptr(y), _ptr(y_lo), y.shape[0], x.shape[1], _ptr(target),
+          _ptr(target_idx), _ptr(col_bias), int(y_offset), int(y_stride), _ptr(mask), 0 if mask is None else mask.shape[1],
+          _ptr(greater), _ptr(margin), _ptr(band_rows), _ptr(band_cols), _ptr(band_count),
+          0 if band_rows is None else band_rows.numel(), _ptr(status), int(num_ctas),
+          others=(y, x_lo, y_lo, target, target_idx, greater, status, col_bias, mask, margin, band_rows, band_cols, band_count))
+
+
+def filter_mask(mask: torch.Tensor, y_rows: int, ptr: Optional[torch.Tensor] = None, cols: Optional[torch.Tensor] = None,
+                ab: Optional[torch.Tensor] = None, num_b: int = 0, keys: Optional[torch.Tensor] = None,
+                offsets: Optional[torch.Tensor] = None, values: Optional[torch.Tensor] = None) -> None:
+    """Set the bits of the known answers of every query in ``mask`` (cleared by the caller): of the CSR ``ptr`` / ``cols``
+    over the batch, or of the pairs in the first two columns of ``ab`` looked up in ``keys`` / ``offsets`` / ``values``
+    (``key = a * num_b + b``, ascending)."""
+    _req(mask, torch.int32, "mask")
+    if ptr is not None:
+        _req(ptr, torch.int64, "ptr")
+        _req(cols, torch.int32, "cols")
+        n = ptr.numel() - 1
+        if cols.numel() == 0:
+            return
+    else:
+        assert ab.dtype == torch.int64 and ab.stride(1) == 1 and ab.shape[1] >= 2
+        for t, name in ((keys, "keys"), (offsets, "offsets"), (values, "values")):
+            _req(t, torch.int64, name)
+        n = ab.shape[0]
+    assert mask.shape[0] >= n
+    _call("dice_filter_mask", mask, n, _ptr(ptr), _ptr(cols), _ptr(ab), 0 if ab is None else ab.stride(0), int(num_b),
+          _ptr(keys), 0 if keys is None else keys.numel(), _ptr(offsets), _ptr(values), _ptr(mask), mask.shape[1], int(y_rows),
+          others=(ptr, cols, ab, keys, offsets, values))
+
+
+def split_rows(src: torch.Tensor, d_pad: int, want_copy: bool = False, margin_factor: Optional[float] = None):
+    """``(hi, lo, copy, margin)`` of fp32 rows: two bf16 terms and (optionally) the fp32 rows, zero-padded to ``d_pad``
+    columns, and ``margin = |row| * margin_factor``."""
+    assert src.is_cuda and src.dtype == torch.float32 and src.dim() == 2
+    if src.stride(1) != 1:
+        src = src.contiguous()
+    n, d = src.shape
+    hi = torch.empty(n, d_pad, dtype=torch.bfloat16, device=src.device)
+    lo = torch.empty_like(hi)
+    copy = torch.empty(n, d_pad, dtype=torch.float32, device=src.device) if want_copy else None
+    margin = None if margin_factor is None else torch.empty(n, dtype=torch.float32, device=src.device)
+    _call("dice_split_rows", src, _ptr(src), src.stride(0), n, d, int(d_pad), _ptr(hi), _ptr(lo), _ptr(copy), _ptr(margin),
+          0.0 if margin_factor is None else float(margin_factor))
+    return hi, lo, copy, margin
+
+
+#: largest k of the selection kernels
+TOPK_MAX = 32
+
+
+def topk_bounded(x: torch.Tensor, y: torch.Tensor, k: int, status: torch.Tensor, overflow: torch.Tensor,
+                 col_bias: Optional[torch.Tensor] = None, y_offset: int = 0, y_stride: int = 1,
+                 floor: Optional[torch.Tensor] = None, cand_cap: Optional[int] = None, kth_only: bool = False):
+    """Best ``k <= 32`` columns of ``x yᵀ`` per row, ``(scores [B, k], ids [B, k])``, best first.  A first pass keeps the
+    largest score of every 32 columns; the k-th largest of those is a score that k columns reach, and a second pass
+    collects what reaches it: at most 32 (k - 1) columns above it, so the lists cannot overflow.  With ``floor`` (a lower
+    bound of each row's k-th best from elsewhere) the first pass is left out and the lists have room for ``cand_cap``
+    scores above it (*overflow* is set where that was not enough).  ``kth_only`` returns the k-th best scores alone."""
+    _req(x, torch.bfloat16, "x")
+    _req(y, torch.bfloat16, "y")
+    if col_bias is not None:
+        _req(col_bias, torch.float32, "col_bias")
+    B, D, n, dev = x.shape[0], x.shape[1], y.shape[0], x.device
+    assert 1 <= k <= min(TOPK_MAX, n) and y.shape[1] == D
+    count = torch.empty(B, 2, dtype=torch.int32, device=dev) if floor is None else torch.zeros(B, 2, dtype=torch.int32, device=dev)
+    if floor is None:
+        groups = 4 * ((n + 127) // 128)
+        gmax = torch.empty(B, groups, dtype=torch.float32, device=dev)
+        _call("dice_rank_group_max", x, _ptr(x), B, _ptr(y), n, D, _ptr(col_bias), _ptr(gmax), groups, _ptr(status), 0,
+              others=(y, col_bias, status))
+        floor = torch.empty(B, dtype=torch.float32, device=dev)
+        _call("dice_topk_floor", gmax, _ptr(gmax), B, groups, int(k), _ptr(floor), _ptr(count))
+        cand_cap = 32 * k
+    cs = torch.empty(B, cand_cap + k, dtype=torch.float32, device=dev)
+    ci = torch.empty(B, cand_cap + k, dtype=torch.int32, device=dev)
+    _call("dice_rank_collect", x, _ptr(x), B, _ptr(y), n, D, _ptr(col_bias), int(y_offset), int(y_stride), _ptr(floor),
+          int(cand_cap), int(k), _ptr(cs), _ptr(ci), _ptr(count), _ptr(status), 0, others=(y, col_bias, floor, status))
+    sc = ix = kth = None
+    if kth_only:
+        kth = torch.empty(B, dtype=torch.float32, device=dev)
+    else:
+        sc = torch.empty(B, k, dtype=torch.float32, device=dev)
+        ix = torch.empty(B, k, dtype=torch.int64, device=dev)
+    _call("dice_topk_select", cs, _ptr(cs), _ptr(ci), _ptr(count), B, int(cand_cap), int(k), int(k), _ptr(sc), _ptr(ix),
+          _ptr(kth), _ptr(overflow), others=(overflow,))
+    return kth if kth_only else (sc, ix)
+
+
+def topk_scan_blocks(B: int, n: int) -> int:
+    """Blocks of :func:`topk_scan` for this shape; 0 where that path does not apply."""
+    return int(_lib.lib().dice_topk_scan_blocks(int(B), int(n)))
+
+
+def topk_scan(q: torch.Tensor, table: torch.Tensor, k: int, done: torch.Tensor, col_bias: Optional[torch.Tensor] = None,
+              y_offset: int = 0, y_stride: int = 1):
+    """Best ``k <= 32`` rows of the bf16 ``table`` for up to four queries ``q`` (fp32 or bf16, rounded to bf16) in one launch;
+    ``done``: int32 zero, left zero, not shared between calls that may overlap."""
+    assert q.dtype in (torch.float32, torch.bfloat16) and q.dim() == 2 and q.stride(1) == 1
+    _req(table, torch.bfloat16, "table")
+    _req(done, torch.int32, "done")
+    if col_bias is not None:
+        _req(col_bias, torch.float32, "col_bias")
+    B, n, dev = q.shape[0], table.shape[0], q.device
+    assert 1 <= k <= min(TOPK_MAX, n)
+    part = topk_scan_blocks(B, n) * B * k
+    ps = torch.empty(part, dtype=torch.float32, device=dev)
+    pi = torch.empty(part, dtype=torch.int32, device=dev)
+    sc = torch.empty(B, k, dtype=torch.float32, device=dev)
+    ix = torch.empty(B, k, dtype=torch.int64, device=dev)
+    _call("dice_topk_scan", q, _ptr(q), int(q.dtype == torch.bfloat16), q.stride(0), B, q.shape[1], _ptr(table), n,
+          table.shape[1], int(k), _ptr(col_bias), int(y_offset), int(y_stride), _ptr(ps), _ptr(pi), _ptr(done), _ptr(sc),
+          _ptr(ix), others=(table, done, col_bias))
+    return sc, ix
+
+
 def eval_band_exact(q: torch.Tensor, y: torch.Tensor, band_rows: torch.Tensor, band_cols: torch.Tensor,
                     band_count: torch.Tensor, target: torch.Tensor, greater: torch.Tensor,
                     col_bias: Optional[torch.Tensor] = None, y_offset: int = 0, y_stride: int = 1) -> None:

@@ -177,3 +177,122 @@ def test_two_stage_topk_over_a_large_table(adversarial):
     ref_s, ref_i = torch.topk(x.float() @ y.float().t(), k, dim=1)
     assert torch.allclose(sc, ref_s, atol=5e-3, rtol=2e-3)
     assert (ix == ref_i).float().mean() > 0.97
+
+
+@pytest.mark.parametrize("nx,ny,D", [(1, 1, 64), (129, 127, 64), (256, 128, 128), (257, 129, 128), (600, 40000, 256), (100, 300, 256)])
+@pytest.mark.parametrize("bias", [False, True])
+def test_masked_counts(nx, ny, D, bias):
+    """Columns in the mask never count; one and two row planes, partial planes and tiles.  Integer operands: exact sums."""
+    torch.manual_seed(nx + ny)
+    x = torch.randint(-3, 4, (nx, D), device=DEV).to(torch.bfloat16)
+    y = torch.randint(-3, 4, (ny, D), device=DEV).to(torch.bfloat16)
+    b = torch.randint(-9, 10, (ny,), device=DEV).float() if bias else None
+    scores = x.float() @ y.float().t() + (b if bias else 0.0)
+    tgt = torch.randint(0, ny, (nx,), device=DEV, dtype=torch.int32)
+    ts = scores[torch.arange(nx, device=DEV), tgt.long()].contiguous()
+    drop = torch.rand(nx, ny, device=DEV) < 0.3
+    words = (ny + 127) // 128 * 4
+    mask = torch.zeros(nx, words, dtype=torch.int32, device=DEV)
+    ptr = torch.zeros(nx + 1, dtype=torch.int64, device=DEV)
+    ptr[1:] = drop.sum(1).cumsum(0)
+    K.filter_mask(mask, ny, ptr=ptr, cols=drop.nonzero()[:, 1].to(torch.int32).contiguous())
+    greater = torch.zeros(nx, dtype=torch.int32, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    K.rank_count(x, y, ts, tgt, greater, status, col_bias=b, mask=mask)
+    assert int(status) == 0
+    beats = (scores > ts[:, None]) & ~drop
+    assert torch.equal(greater.long(), beats.sum(1))
+
+
+@pytest.mark.parametrize("pairs", [1, 31, 33, 34, 1100, 40000])
+def test_filter_mask_by_pair(pairs):
+    """The pair search over sorted keys finds exactly the stored pairs (32-ary search: sizes around its step)."""
+    g = torch.Generator().manual_seed(pairs)
+    num_b, ny = 7, 333
+    keys = torch.randperm(3 * pairs, generator=g)[:pairs].sort().values
+    counts = torch.randint(0, 5, (pairs,), generator=g)
+    offsets = torch.zeros(pairs + 1, dtype=torch.int64)
+    offsets[1:] = counts.cumsum(0)
+    values = torch.randint(0, ny, (int(offsets[-1]) + 1,), generator=g)
+    ask = torch.cat([torch.arange(0, 40), torch.randint(0, 3 * pairs + 5, (500,), generator=g), torch.tensor([3 * pairs - 1, 3 * pairs])])
+    ab = torch.stack((ask // num_b, ask % num_b, torch.zeros_like(ask)), 1).to(DEV)
+    mask = torch.zeros(len(ask), 12, dtype=torch.int32, device=DEV)
+    K.filter_mask(mask, ny, ab=ab, num_b=num_b, keys=keys.to(DEV), offsets=offsets.to(DEV), values=values.to(DEV))
+    where = {int(k): i for i, k in enumerate(keys)}
+    got = mask.cpu()
+    for row, k in enumerate(ask.tolist()):
+        want = torch.zeros(12 * 32, dtype=torch.bool)
+        if k in where:
+            want[values[offsets[where[k]]:offsets[where[k] + 1]]] = True
+        bits = (got[row].view(-1, 1) >> torch.arange(32)) & 1
+        assert torch.equal(bits.bool().reshape(-1), want), k
+
+
+def _check_topk(sc, ix, scores, k):
+    ref, _ = torch.topk(scores, k, dim=1)
+    assert torch.equal(sc, ref)
+    assert torch.equal(torch.gather(scores, 1, ix), sc) and all(len(set(r)) == k for r in ix.tolist())
+
+
+@pytest.mark.parametrize("n", [1, 2, 33, 128, 129, 2047, 40000, 140000])
+@pytest.mark.parametrize("B,D", [(1, 64), (4, 128), (5, 64), (130, 128), (300, 256)])
+def test_topk_integer_scores_with_ties(n, B, D):
+    """Small integers make exact sums and many ties: best scores, distinct ids that have them; few queries (one scan) and
+    many (tensor cores), fewer columns than groups, one tile, several, the two-stage path; a constant table."""
+    torch.manual_seed(n + B)
+    x = torch.randint(-1, 2, (B, D), device=DEV).to(torch.bfloat16)
+    y = torch.randint(-1, 2, (n, D), device=DEV).to(torch.bfloat16)
+    if n > 131072:   # few values on the sample's floor: otherwise the ties alone would not fit any list
+        y = (y.float() + torch.randint(-3, 4, (n, D), device=DEV)).to(torch.bfloat16)
+    for k in sorted({1, min(n, 10), min(n, 32)}):
+        r = FusedRanker(y)
+        sc, ix = r.topk(x.float() if B == 1 else x, k)
+        r.check()
+        _check_topk(sc, ix, x.float() @ y.float().t(), k)
+    if n <= 40000:
+        bias = torch.randint(-2, 3, (n,), device=DEV).float()
+        r = FusedRanker(torch.zeros_like(y), col_bias=bias)       # n columns, five different scores
+        sc, ix = r.topk(x, min(n, 32))
+        r.check()
+        _check_topk(sc, ix, bias.expand(B, -1), min(n, 32))
+
+
+def test_topk_skips_what_is_not_a_score():
+    x = torch.ones(3, 64, device=DEV)
+    y = torch.arange(200, device=DEV).float()[:, None].expand(-1, 64).contiguous()
+    bias = torch.zeros(200, device=DEV)
+    bias[150:] = float("-inf")
+    bias[140:150] = float("nan")
+    for q in (x, x.repeat(3, 1)):
+        r = FusedRanker(y[:, :64], col_bias=bias)
+        sc, ix = r.topk(q, 5)
+        assert ix.tolist() == [[139, 138, 137, 136, 135]] * q.shape[0] and torch.isfinite(sc).all()
+        r = FusedRanker(y[148:], col_bias=bias[148:].contiguous())
+        sc, ix = r.topk(q, 5)
+        assert (ix == -1).all() and (sc == float("-inf")).all()
+
+
+def test_split_scores_stay_within_the_margin():
+    """The margin of the band must cover the error of the split GEMM: no pair outside the band may be decided wrongly."""
+    for D in (64, 128, 256):
+        torch.manual_seed(D)
+        x, y = torch.randn(400, D, device=DEV), torch.randn(6000, D, device=DEV) * torch.rand(6000, 1, device=DEV)
+        exact = x.double() @ y.double().t()
+        tgt = torch.randint(0, 6000, (400,), device=DEV, dtype=torch.int32)
+        ts = exact[torch.arange(400, device=DEV), tgt.long()].float().contiguous()
+        factor = float(y.norm(dim=1).max()) * FusedRanker.MARGIN[D]
+        xh, xl, _, margin = K.split_rows(x, D, margin_factor=factor)
+        yh, yl, _, _ = K.split_rows(y, D)
+        greater = torch.zeros(400, dtype=torch.int32, device=DEV)
+        rows, cols = (torch.empty(1 << 20, dtype=torch.int32, device=DEV) for _ in range(2))
+        count = torch.zeros(1, dtype=torch.int64, device=DEV)
+        status = torch.zeros(1, dtype=torch.int32, device=DEV)
+        K.rank_count(xh, yh, ts, tgt, greater, status, x_lo=xl, y_lo=yl, margin=margin, band_rows=rows, band_cols=cols,
+                     band_count=count)
+        n = int(count)
+        assert int(status) == 0 and n < 0.01 * 400 * 6000
+        band = torch.zeros(400, 6000, dtype=torch.bool, device=DEV)
+        band[rows[:n].long(), cols[:n].long()] = True
+        beats = exact > ts[:, None].double()
+        beats[torch.arange(400, device=DEV), tgt.long()] = False
+        assert torch.equal(greater.long(), (beats & ~band).sum(1))
