@@ -19,8 +19,9 @@
 // candidates given by the caller go through red.add into the gradient table and a flag per row.
 //
 // Measured against the launch sequence lookup / score / backward / sweeps (one triple per query, scalar atomics): 10 000
-// positives x 11, D = 128, 123 182 rows, 37 relations 640 -> 160 us; 1024 x 100 given candidates, D = 256, 14 541 rows
-// 131 -> 101 us; 32 768 x 129, D = 128, 5 million rows, sparse 5207 -> 3435 us.
+// positives x 11, D = 128, 123 182 rows, 37 relations 640 -> 128 us; 1024 x 100 given candidates, D = 256, 14 541 rows
+// 131 -> 85 us; 32 768 x 129, D = 128, 5 million rows, sparse 5207 -> 2530 us (the update of 2.9 million rows moves 8.7 GB
+// in 1.9 ms).
 #include "algebra.cuh"
 #include "dice_b200.h"
 #include "optim.cuh"
@@ -256,14 +257,18 @@ __device__ __forceinline__ float transpose_sum(float (&a)[CH], int lane) {
 }
 
 constexpr int GRAD_THREADS = 256;
+// Candidate rows in flight (of up to 128 floats) and resident blocks per SM.  Measured (4, 4) / (8, 2): 32 768 x 129 on 5
+// million rows, D = 128: 609 / 660 us, 10 000 x 11: 30 / 39 us.
+constexpr int GRAD_CH = 4;
+constexpr int GRAD_B = 4;
 
 // One warp per part of a group (`split` parts share the candidates of a group where there are few groups).  CH candidate
 // rows are in flight at a time.
 template <int K, int V, int NC>
-__global__ void __launch_bounds__(GRAD_THREADS, 2) grad_kernel(const GradParams p) {
+__global__ void __launch_bounds__(GRAD_THREADS, GRAD_B) grad_kernel(const GradParams p) {
   using F = Frag<K, V, NC>;
   constexpr int PL = K * V * NC;                       // floats of a row per lane
-  constexpr int CH = PL <= 4 ? 8 : PL <= 8 ? 4 : 2;
+  constexpr int CH = PL <= 4 ? GRAD_CH : PL <= 8 ? GRAD_CH / 2 : GRAD_CH / 4;
   constexpr int LPC = 32 / CH;                         // lanes that end up with a candidate's score
   const int lane = threadIdx.x & 31;
   const int w = p.D / K;
@@ -355,15 +360,19 @@ __global__ void __launch_bounds__(GRAD_THREADS, 2) grad_kernel(const GradParams 
           id = -1;
         }
       }
+      // a drawn entity's chain: the link is exchanged now, its value is only needed when the node is written
+      const bool listed = chained && c > 0 && id >= 0;
+      const int node = n * p.C + c;   // N * C fits 31 bits (checked on the host)
+      int next = -1;
+      if (listed) next = atomicExch(p.list_head + id, node);
       float g_mine = 0.f;
       const int count = min(32, c_hi - c0);
       for (int s0 = 0; s0 < count; s0 += CH) {
         F row[CH];
-        long long e[CH];
 #pragma unroll
-        for (int j = 0; j < CH; ++j) {
-          e[j] = __shfl_sync(0xffffffffu, id, s0 + j);   // -1 past the end or out of range: row 0 stands in
-          frag_load<K, V, NC>(p.ent + (e[j] < 0 ? 0ll : e[j]) * p.D, w, lane, row[j]);
+        for (int j = 0; j < CH; ++j) {   // -1 past the end or out of range: row 0 stands in
+          const long long e = __shfl_sync(0xffffffffu, id, s0 + j);
+          frag_load<K, V, NC>(p.ent + (e < 0 ? 0ll : e) * p.D, w, lane, row[j]);
         }
         float a[CH];
 #pragma unroll
@@ -402,22 +411,17 @@ __global__ void __launch_bounds__(GRAD_THREADS, 2) grad_kernel(const GradParams 
             FRAG_LOOP(k, cc, u) row[j].x[k][cc][u] = fv.x[k][cc][u] - row[j].x[k][cc][u];
           }
           FRAG_LOOP(k, cc, u) acc.x[k][cc][u] = fmaf(gj, row[j].x[k][cc][u], acc.x[k][cc][u]);
-          const bool listed = chained && c0 + s0 + j > 0;
-          if (e[j] >= 0 && !listed) {
-            if (p.translation) frag_red<K, V, NC>(p.g_ent + e[j] * p.D, w, lane, row[j], -gj);
-            else frag_red<K, V, NC>(p.g_ent + e[j] * p.D, w, lane, fv, gj);
+          if (!chained || c0 + s0 + j == 0) {   // uniform
+            const long long e = __shfl_sync(0xffffffffu, id, s0 + j);
+            if (e >= 0) {
+              if (p.translation) frag_red<K, V, NC>(p.g_ent + e * p.D, w, lane, row[j], -gj);
+              else frag_red<K, V, NC>(p.g_ent + e * p.D, w, lane, fv, gj);
+            }
           }
         }
       }
-      if (id >= 0) {
-        if (chained && c > 0) {
-          const int node = n * p.C + c;   // N * C fits 31 bits (checked on the host)
-          const int next = atomicExch(p.list_head + id, node);
-          p.nodes[node] = make_int2(next, __float_as_int(g_mine));
-        } else {
-          p.touched[id] = 1;
-        }
-      }
+      if (listed) p.nodes[node] = make_int2(next, __float_as_int(g_mine));
+      else if (id >= 0) p.touched[id] = 1;
     }
 
     // back through F to the fixed entity and the relation
@@ -509,13 +513,12 @@ struct UpdateParams {
   const int2* nodes;
   const float* fixed;
   long long rows;
-  int D, C, translation;
+  int D, C, translation, chunk;
   float* P[2];               // relation table, coefficient (or null)
   float* gP[2];
   float* mP[2];
   float* vP[2];
   long long nP[2];
-  int kind;
   float lr, beta1, beta2, eps, weight_decay;
   double* loss;
   float* loss_out;
@@ -524,16 +527,21 @@ struct UpdateParams {
 };
 
 constexpr int UPDATE_THREADS = 256;
+// Resident blocks per SM and float4s in flight per thread.  Measured (8, 1) / (6, 1) / (5, 1) / (4, 2): 123 182 rows x 128
+// 82 / 102 / 96 / 117 us, 14 541 x 256 25 / 35 / 34 / 38 us, sparse 2.9 of 5 million rows x 128 1893 / 1994 / 1937 / 2147 us.
+constexpr int UPDATE_B = 8;
+constexpr int UPDATE_R = 1;
 
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
 
+template <int KIND>
 __device__ __forceinline__ void update4(const UpdateParams& p, const OptStepConsts& c, float4& w, const float4& g, float4& m,
                                         float4& v) {
-  w.x = opt_update(p.kind, w.x, g.x, m.x, v.x, p.lr, p.beta1, p.beta2, p.eps, p.weight_decay, c.inv_bc1, c.inv_sqrt_bc2, c.clip, c.first_step);
-  w.y = opt_update(p.kind, w.y, g.y, m.y, v.y, p.lr, p.beta1, p.beta2, p.eps, p.weight_decay, c.inv_bc1, c.inv_sqrt_bc2, c.clip, c.first_step);
-  w.z = opt_update(p.kind, w.z, g.z, m.z, v.z, p.lr, p.beta1, p.beta2, p.eps, p.weight_decay, c.inv_bc1, c.inv_sqrt_bc2, c.clip, c.first_step);
-  w.w = opt_update(p.kind, w.w, g.w, m.w, v.w, p.lr, p.beta1, p.beta2, p.eps, p.weight_decay, c.inv_bc1, c.inv_sqrt_bc2, c.clip, c.first_step);
+  w.x = opt_update(KIND, w.x, g.x, m.x, v.x, p.lr, p.beta1, p.beta2, p.eps, p.weight_decay, c.inv_bc1, c.inv_sqrt_bc2, c.clip, c.first_step);
+  w.y = opt_update(KIND, w.y, g.y, m.y, v.y, p.lr, p.beta1, p.beta2, p.eps, p.weight_decay, c.inv_bc1, c.inv_sqrt_bc2, c.clip, c.first_step);
+  w.z = opt_update(KIND, w.z, g.z, m.z, v.z, p.lr, p.beta1, p.beta2, p.eps, p.weight_decay, c.inv_bc1, c.inv_sqrt_bc2, c.clip, c.first_step);
+  w.w = opt_update(KIND, w.w, g.w, m.w, v.w, p.lr, p.beta1, p.beta2, p.eps, p.weight_decay, c.inv_bc1, c.inv_sqrt_bc2, c.clip, c.first_step);
 }
 
 // g += s * F, or for distances -s * (F - w) with the row's own values w
@@ -546,82 +554,36 @@ __device__ __forceinline__ void add_triple(bool translation, float s, const floa
   }
 }
 
-// Every row: D / 4 threads per row, U rows of each such group in flight.  The row's flag and list head are read by all of
-// its threads before one of them clears them (one block barrier per U rows).
-__device__ __forceinline__ void update_dense(const UpdateParams& p, const OptStepConsts& c) {
-  constexpr int U = 2;
-  const int tpr = p.D / 4;
-  const int rpb = UPDATE_THREADS / tpr;
-  const int sub = threadIdx.x / tpr;
-  const int d = (threadIdx.x % tpr) * 4;
-  const bool active = sub < rpb;
-  for (long long base = static_cast<long long>(blockIdx.x) * rpb * U; base < p.rows;
-       base += static_cast<long long>(gridDim.x) * rpb * U) {
-    float4 w[U], m[U], v[U];
-    int head[U];
-    bool dense[U], in[U];
-    size_t off[U];
-#pragma unroll
-    for (int j = 0; j < U; ++j) {
-      const long long row = base + static_cast<long long>(j) * rpb + sub;
-      in[j] = active && row < p.rows;
-      off[j] = static_cast<size_t>(row) * p.D + d;
-      head[j] = -1;
-      dense[j] = false;
-      m[j] = v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (in[j]) {
-        w[j] = ld4(p.E + off[j]);
-        if (p.kind != 2) { m[j] = ld4(p.mE + off[j]); v[j] = ld4(p.vE + off[j]); }
-        dense[j] = p.touched[row] != 0;
-        if (p.list_head != nullptr) head[j] = p.list_head[row];
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < U; ++j) {
-      if (!in[j]) continue;
-      const long long row = base + static_cast<long long>(j) * rpb + sub;
-      if (d == 0) {
-        if (dense[j]) p.touched[row] = 0;
-        if (head[j] >= 0) p.list_head[row] = -1;
-      }
-      float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (dense[j]) {
-        g = ld4(p.gE + off[j]);
-        st4(p.gE + off[j], make_float4(0.f, 0.f, 0.f, 0.f));
-      }
-      for (int node = head[j]; node >= 0;) {
-        const int2 nd = p.nodes[node];
-        add_triple(p.translation, __int_as_float(nd.y), ld4(p.fixed + static_cast<size_t>(node / p.C) * p.D + d), w[j], g);
-        node = nd.x;
-      }
-      update4(p, c, w[j], g, m[j], v[j]);
-      st4(p.E + off[j], w[j]);
-      if (p.kind != 2) { st4(p.mE + off[j], m[j]); st4(p.vE + off[j], v[j]); }
-    }
-  }
-}
+// A block takes `chunk` <= 256 consecutive rows.  One thread per row reads the row's flag and list head, clears them and
+// follows the links of the first CHAIN triples (their latencies overlap over the rows); the rows to update (all of them, or
+// with SPARSE the ones with a gradient) are compacted into shared memory in row order.  Then the float4s of these rows are
+// dealt to the threads, with nothing dependent left to load: walking a chain while holding the row left
+// the memory system idle (5M rows x 128, 2.9M of them touched, TransE: 2734 us).
+constexpr int CHAIN = 6;
 
-// Only rows with a gradient.  A block takes 256 consecutive rows, compacts the ones to update into shared memory in row
-// order and deals them to its warps, R rows per warp in flight.
-__device__ __forceinline__ void update_sparse(const UpdateParams& p, const OptStepConsts& c) {
-  constexpr int R = 4;
-  __shared__ int s_head[UPDATE_THREADS];
-  __shared__ unsigned short s_row[UPDATE_THREADS];   // row of the chunk, bit 15: has a gradient row
+template <bool SPARSE, int KIND>
+__device__ __forceinline__ void update_rows(const UpdateParams& p, const OptStepConsts& c) {
+  constexpr int R = UPDATE_R;
+  __shared__ float s_g[UPDATE_THREADS][CHAIN];
+  __shared__ int s_n[UPDATE_THREADS][CHAIN];
+  __shared__ int s_rest[UPDATE_THREADS];             // first node of a longer chain's rest, or -1
+  __shared__ unsigned short s_row[UPDATE_THREADS];   // row of the chunk; bit 15: has a gradient row; bits 8..10: triples
   __shared__ int s_count[UPDATE_THREADS / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (long long base = static_cast<long long>(blockIdx.x) * UPDATE_THREADS; base < p.rows;
-       base += static_cast<long long>(gridDim.x) * UPDATE_THREADS) {
+  const int tpr = p.D / 4;
+  for (long long base = static_cast<long long>(blockIdx.x) * p.chunk; base < p.rows;
+       base += static_cast<long long>(gridDim.x) * p.chunk) {
     const long long mine = base + threadIdx.x;
+    const bool in = threadIdx.x < p.chunk && mine < p.rows;
     bool dense = false;
-    int head = -1;
-    if (mine < p.rows) {
+    int node = -1;
+    if (in) {
       dense = p.touched[mine] != 0;
+      if (p.list_head != nullptr) node = p.list_head[mine];
       if (dense) p.touched[mine] = 0;
-      if (p.list_head != nullptr) head = p.list_head[mine];
-      if (head >= 0) p.list_head[mine] = -1;
+      if (node >= 0) p.list_head[mine] = -1;
     }
-    const bool flag = dense || head >= 0;
+    const bool flag = SPARSE ? dense || node >= 0 : in;
     const unsigned int bits = __ballot_sync(0xffffffffu, flag);
     if (lane == 0) s_count[warp] = __popc(bits);
     __syncthreads();
@@ -634,66 +596,67 @@ __device__ __forceinline__ void update_sparse(const UpdateParams& p, const OptSt
     }
     if (flag) {
       const int at = before + __popc(bits & ((1u << lane) - 1u));
-      s_row[at] = static_cast<unsigned short>(threadIdx.x | (dense ? 0x8000 : 0));
-      s_head[at] = head;
+      int links = 0;
+#pragma unroll
+      for (int l = 0; l < CHAIN; ++l) {
+        if (node < 0) break;
+        const int2 nd = p.nodes[node];
+        s_n[at][l] = node / p.C;
+        s_g[at][l] = __int_as_float(nd.y);
+        node = nd.x;
+        ++links;
+      }
+      s_rest[at] = node;
+      s_row[at] = static_cast<unsigned short>(threadIdx.x | (links << 8) | (dense ? 0x8000 : 0));
     }
     __syncthreads();
-    for (int i0 = warp * R; i0 < total; i0 += (UPDATE_THREADS / 32) * R) {
-      for (int d = lane * 4; d < p.D; d += 128) {
-        float4 w[R], m[R], v[R], g[R];
-        size_t off[R];
-        int node[R];
+    const int items = total * tpr;
+    for (int q0 = threadIdx.x; q0 < items; q0 += UPDATE_THREADS * R) {
+      float4 w[R], m[R], v[R], g[R];
+      size_t off[R];
+      int at[R], d[R];
 #pragma unroll
-        for (int j = 0; j < R; ++j) {
-          const int i = i0 + j < total ? i0 + j : i0;
-          const int rc = s_row[i];
-          node[j] = i0 + j < total ? s_head[i] : -1;
-          off[j] = static_cast<size_t>(base + (rc & 0x7fff)) * p.D + d;
-          w[j] = ld4(p.E + off[j]);
-          m[j] = v[j] = g[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (p.kind != 2) { m[j] = ld4(p.mE + off[j]); v[j] = ld4(p.vE + off[j]); }
-          if ((rc & 0x8000) && i0 + j < total) {
-            g[j] = ld4(p.gE + off[j]);
-            st4(p.gE + off[j], make_float4(0.f, 0.f, 0.f, 0.f));
-          }
+      for (int j = 0; j < R; ++j) {
+        const int q = q0 + j * UPDATE_THREADS < items ? q0 + j * UPDATE_THREADS : q0;
+        at[j] = q / tpr;
+        d[j] = (q - at[j] * tpr) * 4;
+        const int rc = s_row[at[j]];
+        off[j] = static_cast<size_t>(base + (rc & 0xff)) * p.D + d[j];
+        w[j] = ld4(p.E + off[j]);
+        m[j] = v[j] = g[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (KIND != 2) { m[j] = ld4_once(p.mE + off[j]); v[j] = ld4_once(p.vE + off[j]); }
+        if ((rc & 0x8000) && (j == 0 || q != q0)) {
+          g[j] = ld4(p.gE + off[j]);
+          st4(p.gE + off[j], make_float4(0.f, 0.f, 0.f, 0.f));
         }
-        // the R chains are walked together: their loads are independent (ends are -1)
-        while ((node[0] & node[1] & node[2] & node[3]) >= 0) {
-          int2 nd[R];
-          float4 f[R];
+      }
 #pragma unroll
-          for (int j = 0; j < R; ++j) {
-            nd[j] = make_int2(-1, 0);
-            f[j] = w[j];
-            if (node[j] >= 0) {
-              nd[j] = p.nodes[node[j]];
-              f[j] = ld4(p.fixed + static_cast<size_t>(node[j] / p.C) * p.D + d);
-            }
-          }
-#pragma unroll
-          for (int j = 0; j < R; ++j) {
-            if (node[j] < 0) continue;
-            add_triple(p.translation, __int_as_float(nd[j].y), f[j], w[j], g[j]);
-            node[j] = nd[j].x;
-          }
+      for (int j = 0; j < R; ++j) {
+        const int links = (s_row[at[j]] >> 8) & 7;
+        for (int l = 0; l < links; ++l)
+          add_triple(p.translation, s_g[at[j]][l], ld4(p.fixed + static_cast<size_t>(s_n[at[j]][l]) * p.D + d[j]), w[j], g[j]);
+        for (int rest = links == CHAIN ? s_rest[at[j]] : -1; rest >= 0;) {
+          const int2 nd = p.nodes[rest];
+          add_triple(p.translation, __int_as_float(nd.y), ld4(p.fixed + static_cast<size_t>(rest / p.C) * p.D + d[j]), w[j], g[j]);
+          rest = nd.x;
         }
+      }
 #pragma unroll
-        for (int j = 0; j < R; ++j) {
-          if (i0 + j >= total) continue;
-          update4(p, c, w[j], g[j], m[j], v[j]);
-          st4(p.E + off[j], w[j]);
-          if (p.kind != 2) { st4(p.mE + off[j], m[j]); st4(p.vE + off[j], v[j]); }
-        }
+      for (int j = 0; j < R; ++j) {
+        if (j > 0 && q0 + j * UPDATE_THREADS >= items) continue;
+        update4<KIND>(p, c, w[j], g[j], m[j], v[j]);
+        st4(p.E + off[j], w[j]);
+        if (KIND != 2) { st4_once(p.mE + off[j], m[j]); st4_once(p.vE + off[j], v[j]); }
       }
     }
     __syncthreads();   // the lists are rebuilt for the next chunk
   }
 }
 
-template <bool SPARSE>
-__global__ void __launch_bounds__(UPDATE_THREADS) update_kernel(const UpdateParams p) {
+template <bool SPARSE, int KIND>
+__global__ void __launch_bounds__(UPDATE_THREADS, UPDATE_B) update_kernel(const UpdateParams p) {
   const long long t = *p.step + 1;
-  const OptStepConsts c = opt_step_consts(p.kind, t, p.beta1, p.beta2);
+  const OptStepConsts c = opt_step_consts(KIND, t, p.beta1, p.beta2);
   const long long tid = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
 #pragma unroll
@@ -703,14 +666,13 @@ __global__ void __launch_bounds__(UPDATE_THREADS) update_kernel(const UpdatePara
       const float g = p.gP[s][i];
       p.gP[s][i] = 0.f;
       float m = 0.f, v = 0.f;
-      if (p.kind != 2) { m = p.mP[s][i]; v = p.vP[s][i]; }
-      p.P[s][i] = opt_update(p.kind, p.P[s][i], g, m, v, p.lr, p.beta1, p.beta2, p.eps, p.weight_decay, c.inv_bc1,
+      if (KIND != 2) { m = p.mP[s][i]; v = p.vP[s][i]; }
+      p.P[s][i] = opt_update(KIND, p.P[s][i], g, m, v, p.lr, p.beta1, p.beta2, p.eps, p.weight_decay, c.inv_bc1,
                              c.inv_sqrt_bc2, c.clip, c.first_step);
-      if (p.kind != 2) { p.mP[s][i] = m; p.vP[s][i] = v; }
+      if (KIND != 2) { p.mP[s][i] = m; p.vP[s][i] = v; }
     }
   }
-  if constexpr (SPARSE) update_sparse(p, c);
-  else update_dense(p, c);
+  update_rows<SPARSE, KIND>(p, c);
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
@@ -727,7 +689,7 @@ template <int K, int V, int NC>
 static int launch_grad(const GradParams& p, cudaStream_t s) {
   const long long warps = static_cast<long long>(p.N) * p.split;
   long long blocks = (warps * 32 + GRAD_THREADS - 1) / GRAD_THREADS;
-  if (blocks > 148 * 16) blocks = 148 * 16;
+  if (blocks > 148 * 64) blocks = 148 * 64;
   grad_kernel<K, V, NC><<<static_cast<unsigned>(blocks), GRAD_THREADS, 0, s>>>(p);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
@@ -812,16 +774,28 @@ extern "C" int dice_sampled_update(int kind, int sparse, float* E, float* gE, fl
   const uintptr_t al = reinterpret_cast<uintptr_t>(E) | reinterpret_cast<uintptr_t>(gE) | reinterpret_cast<uintptr_t>(mE) |
                        reinterpret_cast<uintptr_t>(vE) | reinterpret_cast<uintptr_t>(fixed);
   if (al & 15) return -5;
-  UpdateParams p{E, gE, mE, vE, touched, list_head, static_cast<const int2*>(nodes), fixed, rows, D, C, translation,
-                 {R, coeff}, {gR, gC}, {mR, mC}, {vR, vC}, {nR, nC}, kind, lr, beta1, beta2, eps, weight_decay,
+  UpdateParams p{E, gE, mE, vE, touched, list_head, static_cast<const int2*>(nodes), fixed, rows, D, C, translation, 0,
+                 {R, coeff}, {gR, gC}, {mR, mC}, {vR, vC}, {nR, nC}, lr, beta1, beta2, eps, weight_decay,
                  loss, loss_out, step, done};
-  const long long rpb = sparse ? UPDATE_THREADS : 2 * (UPDATE_THREADS / (D / 4));
-  long long blocks = (rows + rpb - 1) / rpb;
+  // as many blocks as are resident (148 SMs x UPDATE_B), each with the same number of equally long chunks: a partial second
+  // wave of blocks costs as much as a full one
+  const long long resident = 148ll * UPDATE_B;
+  const long long passes = (rows + resident * UPDATE_THREADS - 1) / (resident * UPDATE_THREADS);
+  p.chunk = static_cast<int>((rows + resident * passes - 1) / (resident * passes));
+  long long blocks = (rows + p.chunk - 1) / p.chunk;
   const long long other = (nR + UPDATE_THREADS - 1) / UPDATE_THREADS;
   if (blocks < other) blocks = other;
-  if (blocks > 148 * 8) blocks = 148 * 8;
+  if (blocks > resident) blocks = resident;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (sparse) update_kernel<true><<<static_cast<unsigned>(blocks), UPDATE_THREADS, 0, s>>>(p);
-  else update_kernel<false><<<static_cast<unsigned>(blocks), UPDATE_THREADS, 0, s>>>(p);
+  const dim3 grid(static_cast<unsigned>(blocks));
+  switch (sparse ? 4 + kind : kind) {
+    case 0: update_kernel<false, 0><<<grid, UPDATE_THREADS, 0, s>>>(p); break;
+    case 1: update_kernel<false, 1><<<grid, UPDATE_THREADS, 0, s>>>(p); break;
+    case 2: update_kernel<false, 2><<<grid, UPDATE_THREADS, 0, s>>>(p); break;
+    case 3: update_kernel<false, 3><<<grid, UPDATE_THREADS, 0, s>>>(p); break;
+    case 4: update_kernel<true, 0><<<grid, UPDATE_THREADS, 0, s>>>(p); break;
+    case 5: update_kernel<true, 1><<<grid, UPDATE_THREADS, 0, s>>>(p); break;
+    default: update_kernel<true, 2><<<grid, UPDATE_THREADS, 0, s>>>(p); break;
+  }
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }

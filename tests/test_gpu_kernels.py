@@ -517,3 +517,33 @@ def test_owned_row_list_and_dq_pull(W, rank, n, D):
     K.owned_rows(bad, n, W, rank, NE, rows, count, status)
     torch.cuda.synchronize()
     assert int(status) != 0
+
+
+@pytest.mark.parametrize("kind", [0, 1, 3])
+def test_optimizer_quotient_over_the_range_of_second_moments(kind):
+    """Update of one step against 64-bit arithmetic: fp32 rounds m, v, the root, the product with the bias correction, the
+    sum with eps, the quotient and the step size, so 8 units of 2^-24 bound the update; second moments from denormals to
+    1e30, zero and infinity."""
+    n = 1 << 16
+    g = torch.Generator(device=DEV).manual_seed(kind)
+    v = torch.exp(torch.empty(n, device=DEV).uniform_(-87.0, 69.0, generator=g))
+    v[:64] = 0.0
+    v[64:128] = 1e-42
+    v[128:160] = float("inf")
+    m = torch.randn(n, device=DEV, generator=g) * torch.exp(torch.empty(n, device=DEV).uniform_(-20.0, 10.0, generator=g))
+    m[:32] = 0.0
+    grad = torch.zeros(n, device=DEV) if kind != 3 else torch.randn(n, device=DEV, generator=g)
+    w, step = torch.zeros(n, device=DEV), torch.full((1,), 40, dtype=torch.int64, device=DEV)
+    b1, b2, eps, lr = 0.9, 0.999, 1e-8, 0.01
+    m0, v0, g0 = m.double(), v.double(), grad.double()
+    K.optimizer_step(kind, w, grad, m, v, None, step, lr, b1, b2, eps, 0.0)
+    b1, b2, eps, lr = (float(torch.tensor(x, dtype=torch.float32)) for x in (b1, b2, eps, lr))   # as the kernel gets them
+    if kind == 3:
+        ng = (g0 / v0.sqrt().clamp_min(eps)).clamp(-(40 ** 0.25), 40 ** 0.25)
+        want = -lr * (m0 + (1 - b1) * (ng - m0))
+        tol = 2.0 ** -24 * 8 * lr * (m0.abs() + ng.abs()) + 1e-40
+    else:
+        want = -lr / (1 - b1 ** 41) * (b1 * m0) / ((b2 * v0).sqrt() / (1 - b2 ** 41) ** 0.5 + eps)
+        tol = 2.0 ** -24 * 8 * want.abs() + 2.0 ** -24 * 8 * want.abs() + 1e-40   # powers of beta: as many units again
+    assert torch.isfinite(w).all() and float(w[128:160].abs().max()) == (0.0 if kind != 3 else float(w[128:160].abs().max()))
+    assert ((w.double() - want).abs() <= tol).all(), float(((w.double() - want).abs() / tol).max())
