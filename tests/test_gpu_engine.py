@@ -11,6 +11,7 @@ from dice_embeddings_b200.data.datasets import KvsAll, OnevsAllDataset
 from dice_embeddings_b200.data.synthetic import zipf_kg
 from dice_embeddings_b200.models import initialize_model
 from dice_embeddings_b200.ops.fused_step import FusedKvsAllEngine, build_fused_engine
+from dice_embeddings_b200.ops.hybrid_step import ExternalQueryEngine
 
 DEV = torch.device("cuda:0")
 
@@ -199,3 +200,64 @@ def test_pipelined_host_steps_return_the_same_losses():
         b.append(e2.step_from_host_pipelined(x, dp))
     b = b[1:] + [e2.last_loss()]
     assert all(abs(u - v) < 1e-6 * max(1.0, abs(u)) for u, v in zip(a, b)), (a, b)
+
+
+@pytest.mark.parametrize("name,optim", [("ConEx", "Adam"), ("TransE", "AdamW"), ("DualE", "SGD"), ("ConvQ", "Adopt")])
+def test_external_query_step_from_a_graph_equals_plain_launches(name, optim):
+    """Same losses and weights from replayed and plain steps: two batch sizes, a learning-rate change, evaluation mode in
+    between (sums with atomics in another order: 1e-4 of the weights' change)."""
+    engines = []
+    for use_graph in (True, False):
+        torch.manual_seed(0)
+        tr = zipf_kg(700, 9, 6000, seed=1)
+        ds = KvsAll(tr, 700, 9, label_smoothing_rate=0.1).to(DEV)
+        model, _ = initialize_model(dict(model=name, embedding_dim=64, num_entities=700, num_relations=9, optim=optim,
+                                         learning_rate=0.01, scoring_technique="KvsAll", num_of_output_channels=4, kernel_size=3))
+        model = model.to(DEV).train()
+        with torch.no_grad():
+            model.entity_embeddings.weight.mul_(0.3)
+            model.relation_embeddings.weight.mul_(0.3)
+        engines.append((ExternalQueryEngine(model, ds, batch_size=256, lr=1e-3, device=DEV, use_graph=use_graph), ds, model))
+    start = [p.detach().clone() for p in engines[0][2].parameters()]
+    losses = [[], []]
+    for step in range(12):
+        n = 256 if step % 3 else 199
+        for k, (eng, ds, model) in enumerate(engines):
+            if step == 8:
+                eng.optimizer_view().param_groups[0]["lr"] = 5e-4
+            idx = torch.arange(step * 7, step * 7 + n, device=DEV) % len(ds)
+            batch = ds.make_batch(idx)
+            losses[k].append(eng.step((batch[0], idx)))
+    for eng, _, _ in engines:
+        eng.sync_to_model()
+    assert len(engines[0][0]._graphs) > 0 or optim == "Adopt"
+    a, b = (torch.stack(x) for x in losses)
+    assert len({x.data_ptr() for x in losses[0]}) == 12 and a.unique().numel() > 6   # every step's loss is its own tensor
+    assert torch.allclose(a, b, rtol=1e-4), (a, b)
+    for s, (name, p), q in zip(start, engines[0][2].named_parameters(), engines[1][2].parameters()):
+        if name.endswith("conv2d.bias"):
+            continue   # batch normalisation takes its gradient to zero: Adam scales the rounding noise up
+        assert (p - q).abs().max() <= 2e-2 * (q - s).abs().max() + 1e-6
+    for (n1, x), (_, y) in zip(engines[0][2].named_buffers(), engines[1][2].named_buffers()):
+        assert torch.allclose(x.float(), y.float(), rtol=1e-3, atol=1e-5), n1
+
+
+def test_external_query_step_with_hooks_runs_as_plain_launches():
+    tr = zipf_kg(300, 5, 2000, seed=1)
+    ds = KvsAll(tr, 300, 5).to(DEV)
+    model, _ = initialize_model(dict(model="ConEx", embedding_dim=64, num_entities=300, num_relations=5, optim="Adam",
+                                     learning_rate=0.01, scoring_technique="KvsAll", num_of_output_channels=4, kernel_size=3))
+    model = model.to(DEV).train()
+    eng = ExternalQueryEngine(model, ds, batch_size=64, lr=0.01, device=DEV)
+    idx = torch.arange(64, device=DEV)
+    for _ in range(3):
+        eng.step(ds.make_batch(idx)[:1] + (idx,))
+    assert len(eng._graphs) == 1
+    calls = []
+    handle = model.fc1.register_forward_hook(lambda *a: calls.append(1))
+    eng.step(ds.make_batch(idx)[:1] + (idx,))
+    packed = []
+    handle.remove()
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(1) or t, lambda t: t):
+        eng.step(ds.make_batch(idx)[:1] + (idx,))
+    assert len(calls) == 1 and packed
