@@ -19,7 +19,8 @@
 // narrower.  The second X plane then holds the lo part of the same 128 rows.
 //
 // Measured: 8192 queries x 2M rows x 256, COUNT 8855 -> 6808 us (1.26 PFLOP/s); 1024 x 2M x 256, COLLECT 1348 -> 1070 us;
-// evaluation of 20 466 queries x 14 541 x 256 (band, filters and counts) 15.8 -> 0.83 ms on the device.
+// evaluation of 20 466 queries x 14 541 x 256 (band, filters and counts) 15.8 -> 0.56 ms on the device (75 us a batch of 4096
+// for the three GEMMs; with the parts of a 64-row tile side by side in one stage 116 us, the MMA being half as wide).
 //
 // CTA (one per SM, persistent over a range of tiles): warp 0 TMA producer, warp 1 MMA issuer, warps 2..9 epilogue (two per
 // TMEM lane quarter, each one half of the columns; warp (quarter, p) also fills plane p of X).  All waits are bounded.
@@ -69,10 +70,10 @@ template <int D, bool SPLIT>
 struct Cfg {
   static constexpr int NSLAB = D / 64;
   static constexpr int XR = SPLIT ? 128 : 256;         // rows of an X tile
-  static constexpr int BY = SPLIT ? 64 : 128;          // rows of a Y tile
+  static constexpr int BY = 128;                       // rows of a Y tile; with SPLIT its hi and lo parts are two stages
+  static constexpr int PARTS = SPLIT ? 2 : 1;
   static constexpr int YSLAB = BY * 128;
-  static constexpr int PART = NSLAB * YSLAB;           // bytes of a Y tile (hi part)
-  static constexpr int Y_BYTES = SPLIT ? 2 * PART : PART;
+  static constexpr int Y_BYTES = NSLAB * YSLAB;        // bytes of a stage
   static constexpr int NSTAGE = D == 256 ? 3 : D == 128 ? 6 : 8;
   static constexpr int S_COL = D;                      // two planes of D / 2 columns each come first
   static constexpr int NBUF = (512 - D) / BY > 4 ? 4 : (512 - D) / BY;
@@ -174,16 +175,14 @@ rank_tiles_kernel(const __grid_constant__ CUtensorMap tmap_y, const __grid_const
         int x, y0, run;
         p.map.locate(w, x, y0, run);
         const int n = static_cast<int>(min(static_cast<long long>(run), w_end - w));
-        for (int t = 0; t < n; ++t, ++ycount) {
+        for (int t = 0; t < n * C::PARTS; ++t, ++ycount) {
           const uint32_t st = ycount % C::NSTAGE;
           if (!mbar_wait_bounded(y_empty + st, ((ycount / C::NSTAGE) & 1) ^ 1, s_abort)) { ok = false; break; }
           mbar_arrive_expect_tx(y_full + st, C::Y_BYTES);
           uint8_t* dst = sY + st * C::Y_BYTES;
+          const CUtensorMap* tm = SPLIT && (t & 1) ? &tmap_ylo : &tmap_y;
           for (int s = 0; s < C::NSLAB; ++s)
-            tma_load_2d(dst + s * C::YSLAB, &tmap_y, s * 64, (y0 + t) * C::BY, y_full + st);
-          if (SPLIT)
-            for (int s = 0; s < C::NSLAB; ++s)
-              tma_load_2d(dst + C::PART + s * C::YSLAB, &tmap_ylo, s * 64, (y0 + t) * C::BY, y_full + st);
+            tma_load_2d(dst + s * C::YSLAB, tm, s * 64, (y0 + t / C::PARTS) * C::BY, y_full + st);
         }
         w += n;
       }
@@ -219,8 +218,8 @@ rank_tiles_kernel(const __grid_constant__ CUtensorMap tmap_y, const __grid_const
         const int units = units_of(x);
         if (!mbar_wait_bounded(x_full, seg & 1, s_abort)) { ok = false; break; }
         for (int t = 0; t < n && ok; ++t, ++ycount) {
-          const uint32_t st = ycount % C::NSTAGE;
-          const uint64_t yd = ydesc + st * (C::Y_BYTES >> 4);
+          uint32_t st = ycount % C::NSTAGE;
+          uint64_t yd = ydesc + st * (C::Y_BYTES >> 4);
           if (!mbar_wait_bounded(y_full + st, (ycount / C::NSTAGE) & 1, s_abort)) { ok = false; break; }
           for (int u = 0; u < units; ++u, ++g) {
             const uint32_t b = g % C::NBUF;
@@ -230,7 +229,13 @@ rank_tiles_kernel(const __grid_constant__ CUtensorMap tmap_y, const __grid_const
             gemm(d_tmem, u, yd, true);
             if constexpr (SPLIT) {
               gemm(d_tmem, 1, yd, false);
-              gemm(d_tmem, 0, yd + (C::PART >> 4), false);
+              tc_commit(y_empty + st);
+              ++ycount;                       // the lo part is the next stage
+              st = ycount % C::NSTAGE;
+              yd = ydesc + st * (C::Y_BYTES >> 4);
+              if (!mbar_wait_bounded(y_full + st, (ycount / C::NSTAGE) & 1, s_abort)) { ok = false; break; }
+              tc_fence_after();
+              gemm(d_tmem, 0, yd, false);
             }
             tc_commit(s_full + b);
           }
@@ -463,7 +468,7 @@ static int launch(RankParams& p, const void* y, const void* y_lo, int num_ctas, 
   if (rc) return rc;
   p.nx_tiles = (p.x_rows + C::XR - 1) / C::XR;
   p.ny_tiles = (p.y_rows + C::BY - 1) / C::BY;
-  p.map = TileMap::make(p.nx_tiles, p.ny_tiles, C::Y_BYTES, 48ll << 20);
+  p.map = TileMap::make(p.nx_tiles, p.ny_tiles, C::PARTS * C::Y_BYTES, 48ll << 20);
   if (num_ctas <= 0) {
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -542,9 +547,16 @@ __global__ void __launch_bounds__(256) filter_mask_kernel(const MaskParams p) {
     end = p.offsets[lo + 1];
   }
   uint32_t* row = p.mask + i * p.stride;
-  for (long long e = beg + lane; e < end; e += 32) {
-    const long long c = p.ptr != nullptr ? static_cast<long long>(p.cols[e]) : p.values[e];
-    if (c >= 0 && c < p.y_rows) atomicOr(row + (c >> 5), 1u << (c & 31));
+  for (long long e0 = beg + lane; e0 < end; e0 += 128) {   // four loads in flight: popular pairs have thousands of answers
+    long long c[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const long long e = e0 + 32 * j;
+      c[j] = e >= end ? -1 : p.ptr != nullptr ? static_cast<long long>(p.cols[e]) : p.values[e];
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (c[j] >= 0 && c[j] < p.y_rows) atomicOr(row + (c[j] >> 5), 1u << (c[j] & 31));
   }
 }
 

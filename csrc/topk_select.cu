@@ -5,12 +5,16 @@
 //   dice_topk_select   best k of each row's candidate list, sorted
 //   dice_topk_scan     the whole search for a few queries: one pass over the table, one launch
 //
-// A block selects by radix: four passes over the values find the k-th largest key bit by bit (histograms of 256 bins in
-// shared memory), a fifth gathers the winners, one warp sorts them.  The work depends on the number of candidates, not on
-// the capacity of the lists.  Scores that are -inf or NaN are never selected; missing places hold (-inf, -1).
+// A block of 256 threads selects in two passes: the k-th largest of the threads' maxima is reached by k values, so only what
+// reaches it (about k values) is gathered, and each of those counts how many are better.  Where more than 256 values reach
+// the bound (ties), a radix search over histograms in shared memory finds the k-th key instead; as the general method it
+// took five passes and its atomics on the few bins that similar scores share (29 us for one query against 14 541 rows).
+// The work depends on the number of candidates, not on the capacity of the lists.  Scores that are -inf or NaN are never
+// selected; missing places hold (-inf, -1).
 //
 // Measured: top 10 of 1024 queries against 2M rows x 256, everything but the pass over the table 500 -> 80 us (running lists
-// per thread over the sample were 346 of it); one query against 14 541 rows 88 -> 31 us (ten launches before).
+// per thread over the sample were 346 of it); one query against 14 541 rows 88 -> 21 us, 12 of them on the device (ten
+// launches before).
 #include "dice_b200.h"
 #include "ptx_sm100.cuh"
 
@@ -34,11 +38,60 @@ __device__ __forceinline__ float value_of(uint32_t key) {
 }
 
 struct Shared {
-  unsigned int hist[256];
-  unsigned int prefix, need, above, ties;
+  union {
+    unsigned int hist[256];
+    uint32_t list[THREADS];      // keys of the threads' maxima, then of the gathered values
+  };
+  int place[THREADS];            // their positions, then their ids
+  unsigned int prefix, need, above, ties, count;
   uint32_t key[KMAX];
   int id[KMAX];
 };
+
+// Number of s.list entries that come before (key, tie) in the order of decreasing keys and increasing ties (s.place, or the
+// position where BY_POSITION); n is rounded up to a multiple of four, the list is padded with zeros.
+template <bool BY_POSITION>
+__device__ __forceinline__ int rank_in_list(const Shared& s, int n, uint32_t key, int tie) {
+  int rank = 0;
+  for (int j = 0; j < n; j += 4) {
+    const uint4 k4 = *reinterpret_cast<const uint4*>(s.list + j);
+    const int4 p4 = BY_POSITION ? make_int4(j, j + 1, j + 2, j + 3) : *reinterpret_cast<const int4*>(s.place + j);
+    rank += (k4.x > key || (k4.x == key && p4.x < tie)) + (k4.y > key || (k4.y == key && p4.y < tie)) +
+            (k4.z > key || (k4.z == key && p4.z < tie)) + (k4.w > key || (k4.w == key && p4.w < tie));
+  }
+  return rank;
+}
+
+// Gathers into s.list / s.place (positions) every value that can be among the best k of get(0 .. n-1), keys of 0 left out;
+// returns their number, or -1 where there are more than 256 of them.
+template <class Get>
+__device__ int gather_best(Shared& s, int n, int k, Get get) {
+  uint32_t bound = 1u;
+  if (n > THREADS) {
+    uint32_t m = 0u;
+    for (int i = threadIdx.x; i < n; i += THREADS) m = max(m, get(i));
+    s.list[threadIdx.x] = m;
+    if (threadIdx.x == 0) s.prefix = 1u;
+    __syncthreads();
+    const int rank = rank_in_list<true>(s, THREADS, m, threadIdx.x);
+    if (rank == k - 1 && m != 0u) s.prefix = m;
+    __syncthreads();
+    bound = s.prefix;
+  }
+  s.list[threadIdx.x] = 0u;
+  s.place[threadIdx.x] = 0x7fffffff;
+  if (threadIdx.x == 0) s.count = 0u;
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += THREADS) {
+    const uint32_t key = get(i);
+    if (key >= bound) {
+      const unsigned int at = atomicAdd(&s.count, 1u);
+      if (at < THREADS) { s.list[at] = key; s.place[at] = i; }
+    }
+  }
+  __syncthreads();
+  return s.count <= THREADS ? static_cast<int>(s.count) : -1;
+}
 
 // k-th largest key among get(0 .. n-1), 0 if fewer than k can be selected; *need = how many of the keys equal to it belong
 // to the best k.  All threads of the block call it and get the result.
@@ -92,9 +145,26 @@ __device__ uint32_t kth_key(Shared& s, int n, int k, Get get, int* need) {
   return key;
 }
 
-// Best k of get(0 .. n-1), sorted (ties by id): put(rank, key, id) is called once per rank by some thread of warp 0.
+// Best k of get(0 .. n-1), sorted (ties by id): put(rank, key, id) is called once per rank by some thread.
 template <class Get, class Id, class Put>
 __device__ void select_best(Shared& s, int n, int k, Get get, Id id, Put put) {
+  const int found = gather_best(s, n, k, get);
+  if (found >= 0) {
+    const int t = threadIdx.x;
+    const uint32_t mine = t < found ? s.list[t] : 0u;
+    const int my_id = t < found ? id(s.place[t]) : 0x7fffffff;
+    __syncthreads();
+    s.place[t] = my_id;
+    __syncthreads();
+    if (t < found) {
+      const int rank = rank_in_list<false>(s, found, mine, my_id);
+      if (rank < k) put(rank, mine, my_id);
+    } else if (t < k) {
+      put(t, 0u, -1);            // fewer than k values
+    }
+    __syncthreads();
+    return;
+  }
   int need;
   const uint32_t kth = kth_key(s, n, k, get, &need);
   if (threadIdx.x < KMAX) { s.key[threadIdx.x] = 0u; s.id[threadIdx.x] = -1; }
@@ -134,8 +204,8 @@ __global__ void __launch_bounds__(THREADS) floor_kernel(const float* __restrict_
   __shared__ Shared s;
   const float* row = gmax + static_cast<size_t>(blockIdx.x) * groups;
   int need;
-  const uint32_t kth = kth_key(s, groups, k, [&](int i) { return key_of(row[i]); }, &need);
-  if (threadIdx.x == 0) {
+  const uint32_t kth = kth_key(s, groups, k, [&](int i) { return key_of(row[i]); }, &need);   // 9 us for 1024 rows of 1024
+  if (threadIdx.x == 0) {                                                                      // maxima; by gathering 17
     floor[blockIdx.x] = value_of(kth);
     cand_count[2 * blockIdx.x] = 0;
     cand_count[2 * blockIdx.x + 1] = 0;
@@ -269,7 +339,7 @@ __global__ void __launch_bounds__(THREADS) scan_kernel(const ScanParams p) {
           p.part_i[out + rank] = id;
         });
   }
-  if (threadIdx.x < 32) __threadfence();   // the winners were written by the first warp
+  __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
     last = atomicAdd(p.done, 1u) == gridDim.x - 1;
@@ -280,8 +350,10 @@ __global__ void __launch_bounds__(THREADS) scan_kernel(const ScanParams p) {
   const int total = static_cast<int>(gridDim.x) * p.k;
   for (int b = 0; b < p.B; ++b) {
     auto slot = [&](int i) -> size_t { return (static_cast<size_t>(i / p.k) * p.B + b) * p.k + i % p.k; };
+    for (int i = threadIdx.x; i < total; i += THREADS) scores[i] = __ldcg(p.part_s + slot(i));
+    __syncthreads();
     select_best(
-        s, total, p.k, [&](int i) { return key_of(__ldcg(p.part_s + slot(i))); },
+        s, total, p.k, [&](int i) { return key_of(scores[i]); },
         [&](int i) { return __ldcg(p.part_i + slot(i)); },
         [&](int rank, uint32_t key, int id) {
           p.out_s[b * p.k + rank] = value_of(key);
@@ -315,7 +387,9 @@ static int launch_scan(const ScanParams& p, int grid, cudaStream_t s) {
     if (cudaFuncSetAttribute(scan_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_SMEM) != cudaSuccess) return -3;
     configured[dev] = true;
   }
-  scan_kernel<D><<<grid, THREADS, static_cast<size_t>(p.B) * p.chunk * 4, s>>>(p);
+  // a block's scores, or in the last block one query's winners of all blocks (148 * 2 * 32 values at most)
+  const size_t smem = 4 * static_cast<size_t>(p.B * p.chunk > grid * p.k ? p.B * p.chunk : grid * p.k);
+  scan_kernel<D><<<grid, THREADS, smem, s>>>(p);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 

@@ -114,7 +114,7 @@ def fused_tail_ranks(model, triples: torch.Tensor, er_vocab, batch_size: int = 4
         for i in range(0, n, batch_size):
             b = triples[i:i + batch_size]
             q, _ = eval_rank.model_queries(model, b[:, :2])
-            ranks[i:i + batch_size] = ranker.ranks_of_pairs(q, b[:, 2], b, er_vocab.num_b, keys, offsets, values)
+            ranker.ranks_of_pairs(q, b[:, 2], b, er_vocab.num_b, keys, offsets, values, out=ranks[i:i + batch_size])
         ranks = ranks.cpu()
         try:
             ranker.check()

@@ -156,22 +156,29 @@ class FusedRanker:
             filt_ptr = filt_ptr.to(torch.int64).contiguous()
             filt_cols = filt_cols.to(torch.int32).contiguous()
             if self.y_offset == 0 and self.y_stride == 1 and self._mask_pays(B, filt_cols.numel()):
-                mask = torch.zeros(B, self._mask_words(), dtype=torch.int32, device=self.device)
+                cleared, mask = self._cleared(B, self._mask_words())
                 kernels.filter_mask(mask, self.table.shape[0], ptr=filt_ptr, cols=filt_cols)
-                filt_ptr = filt_cols = None
+                return self._ranks(q, target, None, None, mask, cleared)
         return self._ranks(q, target, filt_ptr, filt_cols, mask)
+
+    def _cleared(self, B: int, words: int):
+        """Zeros for one batch in one fill: target scores and counts (and the band's counter) and the mask ``[B, words]``."""
+        rows = (B + 3) // 4 * 4
+        buf = torch.zeros(2 * rows + 4 + B * words, dtype=torch.int32, device=self.device)
+        small, mask = buf[:2 * rows + 4], buf[2 * rows + 4:].view(B, words)
+        return (small[:B].view(torch.float32), small[rows:rows + B], small[2 * rows:2 * rows + 2].view(torch.int64)), mask
 
     @torch.no_grad()
     def ranks_of_pairs(self, q: torch.Tensor, target: torch.Tensor, ab: torch.Tensor, num_b: int, keys: torch.Tensor,
-                       offsets: torch.Tensor, values: torch.Tensor) -> torch.Tensor:
+                       offsets: torch.Tensor, values: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """:meth:`ranks` with the filter of query ``i`` given as the pair in the first two columns of ``ab[i]``, looked up on
         the device in a CSR over sorted keys ``a * num_b + b`` (whole table on this device)."""
         assert self.group is None and self.y_offset == 0 and self.y_stride == 1
-        mask = torch.zeros(q.shape[0], self._mask_words(), dtype=torch.int32, device=self.device)
+        cleared, mask = self._cleared(q.shape[0], self._mask_words())
         kernels.filter_mask(mask, self.table.shape[0], ab=ab, num_b=num_b, keys=keys, offsets=offsets, values=values)
-        return self._ranks(q, target, None, None, mask)
+        return self._ranks(q, target, None, None, mask, cleared, out)
 
-    def _ranks(self, q, target, filt_ptr, filt_cols, mask) -> torch.Tensor:
+    def _ranks(self, q, target, filt_ptr, filt_cols, mask, cleared=None, out=None) -> torch.Tensor:
         B = q.shape[0]
         tgt_idx = target.to(torch.int32).contiguous()
         sharded = self.group is not None
@@ -181,8 +188,8 @@ class FusedRanker:
             tgt_part.zero_()   # the count buffers are cleared behind the first barrier: a slower rank may still be
             tgt_score = torch.empty(B, dtype=torch.float32, device=self.device)   # merging the previous call's counts
         else:
-            tgt_part = tgt_score = torch.zeros(B, dtype=torch.float32, device=self.device)
-            greater = torch.zeros(B, dtype=torch.int32, device=self.device)
+            tgt_score, greater, band_count = cleared if cleared is not None else self._cleared(B, 0)[0]
+            tgt_part = tgt_score
             filtered = torch.zeros(B, dtype=torch.int32, device=self.device) if filt_ptr is not None else None
         kw = dict(col_bias=self.col_bias, y_offset=self.y_offset, y_stride=self.y_stride)
         band = {}
@@ -192,7 +199,8 @@ class FusedRanker:
             qk, q_lo, copy, margin = kernels.split_rows(q32, self.d_pad, want_copy=self.d != self.d_pad,
                                                         margin_factor=self.row_norm_max * self.MARGIN[self.d_pad])
             qs, table = copy if copy is not None else q32.contiguous(), self.table_f32
-            band_count = torch.zeros(1, dtype=torch.int64, device=self.device)
+            if sharded:
+                band_count = torch.zeros(1, dtype=torch.int64, device=self.device)
             band = dict(x_lo=q_lo, y_lo=self.table_lo, margin=margin, band_rows=self.band_rows, band_cols=self.band_cols,
                         band_count=band_count)
         else:
@@ -212,7 +220,10 @@ class FusedRanker:
         if self.exact:
             kernels.eval_band_exact(qs, table, self.band_rows, self.band_cols, band_count, tgt_score, greater, **kw)
         if self.group is None:
-            return (greater.add_(1) if filtered is None else 1 + greater - filtered).long()
+            if filtered is not None:
+                greater.sub_(filtered)
+            return torch.add(greater, 1, out=out if out is not None else
+                             torch.empty(B, dtype=torch.int64, device=self.device))
         out = torch.empty(B, dtype=torch.int64, device=self.device)
         self._barrier()                       # every rank's counts are complete
         kernels.merge_ranks(self._tab["greater"], self._tab["filtered"], self.W, out, B, self.status)
@@ -228,7 +239,7 @@ class FusedRanker:
     def _done(self) -> torch.Tensor:
         """Block counter of the scan: calls on one stream follow one another, so there is one per stream."""
         if not torch.cuda.is_current_stream_capturing():
-            key = torch.cuda.current_stream(self.device).cuda_stream
+            key = torch._C._cuda_getCurrentRawStream(self.device.index)
             if key in self._scan_done:
                 return self._scan_done[key]
             if len(self._scan_done) < 64:

@@ -41,8 +41,12 @@ def _call(name: str, anchor: torch.Tensor, *args, others: Sequence[Optional[torc
     for t in others:
         if t is not None and t.device != dev:
             raise KernelError(f"{name}: operands on different devices ({dev} and {t.device})")
-    with torch.cuda.device(dev):
-        rc = getattr(_lib.lib(), name)(*args, torch.cuda.current_stream(dev).cuda_stream)
+    fn = getattr(_lib.lib(), name)
+    if dev.index == torch.cuda.current_device():
+        rc = fn(*args, torch._C._cuda_getCurrentRawStream(dev.index))
+    else:
+        with torch.cuda.device(dev):
+            rc = fn(*args, torch._C._cuda_getCurrentRawStream(dev.index))
     _check(rc, name)
 
 
@@ -685,12 +689,11 @@ def topk_scan(q: torch.Tensor, table: torch.Tensor, k: int, done: torch.Tensor, 
     B, n, dev = q.shape[0], table.shape[0], q.device
     assert 1 <= k <= min(TOPK_MAX, n)
     part = topk_scan_blocks(B, n) * B * k
-    ps = torch.empty(part, dtype=torch.float32, device=dev)
-    pi = torch.empty(part, dtype=torch.int32, device=dev)
+    scratch = torch.empty(2, part, dtype=torch.int32, device=dev)     # scores as bits, positions
     sc = torch.empty(B, k, dtype=torch.float32, device=dev)
     ix = torch.empty(B, k, dtype=torch.int64, device=dev)
     _call("dice_topk_scan", q, _ptr(q), int(q.dtype == torch.bfloat16), q.stride(0), B, q.shape[1], _ptr(table), n,
-          table.shape[1], int(k), _ptr(col_bias), int(y_offset), int(y_stride), _ptr(ps), _ptr(pi), _ptr(done), _ptr(sc),
+          table.shape[1], int(k), _ptr(col_bias), int(y_offset), int(y_stride), _ptr(scratch), scratch.data_ptr() + 4 * part, _ptr(done), _ptr(sc),
           _ptr(ix), others=(table, done, col_bias))
     return sc, ix
 
