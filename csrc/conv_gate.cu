@@ -62,16 +62,14 @@ __device__ __forceinline__ void reduce_to_global(float (&a)[CT], float (&b)[CT],
 #pragma unroll
   for (int c = 0; c < CT; ++c) {
     if (c >= C) break;
-    float sa = warp_sum(a[c]), sb = warp_sum(b[c]);
-    if (lane == 0) { red[warp * 2] = sa; red[warp * 2 + 1] = sb; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double ta = 0, tb = 0;
-      for (int k = 0; k < nw; ++k) { ta += red[k * 2]; tb += red[k * 2 + 1]; }
-      atomicAdd(out_a + c, ta);
-      atomicAdd(out_b + c, tb);
-    }
-    __syncthreads();
+    const float sa = warp_sum(a[c]), sb = warp_sum(b[c]);
+    if (lane == 0) { red[warp * 2 * CT + 2 * c] = sa; red[warp * 2 * CT + 2 * c + 1] = sb; }
+  }
+  __syncthreads();
+  if (threadIdx.x < 2 * C) {   // one thread per total
+    double t = 0;
+    for (int k = 0; k < nw; ++k) t += red[k * 2 * CT + threadIdx.x];
+    atomicAdd((threadIdx.x & 1 ? out_b : out_a) + (threadIdx.x >> 1), t);
   }
 }
 
@@ -83,8 +81,8 @@ __global__ void __launch_bounds__(kThreads) conv_gate_stats(GateShape s, const f
   extern __shared__ float sm[];
   float* ws = sm;                  // C*9
   float* bs = ws + CT * 9;         // C
-  float* red = bs + CT;            // 2 * warps
-  float* xs = red + 2 * (kThreads / 32);
+  float* red = bs + CT;            // 2 * CT * warps
+  float* xs = red + 2 * CT * (kThreads / 32);
   for (int i = threadIdx.x; i < s.C * 9; i += blockDim.x) ws[i] = w[i];
   for (int i = threadIdx.x; i < s.C; i += blockDim.x) bs[i] = bias[i];
   float a[CT], b[CT];
@@ -196,7 +194,7 @@ __global__ void __launch_bounds__(kThreads) conv_gate_bwd_stats(GateShape s, con
   float* mu = sh + CT;
   float* iv = mu + CT;
   float* red = iv + CT;
-  float* xs = red + 2 * (kThreads / 32);
+  float* xs = red + 2 * CT * (kThreads / 32);
   for (int i = threadIdx.x; i < s.C * 9; i += blockDim.x) ws[i] = w[i];
   for (int i = threadIdx.x; i < s.C; i += blockDim.x) {
     bs[i] = bias[i];
@@ -252,8 +250,7 @@ __global__ void __launch_bounds__(kThreads) conv_gate_bwd_apply(GateShape s, int
   float* iv = mu + CT;
   float* kg = iv + CT;    // d gamma / count
   float* kb = kg + CT;    // d beta / count
-  float* red = kb + CT;
-  float* xs = red + kThreads / 32;
+  float* xs = kb + CT;
   const int HW = s.H * s.W, PW = s.W + 2, plane = (s.H + 2) * PW;
   float* dzs = xs + plane;   // C bordered planes
   for (int i = threadIdx.x; i < s.C * 9; i += blockDim.x) ws[i] = w[i];
@@ -312,22 +309,25 @@ __global__ void __launch_bounds__(kThreads) conv_gate_bwd_apply(GateShape s, int
     }
   }
   __syncthreads();
+  // all warps' sums first (the image planes are free now), one thread per total after a single barrier: 80 rounds of two
+  // barriers each took longer than a sample
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  float* part = xs;   // [warps][10 CT]
 #pragma unroll
   for (int c = 0; c < CT; ++c) {
     if (c >= s.C) break;
 #pragma unroll
     for (int t = 0; t < 10; ++t) {
-      float v = warp_sum(t < 9 ? aw[c][t < 9 ? t : 0] : ab[c]);
-      if (lane == 0) red[warp] = v;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        double tot = 0;
-        for (int k = 0; k < nw; ++k) tot += red[k];
-        atomicAdd(dwb + (t < 9 ? c * 9 + t : 9 * s.C + c), tot);
-      }
-      __syncthreads();
+      const float v = warp_sum(t < 9 ? aw[c][t < 9 ? t : 0] : ab[c]);
+      if (lane == 0) part[warp * 10 * CT + c * 10 + t] = v;
     }
+  }
+  __syncthreads();
+  if (threadIdx.x < 10 * s.C) {
+    const int c = threadIdx.x / 10, t = threadIdx.x % 10;
+    double tot = 0;
+    for (int k = 0; k < nw; ++k) tot += part[k * 10 * CT + threadIdx.x];
+    atomicAdd(dwb + (t < 9 ? c * 9 + t : 9 * s.C + c), tot);
   }
 }
 
@@ -349,7 +349,7 @@ int forward_t(GateShape s, int training, const float* X, const float* w, const f
   const double count = (double)s.B * s.H * s.W;
   if (training) {
     if (cudaMemsetAsync(stats, 0, 2 * s.C * sizeof(double), st) != cudaSuccess) return -4;
-    size_t sm = (CT * 10 + 2 * (kThreads / 32) + plane_floats(s.H, s.W)) * sizeof(float);
+    size_t sm = (CT * 10 + 2 * CT * (kThreads / 32) + plane_floats(s.H, s.W)) * sizeof(float);
     conv_gate_stats<CT><<<grid, kThreads, sm, st>>>(s, X, w, bias, stats);
   }
   conv_gate_finalize<<<1, 32, 0, st>>>(s.C, count, training, stats, gamma, beta, run_mean, run_var, momentum, eps, fold);
@@ -365,9 +365,10 @@ int backward_t(GateShape s, int training, const float* X, const float* w, const 
   const double count = (double)s.B * s.H * s.W;
   if (cudaMemsetAsync(bstats, 0, 2 * s.C * sizeof(double), st) != cudaSuccess) return -4;
   if (cudaMemsetAsync(dwb, 0, 10 * s.C * sizeof(double), st) != cudaSuccess) return -4;
-  size_t sm1 = (CT * 14 + 2 * (kThreads / 32) + plane_floats(s.H, s.W)) * sizeof(float);
+  size_t sm1 = (CT * 14 + 2 * CT * (kThreads / 32) + plane_floats(s.H, s.W)) * sizeof(float);
   conv_gate_bwd_stats<CT><<<grid, kThreads, sm1, st>>>(s, X, w, bias, fold, dF, bstats);
-  size_t sm2 = (CT * 16 + kThreads / 32 + (size_t)(1 + s.C) * plane_floats(s.H, s.W)) * sizeof(float);
+  size_t planes = (size_t)(1 + s.C) * plane_floats(s.H, s.W), parts = (size_t)(kThreads / 32) * 10 * CT;
+  size_t sm2 = (CT * 16 + (planes > parts ? planes : parts)) * sizeof(float);
   conv_gate_bwd_apply<CT><<<grid, kThreads, sm2, st>>>(s, training, count, X, w, bias, fold, dF, bstats, dX, dwb);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
