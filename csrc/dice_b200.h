@@ -202,6 +202,7 @@ int dice_bucket_reduce_update(int kind, float* const* p_dst, void* p_mc, const f
                               float weight_decay, float grad_scale, const int* status, void* stream);
 int dice_finish_step(double* acc, float* loss_out, double inv_count, long long* step, const double* const* acc_table,
                      int n_acc, const int* status, void* stream);
+int dice_stage(int n, void* const* dst, const void* const* src, const long long* bytes, void* stream);
 int dice_cast_bf16(const float* src, void* dst, long long n, void* stream);
 int dice_timestamp(unsigned long long* slot, void* stream);
 // Bounded barrier over W ranks on per-rank signal arrays in peer memory (spin_limit 0 = default).

@@ -806,6 +806,27 @@ __global__ void __launch_bounds__(256, KIND < 0 ? 1 : TAIL_B) step_tail_kernel(c
   }
 }
 
+// A batch's arrays into the buffers a captured step reads: one launch instead of one copy (and its gap) per array.
+struct StageParams {
+  void* dst[4];
+  const void* src[4];
+  long long bytes[4];
+  int n;
+};
+
+__global__ void __launch_bounds__(256) stage_kernel(const StageParams p) {
+  const long long tid = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+  const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
+  for (int k = 0; k < p.n; ++k) {
+    const bool wide = ((reinterpret_cast<uintptr_t>(p.dst[k]) | reinterpret_cast<uintptr_t>(p.src[k])) & 15) == 0;
+    const long long n16 = wide ? p.bytes[k] >> 4 : 0;
+    for (long long i = tid; i < n16; i += stride)
+      static_cast<uint4*>(p.dst[k])[i] = static_cast<const uint4*>(p.src[k])[i];
+    for (long long i = (n16 << 2) + tid; i < (p.bytes[k] >> 2); i += stride)   // elements have 4 or 8 bytes
+      static_cast<uint32_t*>(p.dst[k])[i] = static_cast<const uint32_t*>(p.src[k])[i];
+  }
+}
+
 __global__ void cast_bf16_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, long long n) {
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<long long>(gridDim.x) * blockDim.x)
@@ -1032,6 +1053,26 @@ extern "C" int dice_step_tail(int kind, int n_seg, float* const* param, float* c
               : kind == 2 ? step_tail_kernel<2> : step_tail_kernel<3>;
   if (launch_pdl(kern, dim3(static_cast<unsigned>(blocks)), dim3(threads), 0, static_cast<cudaStream_t>(stream), p) != cudaSuccess)
     return -4;
+  return cudaGetLastError() == cudaSuccess ? 0 : -4;
+}
+
+// Copies n <= 4 arrays (bytes[k] a multiple of 4, 4-byte aligned) on the device; dst, src and bytes are host arrays.
+extern "C" int dice_stage(int n, void* const* dst, const void* const* src, const long long* bytes, void* stream) {
+  if (n < 1 || n > 4) return -6;
+  StageParams p{};
+  p.n = n;
+  long long most = 0;
+  for (int k = 0; k < n; ++k) {
+    if (bytes[k] < 0 || (bytes[k] & 3) || ((reinterpret_cast<uintptr_t>(dst[k]) | reinterpret_cast<uintptr_t>(src[k])) & 3)) return -5;
+    p.dst[k] = dst[k];
+    p.src[k] = src[k];
+    p.bytes[k] = bytes[k];
+    most = bytes[k] > most ? bytes[k] : most;
+  }
+  long long blocks = (most / 16 + 255) / 256;
+  if (blocks < 1) blocks = 1;
+  if (blocks > 148 * 8) blocks = 148 * 8;
+  stage_kernel<<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(p);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 

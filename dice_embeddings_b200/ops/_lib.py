@@ -120,6 +120,7 @@ class _Sigs:
     dice_positive_scan = [_p, _p, _i, _p, _p]
     dice_positive_correction = [_p, _p, _p, _p, _p, _p, _p, _p, _p, _f, _f, _i, _i, _i, _i, _p, _i, _p]
     dice_optimizer_step = [_i, _p, _p, _p, _p, _p, _p, _l, _f, _f, _f, _f, _f, _p, _i, _p, _p, _p]
+    dice_stage = [_i, _p, _p, _p, _p]
     dice_cast_bf16 = [_p, _p, _l, _p]
     dice_finish_step = [_p, _p, _d, _p, _p, _i, _p, _p]
     dice_p2p_barrier = [_p, _i, _i, _p, _p, ctypes.c_uint, _p]

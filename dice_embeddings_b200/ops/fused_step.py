@@ -170,8 +170,9 @@ class FusedKvsAllEngine:
             b.gent_tab = K.pointer_table([self.gE], dev)
             b.q_tab = K.pointer_table([b.Q], dev)
             if self.label_mode == "mask":
-                b.mask_q = torch.zeros(n, K.mask_stride(self.NE), dtype=torch.int32, device=dev)
-                b.mask_e = torch.zeros(self.NE, K.mask_stride(n), dtype=torch.int32, device=dev)
+                wq, we = K.mask_stride(self.NE), K.mask_stride(n)      # one buffer: one fill clears both orientations
+                b.masks = torch.zeros(n * wq + self.NE * we, dtype=torch.int32, device=dev)
+                b.mask_q, b.mask_e = b.masks[:n * wq].view(n, wq), b.masks[n * wq:].view(self.NE, we)
             self._bufs[n] = b
         return self._bufs[n]
 
@@ -197,8 +198,7 @@ class FusedKvsAllEngine:
             # of the captured graph) while the main stream gathers and composes the queries
             self._side.wait_stream(main)
             with torch.cuda.stream(self._side):
-                b.mask_q.zero_()
-                b.mask_e.zero_()
+                b.masks.zero_()
                 K.build_label_masks(b.dp, self.offsets, self.values, n, 1, 0, b.mask_q, b.mask_e, first=b.first)
         K.lookup_compose_vec(self.code, self.normalize, b.h, b.r, None, b.ent_tab, 1, self.NE, self.NR, self.R,
                              self.coeff, b.q_tab, 1, 0, 0, None, None, 0, n, self.D, self.status, idx_stride=2)
@@ -310,8 +310,7 @@ class FusedKvsAllEngine:
         x, dp = batch[0], batch[1]
         n = x.shape[0]
         b = self._buffers(n)
-        b.x_in.copy_(x)
-        b.dp.copy_(dp)
+        K.stage((b.x_in, x), (b.dp, dp))
         self._run(b, n)
         return self.loss_out[0]
 

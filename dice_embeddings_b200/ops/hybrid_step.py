@@ -194,8 +194,7 @@ class ExternalQueryEngine:
                 return self._step(x, dp)
         graph, loss, grads = entry
         b = self._buffers(x.shape[0])
-        b.x_in.copy_(x)
-        b.dp.copy_(dp)
+        K.stage((b.x_in, x), (b.dp, dp))
         graph.replay()
         for p, g in grads:
             p.grad = g

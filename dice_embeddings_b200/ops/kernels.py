@@ -448,6 +448,23 @@ def sparse_rows_optimizer(kind: int, param, grad, m, v, shadow, touched: torch.T
           float(weight_decay), others=(grad, m, v, shadow, touched, step))
 
 
+def stage(*pairs) -> None:
+    """Copy ``src`` into ``dst`` for up to four ``(dst, src)`` pairs: one launch where all of them are contiguous tensors of
+    equal shape and type (4 or 8 bytes per element) on one device, ``dst.copy_(src)`` otherwise."""
+    dev = pairs[0][0].device
+    for dst, src in pairs:
+        if dst.device != dev or src.device != dev or dst.dtype != src.dtype or dst.shape != src.shape \
+                or not dst.is_contiguous() or not src.is_contiguous() or dst.element_size() not in (4, 8) \
+                or (dst.data_ptr() | src.data_ptr()) & 3 or type(src) is not torch.Tensor or src.is_conj() or src.is_neg():
+            for d, s in pairs:
+                d.copy_(s)
+            return
+    n = len(pairs)
+    _call("dice_stage", pairs[0][0], n, (ctypes.c_void_p * n)(*[d.data_ptr() for d, _ in pairs]),
+          (ctypes.c_void_p * n)(*[s.data_ptr() for _, s in pairs]),
+          (ctypes.c_longlong * n)(*[d.numel() * d.element_size() for d, _ in pairs]))
+
+
 SAMPLED_DRAW = {"given": 0, "corrupt": 1, "tails": 2}
 
 

@@ -178,20 +178,17 @@ class FusedSampledEngine:
             pos = batch[0]
             key = (pos.shape[0], 1 + self.neg_ratio, "corrupt")
             b = self._buffers(key)
-            b.pos.copy_(pos)
+            K.stage((b.pos, pos))
         elif self.st == "NegSample":
             x, y = batch[0], batch[1]
             key = (x.shape[0], 1, "given")
             b = self._buffers(key)
-            b.x.copy_(x)
-            b.labels.copy_(y.reshape(-1, 1))
+            K.stage((b.x, x), (b.labels, y.reshape(-1, 1)))
         else:
             x, idx, y = batch[0], batch[1], batch[2]
             key = (x.shape[0], idx.shape[1], "given")
             b = self._buffers(key)
-            b.x.copy_(x)
-            b.cand.copy_(idx)
-            b.labels.copy_(y)
+            K.stage((b.x, x), (b.cand, idx), (b.labels, y))
         self._run(b, key)
         return self.loss_out[0]
 

@@ -547,3 +547,21 @@ def test_optimizer_quotient_over_the_range_of_second_moments(kind):
         tol = 2.0 ** -24 * 8 * want.abs() + 2.0 ** -24 * 8 * want.abs() + 1e-40   # powers of beta: as many units again
     assert torch.isfinite(w).all() and float(w[128:160].abs().max()) == (0.0 if kind != 3 else float(w[128:160].abs().max()))
     assert ((w.double() - want).abs() <= tol).all(), float(((w.double() - want).abs() / tol).max())
+
+
+@pytest.mark.parametrize("sizes", [(1,), (3, 1), (4096 * 2, 4096), (1025, 7, 333, 2)])
+def test_stage_copies_every_array(sizes):
+    """Arrays of odd lengths, 4- and 8-byte elements, a source that starts off a 16-byte boundary; what one launch does not
+    take (another type, a strided source) is copied all the same."""
+    dst, src = [], []
+    for i, n in enumerate(sizes):
+        dtype = (torch.int64, torch.float32)[i % 2]
+        full = torch.arange(n + 1, device=DEV).to(dtype) + 1
+        src.append(full[1:] if i % 3 == 1 else full[:n])
+        dst.append(torch.zeros(n, dtype=dtype, device=DEV))
+    K.stage(*zip(dst, src))
+    assert all(torch.equal(d, s) for d, s in zip(dst, src))
+    strided = torch.arange(40, device=DEV).view(20, 2)[:, 0]
+    a, b = torch.zeros(20, dtype=torch.int64, device=DEV), torch.zeros(20, dtype=torch.int64, device=DEV)
+    K.stage((a, strided), (b, strided.to(torch.int32)))
+    assert torch.equal(a, strided) and torch.equal(b, strided)
