@@ -187,7 +187,13 @@ kvsall_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     // The tensor pipe queues only a few MMAs, so a probe of an mbarrier between two of them leaves a bubble of about 90
     // cycles (measured: 1650 cycles per 96-row tile without probes inside a GEMM, 2300 with one per 64-column slab).  All
     // probes therefore sit between GEMMs, back to back so that their latencies overlap, and a tile has one load barrier.
-    if (lane == 0) {
+    // All lanes run this branch and one elected lane issues each MMA and commit: the operands then are warp-uniform values.
+    // Issued from a branch of a single lane, the sixteen MMAs of the first GEMM took 1560 cycles whether 64 or 96 columns
+    // wide.  A tile at D = 256: 2300 -> 2000 cycles; entity / query role 262144 x 4096 x 256 895 / 871 -> 830 / 815 us,
+    // x 128 679 / 519 -> 527 / 404 us, 2M x 8192 x 256 14.6 / 16.0 -> 13.3 / 15.0 ms.  What bounds a tile now is the chain
+    // of a Y stage (load, first GEMM, epilogue, second GEMM: about 6000 cycles) over three stages; five stages of 64 rows
+    // were slower (the first GEMM of half the width costs the same).
+    {
       constexpr uint32_t IDESC_G1 = make_idesc_bf16(BLOCK_X, C::BY, 0, 0);  // S = X · Yᵀ, both K-major
       constexpr uint32_t IDESC_G2 = make_idesc_bf16(BLOCK_X, D, 0, 1);        // out += dS · Y, Y read MN-major
       // descriptors are built once; per MMA only the 14-bit start-address field (16-byte units) is advanced
@@ -197,7 +203,7 @@ kvsall_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
 
       auto issue_g1 = [&](uint32_t gi) {
         const uint32_t st = gi % C::NSTAGE;
-        stamp(gi, 1);
+        if (lane == 0) stamp(gi, 1);
         tc_fence_after();
         const uint64_t yd = ydesc_g1 + st * (C::Y_BYTES >> 4);
         const uint32_t b = gi % C::NBUF;
@@ -208,15 +214,15 @@ kvsall_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
           for (int kk = 0; kk < 4; ++kk) {
             const uint32_t xo = sl * (C::XSLAB >> 4) + kk * 2;  // 16 bf16 = 32 bytes inside the swizzle span
             const uint32_t yo = sl * (C::YSLAB >> 4) + kk * 2;
-            if (sl == 0 && kk == 0) mma_ss(d_tmem, xdesc + xo, yd + yo, IDESC_G1, 0u);
-            else mma_ss(d_tmem, xdesc + xo, yd + yo, IDESC_G1, 1u);
+            if (sl == 0 && kk == 0) mma_ss_warp(d_tmem, xdesc + xo, yd + yo, IDESC_G1, 0u);
+            else mma_ss_warp(d_tmem, xdesc + xo, yd + yo, IDESC_G1, 1u);
           }
         }
-        tc_commit(s_full + b);
+        tc_commit_warp(s_full + b);
       };
       auto issue_g2 = [&](uint32_t gi, bool first, bool last) {
         const uint32_t st = gi % C::NSTAGE;
-        stamp(gi, 2);
+        if (lane == 0) stamp(gi, 2);
         tc_fence_after();
         const uint64_t yd = ydesc_g2 + st * (C::Y_BYTES >> 4);
         const uint32_t a_base = tmem_s0 + (gi % C::NBUF) * C::BY;
@@ -226,11 +232,11 @@ kvsall_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
           const uint32_t a_tmem = a_base + 32 * (k >> 1) + 8 * (k & 1);
           // Y tile as [K = BY rows, N = D]: N blocks of 64 are one slab apart, groups of 8 K-rows 1024 B apart;
           // 16 K-rows = 2048 bytes
-          if (k == 0) mma_ts(tmem_out, a_tmem, yd, IDESC_G2, first ? 0u : 1u);
-          else mma_ts(tmem_out, a_tmem, yd + k * 128, IDESC_G2, 1u);
+          if (k == 0) mma_ts_warp(tmem_out, a_tmem, yd, IDESC_G2, first ? 0u : 1u);
+          else mma_ts_warp(tmem_out, a_tmem, yd + k * 128, IDESC_G2, 1u);
         }
-        tc_commit(y_empty + st);
-        if (last) tc_commit(dx_full);
+        tc_commit_warp(y_empty + st);
+        if (last) tc_commit_warp(dx_full);
       };
 
       TileCursor c1, c2;
@@ -238,20 +244,21 @@ kvsall_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
       c2.start(w_begin, w_end, p.map);
       uint32_t g1 = 0, g2 = 0, idle = 0;
       bool ok = true;
-      while (!c2.done() && ok && !*s_abort) {
+      auto all = [](bool x) { return __all_sync(0xffffffffu, x) != 0; };   // the same in every lane, and known to be
+      while (!c2.done() && ok && all(*s_abort == 0)) {
         bool progressed = false;
         // readiness only ever goes from false to true until this thread consumes it
-        const bool ds_ready = mbar_test_wait(ds_full + g2 % C::NBUF, (g2 / C::NBUF) & 1);
-        const bool y_ready = mbar_test_wait(y_full + g1 % C::NSTAGE, (g1 / C::NSTAGE) & 1);
-        if (g2 < g1 && ds_ready && (!c2.first() || mbar_test_wait(dx_empty, (c2.seg & 1) ^ 1))) {
+        const bool ds_ready = all(mbar_test_wait(ds_full + g2 % C::NBUF, (g2 / C::NBUF) & 1));
+        const bool y_ready = all(mbar_test_wait(y_full + g1 % C::NSTAGE, (g1 / C::NSTAGE) & 1));
+        if (g2 < g1 && ds_ready && (!c2.first() || all(mbar_test_wait(dx_empty, (c2.seg & 1) ^ 1)))) {
           issue_g2(g2, c2.first(), c2.last());
           ++g2;
           c2.advance();
           progressed = true;
         }
-        if (!c1.done() && g1 - g2 < C::NBUF && y_ready && (!c1.first() || mbar_test_wait(x_full, c1.seg & 1))) {
+        if (!c1.done() && g1 - g2 < C::NBUF && y_ready && (!c1.first() || all(mbar_test_wait(x_full, c1.seg & 1)))) {
           issue_g1(g1);
-          if (c1.last()) tc_commit(x_empty);  // last S GEMM of the segment: the X buffer may be refilled
+          if (c1.last()) tc_commit_warp(x_empty);  // last S GEMM of the segment: the X buffer may be refilled
           ++g1;
           c1.advance();
           progressed = true;
@@ -264,7 +271,7 @@ kvsall_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
           __nanosleep(32);
         }
       }
-      if (!ok) fail(ST_TIMEOUT_MMA);
+      if (!ok && lane == 0) fail(ST_TIMEOUT_MMA);
     }
   } else {
     // =========================================================================== epilogue warps

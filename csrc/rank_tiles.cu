@@ -18,7 +18,8 @@
 // within about 1.7e-4 |x| |y| of the exact product (D = 256) instead of 2^-8, and the undecided band is more than 20 times
 // narrower.  The second X plane then holds the lo part of the same 128 rows.
 //
-// Measured: 8192 queries x 2M rows x 256, COUNT 8855 -> 6808 us (1.26 PFLOP/s); 1024 x 2M x 256, COLLECT 1348 -> 1070 us;
+// Measured: 8192 queries x 2M rows x 256, COUNT 8855 -> 6808 us, with warp-uniform MMA issue (see mma_ts_warp)
+// 4096 x 262144 x 256 441 -> 400 us (1.37 PFLOP/s); 1024 x 2M x 256, COLLECT 1348 -> 1070 us;
 // evaluation of 20 466 queries x 14 541 x 256 (band, filters and counts) 15.8 -> 0.56 ms on the device (75 us a batch of 4096
 // for the three GEMMs; with the parts of a 64-row tile side by side in one stage 116 us, the MMA being half as wide).
 //
@@ -198,54 +199,56 @@ rank_tiles_kernel(const __grid_constant__ CUtensorMap tmap_y, const __grid_const
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    // all lanes run this branch; one elected lane issues each MMA and commit
+    {
       constexpr uint32_t IDESC = make_idesc_bf16(128, C::BY, 0, 0);
       const uint64_t ydesc = make_sw128_desc(smem_u32(sY), 16, 1024);
       uint32_t g = 0, ycount = 0, seg = 0;
       bool ok = true;
+      auto all = [](bool x) { return __all_sync(0xffffffffu, x) != 0; };   // the same in every lane, and known to be
       // d (+)= (plane of X) . (Y tile at descriptor yd)^T
       auto gemm = [&](uint32_t d_tmem, uint32_t plane, uint64_t yd, bool first) {
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
           const uint32_t off = (k >> 2) * (C::YSLAB >> 4) + (k & 3) * 2;
-          mma_ts(d_tmem, tmem_base + plane * (D / 2) + k * 8, yd + off, IDESC, (first && k == 0) ? 0u : 1u);
+          mma_ts_warp(d_tmem, tmem_base + plane * (D / 2) + k * 8, yd + off, IDESC, (first && k == 0) ? 0u : 1u);
         }
       };
-      for (long long w = w_begin; w < w_end && ok && !*s_abort;) {
+      for (long long w = w_begin; w < w_end && ok && all(*s_abort == 0);) {
         int x, y0, run;
         p.map.locate(w, x, y0, run);
         const int n = static_cast<int>(min(static_cast<long long>(run), w_end - w));
         const int units = units_of(x);
-        if (!mbar_wait_bounded(x_full, seg & 1, s_abort)) { ok = false; break; }
+        if (!all(mbar_wait_bounded(x_full, seg & 1, s_abort))) { ok = false; break; }
         for (int t = 0; t < n && ok; ++t, ++ycount) {
           uint32_t st = ycount % C::NSTAGE;
           uint64_t yd = ydesc + st * (C::Y_BYTES >> 4);
-          if (!mbar_wait_bounded(y_full + st, (ycount / C::NSTAGE) & 1, s_abort)) { ok = false; break; }
+          if (!all(mbar_wait_bounded(y_full + st, (ycount / C::NSTAGE) & 1, s_abort))) { ok = false; break; }
           for (int u = 0; u < units; ++u, ++g) {
             const uint32_t b = g % C::NBUF;
-            if (!mbar_wait_bounded(s_empty + b, ((g / C::NBUF) & 1) ^ 1, s_abort)) { ok = false; break; }
+            if (!all(mbar_wait_bounded(s_empty + b, ((g / C::NBUF) & 1) ^ 1, s_abort))) { ok = false; break; }
             tc_fence_after();
             const uint32_t d_tmem = tmem_base + C::S_COL + b * C::BY;
             gemm(d_tmem, u, yd, true);
             if constexpr (SPLIT) {
               gemm(d_tmem, 1, yd, false);
-              tc_commit(y_empty + st);
+              tc_commit_warp(y_empty + st);
               ++ycount;                       // the lo part is the next stage
               st = ycount % C::NSTAGE;
               yd = ydesc + st * (C::Y_BYTES >> 4);
-              if (!mbar_wait_bounded(y_full + st, (ycount / C::NSTAGE) & 1, s_abort)) { ok = false; break; }
+              if (!all(mbar_wait_bounded(y_full + st, (ycount / C::NSTAGE) & 1, s_abort))) { ok = false; break; }
               tc_fence_after();
               gemm(d_tmem, 0, yd, false);
             }
-            tc_commit(s_full + b);
+            tc_commit_warp(s_full + b);
           }
-          if (ok) tc_commit(y_empty + st);
+          if (ok) tc_commit_warp(y_empty + st);
         }
-        if (ok) tc_commit(x_empty);
+        if (ok) tc_commit_warp(x_empty);
         w += n;
         ++seg;
       }
-      if (!ok) fail(ST_TIMEOUT_MMA);
+      if (!ok && lane == 0) fail(ST_TIMEOUT_MMA);
     }
   } else {
     // ------------------------------------------------------------------------- epilogue warps

@@ -234,12 +234,17 @@ def test_external_query_step_from_a_graph_equals_plain_launches(name, optim):
     a, b = (torch.stack(x) for x in losses)
     assert len({x.data_ptr() for x in losses[0]}) == 12 and a.unique().numel() > 6   # every step's loss is its own tensor
     assert torch.allclose(a, b, rtol=1e-4), (a, b)
+    # Adam divides a gradient by its own size: an element whose gradient is rounding noise (atomics in another order) may move
+    # by the learning rate either way, 2 * (8 * 1e-3 + 4 * 5e-4) = 0.02 at most over the run.  Few elements are like that,
+    # so the 2-norm of the change is compared; the bias ahead of the batch normalisation is (its true gradient is zero),
+    # and with it the running mean.
     for s, (name, p), q in zip(start, engines[0][2].named_parameters(), engines[1][2].parameters()):
         if name.endswith("conv2d.bias"):
-            continue   # batch normalisation takes its gradient to zero: Adam scales the rounding noise up
-        assert (p - q).abs().max() <= 2e-2 * (q - s).abs().max() + 1e-6
+            assert (p - q).abs().max() <= 0.02
+            continue
+        assert (p - q).norm() <= 1e-2 * (q - s).norm() + 1e-6, (name, float((p - q).norm()), float((q - s).norm()))
     for (n1, x), (_, y) in zip(engines[0][2].named_buffers(), engines[1][2].named_buffers()):
-        assert torch.allclose(x.float(), y.float(), rtol=1e-3, atol=1e-5), n1
+        assert torch.allclose(x.float(), y.float(), rtol=1e-3, atol=0.02 if n1.endswith("running_mean") else 1e-5), n1
 
 
 def test_external_query_step_with_hooks_runs_as_plain_launches():
