@@ -726,6 +726,7 @@ __device__ __forceinline__ void optimizer_segment(const OptParams& p, long long 
 // The sweep over a local gradient with aligned buffers, the rule fixed at compile time.  Bound by memory (seven or eight
 // passes of 4 bytes per weight and the bf16 copy), so what counts is the number of loads in flight: few registers and as
 // many resident warps as they allow.
+// The moments are the first to leave L2, so that weights and gradient, which the rest of the step reads, stay.
 template <int KIND>
 __device__ __forceinline__ void local_segment(const OptParams& p, const OptStepConsts& c) {
   const long long n4 = p.n >> 2;
@@ -769,10 +770,10 @@ __device__ __forceinline__ void local_segment(const OptParams& p, const OptStepC
   }
 }
 
-// KIND 0..3: all segments local and aligned; -1: the general form (gradients summed over ranks, any alignment)
-// Resident blocks per SM.  Measured 4 / 6 / 8 with the moments evicted first: 14 541 x 256 31 / 32 / 36 us, 40 559 x 128
-// 32 / 33 / 39 us (46 with the general form), 2 million x 256 3.57 / 3.69 / 4.06 ms (3.50: 5 TB/s either way, more warps only
-// spread the nine streams further).
+// KIND 0..3: all segments local and aligned, a few times L2 at most; -1: the general form (gradients summed over ranks, any
+// alignment, large tables)
+// Resident blocks per SM.  Measured 4 / 6 / 8: 14 541 x 256 31 / 32 / 36 us, 40 559 x 128 32 / 33 / 39 us (46 with the
+// general form).
 constexpr int TAIL_B = 4;
 template <int KIND>
 __global__ void __launch_bounds__(256, KIND < 0 ? 1 : TAIL_B) step_tail_kernel(const StepTailParams p) {
@@ -1037,7 +1038,9 @@ extern "C" int dice_step_tail(int kind, int n_seg, float* const* param, float* c
   p.n_seg = n_seg;
   p.acc = acc; p.loss_out = loss_out; p.inv_count = inv_count; p.step_rw = step; p.acc_table = acc_table;
   p.n_acc = n_acc; p.done = done; p.status = status;
-  bool local = kind >= 0 && kind <= 3;
+  // Measured with a cold L2, this form / the general one: 14 541 x 256 32 / 40 us, 60 000 x 256 95 / 105 us, 150 000 x 256
+  // (614 MB of weights, gradient and moments) 228 / 230 us, 600 000 x 256 892 / 868 us, 2 million x 256 2.96 / 2.89 ms.
+  bool local = kind >= 0 && kind <= 3 && total * 16 <= (512ll << 20);
   for (int s = 0; s < n_seg; ++s) {
     const OptParams& o = p.seg[s];
     local &= o.grad_table == nullptr && o.grad_mc == nullptr && (reinterpret_cast<uintptr_t>(o.shadow) & 7) == 0 &&
