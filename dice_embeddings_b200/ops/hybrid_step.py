@@ -194,7 +194,7 @@ class ExternalQueryEngine:
                 return self._step(x, dp)
         graph, loss, grads = entry
         b = self._buffers(x.shape[0])
-        K.stage((b.x_in, x), (b.dp, dp))
+        K.stage((b.x_in, x[:, :2]), (b.dp, dp))
         graph.replay()
         for p, g in grads:
             p.grad = g
@@ -230,7 +230,7 @@ class ExternalQueryEngine:
             if o._optimizer_step_pre_hooks or o._optimizer_step_post_hooks:
                 return None
             for g in o.param_groups:
-                opt.append(tuple((k, v) for k, v in sorted(g.items()) if k != "params" and not isinstance(v, torch.Tensor)))
+                opt.append(tuple((k, repr(v)) for k, v in sorted(g.items()) if k != "params"))
                 if any(isinstance(v, torch.Tensor) for k, v in g.items() if k != "params"):
                     return None
                 opt += [t.data_ptr() for p in g["params"] for t in o.state.get(p, {}).values() if isinstance(t, torch.Tensor)]

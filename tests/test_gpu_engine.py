@@ -258,6 +258,8 @@ def test_external_query_step_with_hooks_runs_as_plain_launches():
     for _ in range(3):
         eng.step(ds.make_batch(idx)[:1] + (idx,))
     assert len(eng._graphs) == 1
+    triples = torch.cat((ds.make_batch(idx)[0][:, :2], idx[:, None] % 300), 1)      # further columns are not looked at
+    assert torch.isfinite(eng.step((triples, idx))) and len(eng._graphs) == 1
     calls = []
     handle = model.fc1.register_forward_hook(lambda *a: calls.append(1))
     eng.step(ds.make_batch(idx)[:1] + (idx,))
