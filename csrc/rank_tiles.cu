@@ -378,11 +378,9 @@ rank_tiles_kernel(const __grid_constant__ CUtensorMap tmap_y, const __grid_const
                   if (lane == 31) base = atomicAdd(p.band_count, static_cast<unsigned long long>(incl));
                   base = __shfl_sync(0xffffffffu, base, 31);
                   long long at = static_cast<long long>(base) + incl - nb;
-                  if (band != 0u && at + nb > p.band_cap) {
-                    atomicCAS(p.status, 0, ST_INBOX_OVERFLOW);
-                    band = 0u;
-                  }
-                  while (band) {
+                  // what still fits is written: the second pass reads every slot below min(count, capacity)
+                  if (band != 0u && at + nb > p.band_cap) atomicCAS(p.status, 0, ST_INBOX_OVERFLOW);
+                  while (band != 0u && at < p.band_cap) {
                     const int i = __ffs(band) - 1;
                     band &= band - 1;
                     p.band_rows[at] = x_global[u];

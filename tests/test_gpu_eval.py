@@ -296,3 +296,23 @@ def test_split_scores_stay_within_the_margin():
         beats = exact > ts[:, None].double()
         beats[torch.arange(400, device=DEV), tgt.long()] = False
         assert torch.equal(greater.long(), (beats & ~band).sum(1))
+
+
+@pytest.mark.parametrize("split", [False, True])
+@pytest.mark.parametrize("cap", [1, 45, 1000])
+def test_full_band_list_has_no_gaps(split, cap):
+    """A list that runs full is reported and holds a listed pair in every slot: the second pass reads all of them.  Margins
+    of infinity put every pair but the targets' own into the band."""
+    nx, ny, D = 70, 500, 64
+    x, y = _operands(nx, ny, D, cap)
+    lo = dict(x_lo=torch.zeros_like(x), y_lo=torch.zeros_like(y)) if split else {}
+    tgt = torch.randint(0, ny, (nx,), device=DEV, dtype=torch.int32)
+    rows, cols = (torch.full((cap,), -1, dtype=torch.int32, device=DEV) for _ in range(2))
+    count = torch.zeros(1, dtype=torch.int64, device=DEV)
+    greater, status = torch.zeros(nx, dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    K.rank_count(x, y, torch.zeros(nx, device=DEV), tgt, greater, status, margin=torch.full((nx,), float("inf"), device=DEV),
+                 band_rows=rows, band_cols=cols, band_count=count, **lo)
+    assert int(status) != 0 and int(count) == nx * (ny - 1) and int(greater.sum()) == 0
+    r, c = rows.long(), cols.long()
+    assert ((r >= 0) & (r < nx) & (c >= 0) & (c < ny)).all() and (c != tgt.long()[r.clamp_min(0)]).all()
+    assert torch.unique(r * ny + c).numel() == cap
