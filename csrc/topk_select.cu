@@ -20,6 +20,8 @@
 
 #include <math_constants.h>
 
+#include <cstddef>
+
 namespace dice {
 namespace topk {
 
@@ -37,7 +39,7 @@ __device__ __forceinline__ float value_of(uint32_t key) {
   return __uint_as_float((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key);
 }
 
-struct Shared {
+struct alignas(16) Shared {     // list and place are read four values at a time
   union {
     unsigned int hist[256];
     uint32_t list[THREADS];      // keys of the threads' maxima, then of the gathered values
@@ -47,6 +49,7 @@ struct Shared {
   uint32_t key[KMAX];
   int id[KMAX];
 };
+static_assert(offsetof(Shared, list) % 16 == 0 && offsetof(Shared, place) % 16 == 0, "16-byte loads");
 
 // Number of s.list entries that come before (key, tie) in the order of decreasing keys and increasing ties (s.place, or the
 // position where BY_POSITION); n is rounded up to a multiple of four, the list is padded with zeros.
