@@ -45,7 +45,8 @@ __device__ __forceinline__ float opt_div(float a, float b) {
   const float r = fmaf(fmaf(-b, r0, 1.f), r0, r0);
   const float q = a * r;
   const float res = fmaf(fmaf(-b, q, a), r, q);
-  return r0 == 0.f || fabsf(r0) == __int_as_float(0x7f800000) ? a * r0 : res;   // b infinite or zero
+  if (r0 == 0.f || fabsf(r0) == __int_as_float(0x7f800000)) return a * r0;   // b infinite or zero
+  return fabsf(q) == __int_as_float(0x7f800000) ? q : res;                    // overflow: the residual is not a number
 }
 
 // One parameter element: returns the updated weight; m / v are updated in place (registers).

@@ -549,6 +549,23 @@ def test_optimizer_quotient_over_the_range_of_second_moments(kind):
     assert ((w.double() - want).abs() <= tol).all(), float(((w.double() - want).abs() / tol).max())
 
 
+@pytest.mark.parametrize("tail", [False, True])
+def test_adopt_step_with_an_overflowing_quotient(tail):
+    """A quotient beyond the largest float is clipped in its own direction: gradients that are infinite, or large over a second
+    moment of zero, through the general sweep and through the step tail."""
+    inf = float("inf")
+    g = torch.tensor([inf, -inf, 1e33, -1e33, 3e38, -3e38, 1.0, -1.0], device=DEV)
+    v = torch.tensor([1.0, 1e30, 0.0, 0.0, 1e-12, 0.0, 1e-12, 1.0], device=DEV)
+    m, w, step = torch.zeros(8, device=DEV), torch.zeros(8, device=DEV), torch.full((1,), 15, dtype=torch.int64, device=DEV)
+    sign, ratio = torch.sign(g), (g / v.sqrt().clamp_min(1e-6)).abs().clamp(max=15 ** 0.25)
+    if tail:
+        K.StepTail(3, [dict(param=w, grad=g, m=m, v=v)], step, None, finish=False).launch(0.1, 0.9, 0.999, 1e-6, 0.0)
+    else:
+        K.optimizer_step(3, w, g, m, v, None, step, 0.1, 0.9, 0.999, 1e-6, 0.0)
+    want = -0.1 * 0.1 * sign * ratio                 # lr (1 - beta1) times the clipped quotient, from moments of zero
+    assert torch.allclose(w, want, rtol=1e-5), (w, want)
+
+
 @pytest.mark.parametrize("sizes", [(1,), (3, 1), (4096 * 2, 4096), (1025, 7, 333, 2)])
 def test_stage_copies_every_array(sizes):
     """Arrays of odd lengths, 4- and 8-byte elements, a source that starts off a 16-byte boundary; what one launch does not
