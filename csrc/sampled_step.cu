@@ -370,9 +370,9 @@ __global__ void __launch_bounds__(GRAD_THREADS, GRAD_B) grad_kernel(const GradPa
       for (int s0 = 0; s0 < count; s0 += CH) {
         F row[CH];
 #pragma unroll
-        for (int j = 0; j < CH; ++j) {   // -1 past the end or out of range: row 0 stands in
-          const long long e = __shfl_sync(0xffffffffu, id, s0 + j);
-          frag_load<K, V, NC>(p.ent + (e < 0 ? 0ll : e) * p.D, w, lane, row[j]);
+        for (int j = 0; j < CH; ++j) {   // -1 past the end or out of range: the group's own fixed row stands in (with g = 0 it
+          const long long e = __shfl_sync(0xffffffffu, id, s0 + j);   // adds nothing, unless it is inf or NaN, as is then the group)
+          frag_load<K, V, NC>(p.ent + (e < 0 ? fix_id : e) * p.D, w, lane, row[j]);
         }
         float a[CH];
 #pragma unroll

@@ -245,3 +245,19 @@ def test_sparse_update_of_drawn_tails(name, D, NE, B, k):
     assert (vE - want_v).abs().max() < 1e-6 * g * g + 1e-12
     assert (E - want_p).abs().max() < 0.01 * (1e-5 * g + 1e-9) / 1e-3 * 10 + 1e-6
     assert int(touched.sum()) == 0 and int((head != -1).sum()) == 0
+
+
+@pytest.mark.parametrize("name,D,C", [("DistMult", 64, 6), ("DistMult", 512, 2), ("ComplEx", 128, 33), ("TransE", 100, 5), ("QMult", 256, 1),
+                                      ("OMult", 512, 3)])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_a_row_that_is_not_a_number_stays_where_it_is(name, D, C, bad):
+    """Entities that no triple of the batch names do not reach it, whatever they hold: candidate counts that leave part of the
+    rows in flight empty."""
+    _, m = _pair(name, D, NE=100, scoring="1vsSample")
+    with torch.no_grad():
+        m.entity_embeddings.weight[0] = bad
+        m.entity_embeddings.weight[99] = bad
+    eng = FusedSampledEngine(m, "1vsSample", lr=1.0, device=DEV, use_graph=False)
+    x = torch.stack((torch.randint(1, 99, (30,), device=DEV), torch.randint(0, 12, (30,), device=DEV)), 1)
+    loss = eng.step((x, torch.randint(1, 99, (30, C), device=DEV), torch.rand(30, C, device=DEV).round()))
+    assert torch.isfinite(loss) and torch.isfinite(eng.E[1:99]).all() and torch.isfinite(eng.R).all()
