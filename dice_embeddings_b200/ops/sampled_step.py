@@ -173,6 +173,8 @@ class FusedSampledEngine:
         * NegSample: ``(x [N, 3], labels [N])`` as built by the dataset, or ``(positives [B, 3],)`` to have the
           corruptions drawn by the device generator;
         * 1vsSample / KvsSample: ``(x [B, 2], candidate ids [B, C], labels [B, C])``.
+
+        Further columns of ``x`` are not looked at.
         """
         if self.st == "NegSample" and (len(batch) == 1 or batch[1] is None):
             pos = batch[0]
@@ -183,12 +185,12 @@ class FusedSampledEngine:
             x, y = batch[0], batch[1]
             key = (x.shape[0], 1, "given")
             b = self._buffers(key)
-            K.stage((b.x, x), (b.labels, y.reshape(-1, 1)))
+            K.stage((b.x, x[:, :3]), (b.labels, y.reshape(-1, 1)))
         else:
             x, idx, y = batch[0], batch[1], batch[2]
             key = (x.shape[0], idx.shape[1], "given")
             b = self._buffers(key)
-            K.stage((b.x, x), (b.cand, idx), (b.labels, y))
+            K.stage((b.x, x[:, :2]), (b.cand, idx), (b.labels, y))
         self._run(b, key)
         return self.loss_out[0]
 

@@ -240,7 +240,7 @@ class ShardedSampledEngine:
             key = (x.shape[0], idx.shape[1], 0)
             b = self._buffers(key)
             if self.W == 1:
-                b.x.copy_(x)
+                b.x.copy_(x[:, :2])
             else:
                 b.h.copy_(x[:, 0])
                 b.r.copy_(x[:, 1])

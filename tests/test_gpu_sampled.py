@@ -261,3 +261,30 @@ def test_a_row_that_is_not_a_number_stays_where_it_is(name, D, C, bad):
     x = torch.stack((torch.randint(1, 99, (30,), device=DEV), torch.randint(0, 12, (30,), device=DEV)), 1)
     loss = eng.step((x, torch.randint(1, 99, (30, C), device=DEV), torch.rand(30, C, device=DEV).round()))
     assert torch.isfinite(loss) and torch.isfinite(eng.E[1:99]).all() and torch.isfinite(eng.R).all()
+
+
+@pytest.mark.parametrize("engine", ["1vsSample", "NegSample", "one rank"])
+def test_further_columns_of_a_batch_are_not_looked_at(engine):
+    """Index rows with more columns than the step needs: the same step as on the columns it needs."""
+    import torch.distributed as dist
+    st = "NegSample" if engine == "NegSample" else "1vsSample"
+    pair = _pair("ComplEx", 64, scoring=st)
+    gen = torch.Generator(device=DEV).manual_seed(0)
+    x = torch.randint(0, 12, (30, 5), device=DEV, generator=gen)
+    y = torch.rand(30, 1 if st == "NegSample" else 7, device=DEV, generator=gen).round()
+    rest = (y[:, 0],) if st == "NegSample" else (torch.randint(0, 600, (30, 7), device=DEV, generator=gen), y)
+    out = []
+    try:
+        if engine == "one rank":
+            from dice_embeddings_b200.parallel.sharded_sampled import ShardedSampledEngine
+            dist.init_process_group("nccl", store=dist.HashStore(), rank=0, world_size=1, device_id=DEV)
+        for m, cols in zip(pair, (5, 3 if st == "NegSample" else 2)):
+            if engine == "one rank":
+                eng = ShardedSampledEngine(m, st, batch_size=30, lr=5.0, device=DEV, use_graph=False)
+            else:
+                eng = FusedSampledEngine(m, st, lr=5.0, device=DEV, use_graph=False)
+            out.append((float(eng.step((x[:, :cols].contiguous(), *rest))), eng.E.clone()))
+        assert abs(out[0][0] - out[1][0]) < 1e-6 and torch.allclose(out[0][1], out[1][1], atol=1e-5)
+    finally:
+        if dist.is_initialized():
+            dist.destroy_process_group()
