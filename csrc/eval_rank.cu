@@ -332,7 +332,8 @@ __global__ void eval_sparse_kernel(const T* __restrict__ q, const T* __restrict_
                                    int D, int y_rows, int y_offset, int y_stride, const int* __restrict__ target,
                                    const float* __restrict__ col_bias, const float* __restrict__ target_in,
                                    const long long* __restrict__ filt_ptr, const int* __restrict__ filt_cols,
-                                   float* __restrict__ target_score, int* __restrict__ filtered_greater) {
+                                   const int* __restrict__ repeated, float* __restrict__ target_score,
+                                   int* __restrict__ filtered_greater) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= n) return;
@@ -368,14 +369,21 @@ __global__ void eval_sparse_kernel(const T* __restrict__ q, const T* __restrict_
     if (lane == 0 && target_score != nullptr) target_score[warp] = ts;
   }
   if (filt_ptr == nullptr || filtered_greater == nullptr) return;
+  if (repeated != nullptr && repeated[warp] == 0) return;
   int cnt = 0;
-  for (long long e = filt_ptr[warp]; e < filt_ptr[warp + 1]; ++e) {
+  const long long beg = filt_ptr[warp], end = filt_ptr[warp + 1];
+  for (long long e = beg; e < end; ++e) {
     const int j = filt_cols[e];
     const int jl = local_row(j);
     if (j == tg || jl < 0) continue;
+    if (repeated != nullptr) {   // the first mention is in the mask: count the further ones
+      bool seen = false;
+      for (long long f = beg + lane; f < e; f += 32) seen |= filt_cols[f] == j;
+      if (!__any_sync(0xffffffffu, seen)) continue;
+    }
     cnt += dot(jl) > ts ? 1 : 0;
   }
-  if (lane == 0) filtered_greater[warp] = cnt;
+  if (lane == 0) filtered_greater[warp] = repeated != nullptr ? -cnt : cnt;
 }
 
 // Exact second pass of the band mode: one warp per undecided (query, entity) pair, fp32 operands; the pair counts
@@ -510,9 +518,12 @@ extern "C" int dice_eval_rank_cand_cap(int x_rows, int y_rows, int D, int k, int
   return worst * 2 * k;
 }
 
+// Target scores, and per query the number of listed entities that beat the target, as often as they are listed.  With
+// repeated [n] (see dice_filter_mask) only second and further mentions in the flagged lists count, and
+// filtered_greater[i] is set to minus their number (left alone where the flag is zero).
 extern "C" int dice_eval_sparse(const void* q, const void* y, int n, int D, int y_rows, int y_offset, int y_stride,
                                 const int* target, const float* col_bias, const float* target_in,
-                                const long long* filt_ptr, const int* filt_cols, float* target_score,
+                                const long long* filt_ptr, const int* filt_cols, const int* repeated, float* target_score,
                                 int* filtered_greater, int fp32_operands, void* stream) {
   using namespace dice::evalk;
   if (n <= 0) return 0;
@@ -522,11 +533,13 @@ extern "C" int dice_eval_sparse(const void* q, const void* y, int n, int D, int 
   if (fp32_operands)
     eval_sparse_kernel<float><<<blocks, threads, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const float*>(q), static_cast<const float*>(y), n, D, y_rows, y_offset,
-        y_stride > 0 ? y_stride : 1, target, col_bias, target_in, filt_ptr, filt_cols, target_score, filtered_greater);
+        y_stride > 0 ? y_stride : 1, target, col_bias, target_in, filt_ptr, filt_cols, repeated,
+        target_score, filtered_greater);
   else
     eval_sparse_kernel<__nv_bfloat16><<<blocks, threads, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(y), n, D, y_rows, y_offset,
-        y_stride > 0 ? y_stride : 1, target, col_bias, target_in, filt_ptr, filt_cols, target_score, filtered_greater);
+        y_stride > 0 ? y_stride : 1, target, col_bias, target_in, filt_ptr, filt_cols, repeated,
+        target_score, filtered_greater);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 

@@ -519,6 +519,7 @@ struct MaskParams {
   uint32_t* mask;
   long long stride;
   int y_rows;
+  int* repeated;               // [n] set where a list names an answer more than once; may be null
 };
 
 __global__ void __launch_bounds__(256) filter_mask_kernel(const MaskParams p) {
@@ -557,7 +558,10 @@ __global__ void __launch_bounds__(256) filter_mask_kernel(const MaskParams p) {
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-      if (c[j] >= 0 && c[j] < p.y_rows) atomicOr(row + (c[j] >> 5), 1u << (c[j] & 31));
+      if (c[j] >= 0 && c[j] < p.y_rows) {
+        const uint32_t bit = 1u << (c[j] & 31), before = atomicOr(row + (c[j] >> 5), bit);
+        if (p.repeated != nullptr && (before & bit)) p.repeated[i] = 1;
+      }
   }
 }
 
@@ -667,16 +671,17 @@ extern "C" int dice_rank_collect(const void* x, int x_rows, const void* y, int y
 }
 
 // Sets the mask bits of the known answers of n queries: of (ptr [n + 1], cols), or with ptr == null of the pairs ab (two
-// leading columns, row stride ab_stride) found in keys / offsets / values.  The mask is cleared by the caller.
+// leading columns, row stride ab_stride) found in keys / offsets / values.  With repeated [n], entries of lists that name an
+// answer more than once are set to one.  Mask and flags are cleared by the caller.
 extern "C" int dice_filter_mask(int n, const long long* ptr, const int* cols, const long long* ab, long long ab_stride,
                                 long long num_b, const long long* keys, long long num_keys, const long long* offsets,
-                                const long long* values, unsigned int* mask, long long mask_stride, int y_rows, void* stream) {
+                                const long long* values, unsigned int* mask, long long mask_stride, int y_rows, int* repeated, void* stream) {
   using namespace dice::rankk;
   if (n <= 0) return 0;
   if (mask == nullptr || mask_stride * 32 < y_rows) return -7;
   if (ptr == nullptr ? (ab == nullptr || (num_keys > 0 && (keys == nullptr || offsets == nullptr || values == nullptr))) : cols == nullptr)
     return -7;
-  const MaskParams p{n, ptr, cols, ab, ab_stride, num_b, keys, num_keys, offsets, values, mask, mask_stride, y_rows};
+  const MaskParams p{n, ptr, cols, ab, ab_stride, num_b, keys, num_keys, offsets, values, mask, mask_stride, y_rows, repeated};
   filter_mask_kernel<<<(n + 7) / 8, 256, 0, static_cast<cudaStream_t>(stream)>>>(p);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }

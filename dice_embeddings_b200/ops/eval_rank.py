@@ -149,24 +149,27 @@ class FusedRanker:
     def ranks(self, q: torch.Tensor, target: torch.Tensor, filt_ptr: Optional[torch.Tensor] = None,
               filt_cols: Optional[torch.Tensor] = None) -> torch.Tensor:
         """Filtered ranks ``[B]`` (int64) of entity ``target[i]`` for query vector ``q[i]``.  The filter of query
-        ``i`` is ``filt_cols[filt_ptr[i]:filt_ptr[i+1]]`` (global entity ids; the target itself is ignored)."""
+        ``i`` is ``filt_cols[filt_ptr[i]:filt_ptr[i+1]]`` (global entity ids; the target itself is ignored).  An answer that
+        beats the target is subtracted as often as its list names it (see ``filtered_rank_from_scores``); the lists of a
+        :class:`PairCSR` name every answer once."""
         B = q.shape[0]
-        mask = None
         if filt_ptr is not None:
             filt_ptr = filt_ptr.to(torch.int64).contiguous()
             filt_cols = filt_cols.to(torch.int32).contiguous()
             if self.y_offset == 0 and self.y_stride == 1 and self._mask_pays(B, filt_cols.numel()):
-                cleared, mask = self._cleared(B, self._mask_words())
-                kernels.filter_mask(mask, self.table.shape[0], ptr=filt_ptr, cols=filt_cols)
-                return self._ranks(q, target, None, None, mask, cleared)
-        return self._ranks(q, target, filt_ptr, filt_cols, mask)
+                cleared, mask, repeated = self._cleared(B, self._mask_words())
+                kernels.filter_mask(mask, self.table.shape[0], ptr=filt_ptr, cols=filt_cols, repeated=repeated)
+                return self._ranks(q, target, filt_ptr, filt_cols, mask, cleared, repeated=repeated)
+        return self._ranks(q, target, filt_ptr, filt_cols, None)
 
     def _cleared(self, B: int, words: int):
-        """Zeros for one batch in one fill: target scores and counts (and the band's counter) and the mask ``[B, words]``."""
+        """Zeros for one batch in one fill: target scores and counts (and the band's counter), the mask ``[B, words]`` and the
+        flags of lists that repeat an answer."""
         rows = (B + 3) // 4 * 4
-        buf = torch.zeros(2 * rows + 4 + B * words, dtype=torch.int32, device=self.device)
-        small, mask = buf[:2 * rows + 4], buf[2 * rows + 4:].view(B, words)
-        return (small[:B].view(torch.float32), small[rows:rows + B], small[2 * rows:2 * rows + 2].view(torch.int64)), mask
+        buf = torch.zeros(3 * rows + 4 + B * words, dtype=torch.int32, device=self.device)
+        small, mask = buf[:3 * rows + 4], buf[3 * rows + 4:].view(B, words)
+        return (small[:B].view(torch.float32), small[rows:rows + B], small[2 * rows:2 * rows + 2].view(torch.int64)), mask, \
+            small[2 * rows + 4:2 * rows + 4 + B]
 
     @torch.no_grad()
     def ranks_of_pairs(self, q: torch.Tensor, target: torch.Tensor, ab: torch.Tensor, num_b: int, keys: torch.Tensor,
@@ -174,11 +177,11 @@ class FusedRanker:
         """:meth:`ranks` with the filter of query ``i`` given as the pair in the first two columns of ``ab[i]``, looked up on
         the device in a CSR over sorted keys ``a * num_b + b`` (whole table on this device)."""
         assert self.group is None and self.y_offset == 0 and self.y_stride == 1
-        cleared, mask = self._cleared(q.shape[0], self._mask_words())
+        cleared, mask, _ = self._cleared(q.shape[0], self._mask_words())
         kernels.filter_mask(mask, self.table.shape[0], ab=ab, num_b=num_b, keys=keys, offsets=offsets, values=values)
         return self._ranks(q, target, None, None, mask, cleared, out)
 
-    def _ranks(self, q, target, filt_ptr, filt_cols, mask, cleared=None, out=None) -> torch.Tensor:
+    def _ranks(self, q, target, filt_ptr, filt_cols, mask, cleared=None, out=None, repeated=None) -> torch.Tensor:
         B = q.shape[0]
         tgt_idx = target.to(torch.int32).contiguous()
         sharded = self.group is not None
@@ -190,7 +193,8 @@ class FusedRanker:
         else:
             tgt_score, greater, band_count = cleared if cleared is not None else self._cleared(B, 0)[0]
             tgt_part = tgt_score
-            filtered = torch.zeros(B, dtype=torch.int32, device=self.device) if filt_ptr is not None else None
+            # with a mask the lists are only looked at for repeated answers, whose further mentions come off the counts directly
+            filtered = torch.zeros(B, dtype=torch.int32, device=self.device) if filt_ptr is not None and mask is None else None
         kw = dict(col_bias=self.col_bias, y_offset=self.y_offset, y_stride=self.y_stride)
         band = {}
         if self.exact:
@@ -215,7 +219,8 @@ class FusedRanker:
             if filt_ptr is not None:
                 kernels.eval_sparse(qs, table, tgt_idx, None, filtered, filt_ptr, filt_cols, target_in=tgt_score, **kw)
         else:
-            kernels.eval_sparse(qs, table, tgt_idx, tgt_score, filtered, filt_ptr, filt_cols, **kw)
+            kernels.eval_sparse(qs, table, tgt_idx, tgt_score, filtered if mask is None else greater, filt_ptr, filt_cols,
+                                repeated=repeated, **kw)
         kernels.rank_count(qk, self.table, tgt_score, tgt_idx, greater, self.status, mask=mask, **band, **kw)
         if self.exact:
             kernels.eval_band_exact(qs, table, self.band_rows, self.band_cols, band_count, tgt_score, greater, **kw)

@@ -609,10 +609,12 @@ def rank_count(x: torch.Tensor, y: torch.Tensor, target: torch.Tensor, target_id
 
 def filter_mask(mask: torch.Tensor, y_rows: int, ptr: Optional[torch.Tensor] = None, cols: Optional[torch.Tensor] = None,
                 ab: Optional[torch.Tensor] = None, num_b: int = 0, keys: Optional[torch.Tensor] = None,
-                offsets: Optional[torch.Tensor] = None, values: Optional[torch.Tensor] = None) -> None:
+                offsets: Optional[torch.Tensor] = None, values: Optional[torch.Tensor] = None,
+                repeated: Optional[torch.Tensor] = None) -> None:
     """Set the bits of the known answers of every query in ``mask`` (cleared by the caller): of the CSR ``ptr`` / ``cols``
     over the batch, or of the pairs in the first two columns of ``ab`` looked up in ``keys`` / ``offsets`` / ``values``
-    (``key = a * num_b + b``, ascending)."""
+    (``key = a * num_b + b``, ascending).  ``repeated`` (int32 per query, zeros before) is set to one where a list names an
+    answer more than once."""
     _req(mask, torch.int32, "mask")
     if ptr is not None:
         _req(ptr, torch.int64, "ptr")
@@ -626,9 +628,12 @@ def filter_mask(mask: torch.Tensor, y_rows: int, ptr: Optional[torch.Tensor] = N
             _req(t, torch.int64, name)
         n = ab.shape[0]
     assert mask.shape[0] >= n
+    if repeated is not None:
+        _req(repeated, torch.int32, "repeated")
+        assert repeated.numel() >= n
     _call("dice_filter_mask", mask, n, _ptr(ptr), _ptr(cols), _ptr(ab), 0 if ab is None else ab.stride(0), int(num_b),
           _ptr(keys), 0 if keys is None else keys.numel(), _ptr(offsets), _ptr(values), _ptr(mask), mask.shape[1], int(y_rows),
-          others=(ptr, cols, ab, keys, offsets, values))
+          _ptr(repeated), others=(ptr, cols, ab, keys, offsets, values, repeated))
 
 
 def split_rows(src: torch.Tensor, d_pad: int, want_copy: bool = False, margin_factor: Optional[float] = None):
@@ -738,9 +743,11 @@ def eval_rank_cand_cap(x_rows: int, y_rows: int, D: int, k: int, num_ctas: int =
 def eval_sparse(q: torch.Tensor, y: torch.Tensor, target_idx: torch.Tensor, target_score: Optional[torch.Tensor],
                 filtered_greater: Optional[torch.Tensor], filt_ptr: Optional[torch.Tensor] = None,
                 filt_cols: Optional[torch.Tensor] = None, col_bias: Optional[torch.Tensor] = None,
-                target_in: Optional[torch.Tensor] = None, y_offset: int = 0, y_stride: int = 1) -> None:
+                target_in: Optional[torch.Tensor] = None, y_offset: int = 0, y_stride: int = 1,
+                repeated: Optional[torch.Tensor] = None) -> None:
     """Gather-dots of the ranking protocol: the target score of each query and the number of filtered entities (CSR
-    ``filt_ptr`` int64 / ``filt_cols`` int32) that beat it."""
+    ``filt_ptr`` int64 / ``filt_cols`` int32) that beat it.  With the ``repeated`` flags of :func:`filter_mask` only second
+    and further mentions in the flagged lists count, and ``filtered_greater`` (zeros before) receives minus their number."""
     fp32 = q.dtype == torch.float32
     _req(q, torch.float32 if fp32 else torch.bfloat16, "q")
     _req(y, q.dtype, "y")
@@ -748,10 +755,13 @@ def eval_sparse(q: torch.Tensor, y: torch.Tensor, target_idx: torch.Tensor, targ
     if filt_ptr is not None:
         _req(filt_ptr, torch.int64, "filt_ptr")
         _req(filt_cols, torch.int32, "filt_cols")
+    if repeated is not None:
+        _req(repeated, torch.int32, "repeated")
+        assert repeated.numel() >= q.shape[0]
     _call("dice_eval_sparse", q, _ptr(q), _ptr(y), q.shape[0], q.shape[1], y.shape[0], int(y_offset), int(y_stride),
-          _ptr(target_idx), _ptr(col_bias), _ptr(target_in), _ptr(filt_ptr), _ptr(filt_cols), _ptr(target_score),
-          _ptr(filtered_greater), int(fp32),
-          others=(y, target_idx, col_bias, target_in, filt_ptr, filt_cols, target_score, filtered_greater))
+          _ptr(target_idx), _ptr(col_bias), _ptr(target_in), _ptr(filt_ptr), _ptr(filt_cols), _ptr(repeated),
+          _ptr(target_score), _ptr(filtered_greater), int(fp32),
+          others=(y, target_idx, col_bias, target_in, filt_ptr, filt_cols, repeated, target_score, filtered_greater))
 
 
 def peer_sum_f32(table: torch.Tensor, W: int, out: torch.Tensor, n: int, status: Optional[torch.Tensor] = None) -> None:

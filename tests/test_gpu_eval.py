@@ -316,3 +316,25 @@ def test_full_band_list_has_no_gaps(split, cap):
     r, c = rows.long(), cols.long()
     assert ((r >= 0) & (r < nx) & (c >= 0) & (c < ny)).all() and (c != tgt.long()[r.clamp_min(0)]).all()
     assert torch.unique(r * ny + c).numel() == cap
+
+
+@pytest.mark.parametrize("exact", [False, True])
+@pytest.mark.parametrize("masked", [False, True])
+def test_repeated_answers_in_a_filter(exact, masked):
+    """An answer that a list names several times is subtracted as often as it is named, whether the answers are masked or
+    scored one by one; lists without repeats, with the target, and empty ones.  Integer operands: exact scores."""
+    from dice_embeddings_b200.evaluation.ranking import filtered_rank_from_scores
+    torch.manual_seed(5)
+    nx, ny, D = 60, 400, 64
+    x, y = torch.randint(-3, 4, (nx, D), device=DEV).float(), torch.randint(-3, 4, (ny, D), device=DEV).float()
+    tgt = torch.randint(0, ny, (nx,), device=DEV)
+    lists = [torch.randint(0, 25, (90,)) if i % 3 == 0 else torch.randperm(ny)[:40] if i % 3 == 1 else torch.zeros(0).long() for i in range(nx)]
+    lists[0][7:9] = int(tgt[0])
+    ptr = torch.zeros(nx + 1, dtype=torch.int64)
+    ptr[1:] = torch.tensor([len(a) for a in lists]).cumsum(0)
+    rows, cols = torch.repeat_interleave(torch.arange(nx), ptr[1:] - ptr[:-1]).to(DEV), torch.cat(lists).to(DEV)
+    r = FusedRanker(y, exact=exact)
+    r._mask_pays = lambda *a: masked
+    got = r.ranks(x, tgt, ptr.to(DEV), cols.to(torch.int32))
+    r.check()
+    assert torch.equal(got, filtered_rank_from_scores(x @ y.t(), tgt, rows, cols))
