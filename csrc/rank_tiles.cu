@@ -82,7 +82,7 @@ struct Cfg {
   static_assert(SMEM_BYTES <= 227 * 1024 && NBUF >= 2, "layout");
 };
 
-// bit i set where r[i] > t (false for NaN): the sign of t - r[i], shifted in from the top column down
+// bit i set where r[i] > t (false for NaN; t must not be -0): the sign of t - r[i], shifted in from the top column down
 __device__ __forceinline__ uint32_t above(const uint32_t (&r)[32], float t) {
   const uint64_t tt = pack2(t, t), minus = pack2(-1.f, -1.f);
   uint32_t hi = 0u, lo = 0u;
@@ -302,11 +302,12 @@ rank_tiles_kernel(const __grid_constant__ CUtensorMap tmap_y, const __grid_const
         tgt_col[u] = -1;
         cnt[u] = 0;
         if (valid[u]) {
-          if constexpr (MODE == COUNT) hi[u] = p.target[x_global[u]];
+          // + 0 turns -0 into +0: the sign of -0 - (+0) would count a score of zero as above
+          if constexpr (MODE == COUNT) hi[u] = p.target[x_global[u]] + 0.f;
           if constexpr (MODE == BAND) {
             const float t = p.target[x_global[u]], mg = p.margin[x_global[u]];
-            hi[u] = t + mg;
-            lo[u] = t - mg;
+            hi[u] = t + mg + 0.f;
+            lo[u] = t - mg + 0.f;
           }
           if constexpr (MODE == COLLECT) {
             hi[u] = p.floor[x_global[u]];

@@ -338,3 +338,20 @@ def test_repeated_answers_in_a_filter(exact, masked):
     got = r.ranks(x, tgt, ptr.to(DEV), cols.to(torch.int32))
     r.check()
     assert torch.equal(got, filtered_rank_from_scores(x @ y.t(), tgt, rows, cols))
+
+
+def test_a_target_of_minus_zero():
+    """-0 is not below +0: scores of zero are not above a target of -0, in the counting and in the band form."""
+    x, y = torch.zeros(5, 64, dtype=torch.bfloat16, device=DEV), _operands(1, 300, 64, 0)[1]
+    bias = torch.zeros(300, device=DEV)
+    bias[7], bias[9] = 1e-38, -0.0
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    for band in (False, True):
+        kw = {}
+        if band:
+            lists = [torch.zeros(2000, dtype=torch.int32, device=DEV) for _ in range(2)]
+            count = torch.zeros(1, dtype=torch.int64, device=DEV)
+            kw = dict(margin=torch.zeros(5, device=DEV), band_rows=lists[0], band_cols=lists[1], band_count=count)
+        greater = torch.zeros(5, dtype=torch.int32, device=DEV)
+        K.rank_count(x, y, torch.full((5,), -0.0, device=DEV), None, greater, status, col_bias=bias, **kw)
+        assert greater.tolist() == [1] * 5 and int(status) == 0 and (not band or int(count) == 0)
