@@ -70,7 +70,7 @@ int dice_filter_mask(int n, const long long* ptr, const int* cols, const long lo
                      const long long* keys, long long num_keys, const long long* offsets, const long long* values,
                      unsigned int* mask, long long mask_stride, int y_rows, int* repeated, void* stream);
 int dice_split_rows(const float* src, long long src_stride, long long n, int d, int d_pad, void* hi, void* lo, float* copy,
-                    float* margin, float factor, void* stream);
+                    float* margin, float factor, float offset, void* stream);
 int dice_topk_floor(const float* gmax, int rows, int groups, int k, float* floor, int* cand_count, void* stream);
 int dice_topk_select(const float* score, const int* idx, const int* count, int rows, int cand_cap, int tie_cap, int k,
                      float* out_s, long long* out_i, float* kth_score, int* overflow, void* stream);

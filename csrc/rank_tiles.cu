@@ -567,10 +567,10 @@ __global__ void __launch_bounds__(256) filter_mask_kernel(const MaskParams p) {
 }
 
 // Rows of fp32 [n, d] as hi + lo in bf16, zero-padded to d_pad columns, an fp32 copy of that width (optional) and
-// margin[row] = |row| * factor + 1e-30 (optional).  One warp per row.
+// margin[row] = |row| * factor + offset (optional).  One warp per row.
 __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ src, long long src_stride, long long n, int d,
                                                          int d_pad, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo,
-                                                         float* __restrict__ copy, float* __restrict__ margin, float factor) {
+                                                         float* __restrict__ copy, float* __restrict__ margin, float factor, float offset) {
   const int lane = threadIdx.x & 31;
   const long long warps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
   for (long long i = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
@@ -586,7 +586,7 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-    if (lane == 0 && margin != nullptr) margin[i] = sqrtf(sq) * factor + 1e-30f;
+    if (lane == 0 && margin != nullptr) margin[i] = sqrtf(sq) * factor + offset;
   }
 }
 
@@ -688,13 +688,13 @@ extern "C" int dice_filter_mask(int n, const long long* ptr, const int* cols, co
 }
 
 extern "C" int dice_split_rows(const float* src, long long src_stride, long long n, int d, int d_pad, void* hi, void* lo,
-                               float* copy, float* margin, float factor, void* stream) {
+                               float* copy, float* margin, float factor, float offset, void* stream) {
   using namespace dice::rankk;
   if (n <= 0) return 0;
   if (d <= 0 || d > d_pad || src == nullptr || hi == nullptr || lo == nullptr) return -6;
   long long blocks = (n + 7) / 8;
   if (blocks > 148 * 16) blocks = 148 * 16;
   split_rows_kernel<<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      src, src_stride, n, d, d_pad, static_cast<__nv_bfloat16*>(hi), static_cast<__nv_bfloat16*>(lo), copy, margin, factor);
+      src, src_stride, n, d, d_pad, static_cast<__nv_bfloat16*>(hi), static_cast<__nv_bfloat16*>(lo), copy, margin, factor, offset);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }

@@ -135,7 +135,7 @@ class _Sigs:
     dice_rank_group_max = [_p, _i, _p, _i, _i, _p, _p, _i, _p, _i, _p]
     dice_rank_collect = [_p, _i, _p, _i, _i, _p, _i, _i, _p, _i, _i, _p, _p, _p, _p, _i, _p]
     dice_filter_mask = [_i, _p, _p, _p, _l, _l, _p, _l, _p, _p, _p, _l, _i, _p, _p]
-    dice_split_rows = [_p, _l, _l, _i, _i, _p, _p, _p, _p, _f, _p]
+    dice_split_rows = [_p, _l, _l, _i, _i, _p, _p, _p, _p, _f, _f, _p]
     dice_topk_floor = [_p, _i, _i, _i, _p, _p, _p]
     dice_topk_select = [_p, _p, _p, _i, _i, _i, _i, _p, _p, _p, _p, _p]
     dice_topk_scan_blocks = [_i, _i]

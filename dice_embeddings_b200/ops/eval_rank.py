@@ -50,7 +50,7 @@ class FusedRanker:
                  y_stride: int = 1, group=None, exact: bool = False, band_capacity: int = 1 << 24):
         """``exact``: ranks equal those of an fp32 scoring of the same operands.  The tensor cores still do the bulk of the
         work, on operands split into two bf16 terms each; such a score differs from its fp32 value by at most
-        ``MARGIN[d] · ‖q‖ · ‖e‖``, so only entities within that margin of the target are undecided, and exactly those
+        ``MARGIN[d] · ‖q‖ · ‖e‖`` (plus the rounding of the bias), so only entities within that margin of the target are undecided, and exactly those
         (well below a tenth of a percent) are re-scored in fp32 by a second, sparse pass."""
         assert table.is_cuda, "the fused ranker runs on a CUDA device"
         self.d = table.shape[1]
@@ -68,6 +68,9 @@ class FusedRanker:
         else:
             self.table = to_kernel_operand(table, self.d_pad)
         self.col_bias = None if col_bias is None else col_bias.detach().float().contiguous()
+        self.bias_max = 0.0
+        if self.exact and self.col_bias is not None and table.shape[0]:
+            self.bias_max = float(self.col_bias.abs().nan_to_num(0.0, 0.0).max())   # a column at -inf is undecided for no one
         self.y_offset, self.y_stride, self.group = int(y_offset), int(y_stride), group
         self.device = table.device
         self._flags = torch.zeros(2, dtype=torch.int32, device=self.device)
@@ -81,10 +84,10 @@ class FusedRanker:
             self.W, self.rank = dist.get_world_size(group), dist.get_rank(group)
             if self.W == 1:
                 self.group = None
-            elif self.exact:   # the margin of the band mode needs the largest row norm over all shards: once, here
-                emax = torch.tensor([self.row_norm_max], device=self.device)
+            elif self.exact:   # the margin of the band mode needs the largest row norm and bias over all shards: once, here
+                emax = torch.tensor([self.row_norm_max, self.bias_max], device=self.device)
                 dist.all_reduce(emax, op=dist.ReduceOp.MAX, group=group)
-                self.row_norm_max = float(emax.item())
+                self.row_norm_max, self.bias_max = emax.tolist()
 
     # ------------------------------------------------------------------ cross-rank merge (symmetric heap + barrier)
     K_CAP = 32
@@ -130,6 +133,9 @@ class FusedRanker:
     #: relative error of a split score for each padded width: the terms left out of (hi + lo)(hi + lo) are at most
     #: 3 · 2^-16, the accumulation of 3 d products and of the fp32 reference at most 4 d · 2^-23
     MARGIN = {d: 3 * 2.0 ** -16 + 4 * d * 2.0 ** -23 for d in SUPPORTED_D}
+    #: error relative to the largest column bias: the sum with it is rounded once for either score and once for the bounds of
+    #: the band, by 2^-24 of it each (the score's share of those sums is far inside MARGIN)
+    BIAS_MARGIN = 2.0 ** -22
     #: largest bit mask of known answers (bytes); beyond it the known answers are scored one by one
     MASK_LIMIT = 512 << 20
 
@@ -201,7 +207,8 @@ class FusedRanker:
             # target scores and filtered counts from the fp32 operands, dense counts from the split ones
             q32 = q.detach().float()
             qk, q_lo, copy, margin = kernels.split_rows(q32, self.d_pad, want_copy=self.d != self.d_pad,
-                                                        margin_factor=self.row_norm_max * self.MARGIN[self.d_pad])
+                                                        margin_factor=self.row_norm_max * self.MARGIN[self.d_pad],
+                                                        margin_offset=self.bias_max * self.BIAS_MARGIN)
             qs, table = copy if copy is not None else q32.contiguous(), self.table_f32
             if sharded:
                 band_count = torch.zeros(1, dtype=torch.int64, device=self.device)

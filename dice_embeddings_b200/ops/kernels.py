@@ -636,9 +636,10 @@ def filter_mask(mask: torch.Tensor, y_rows: int, ptr: Optional[torch.Tensor] = N
           _ptr(repeated), others=(ptr, cols, ab, keys, offsets, values, repeated))
 
 
-def split_rows(src: torch.Tensor, d_pad: int, want_copy: bool = False, margin_factor: Optional[float] = None):
+def split_rows(src: torch.Tensor, d_pad: int, want_copy: bool = False, margin_factor: Optional[float] = None,
+               margin_offset: float = 0.0):
     """``(hi, lo, copy, margin)`` of fp32 rows: two bf16 terms and (optionally) the fp32 rows, zero-padded to ``d_pad``
-    columns, and ``margin = |row| * margin_factor``."""
+    columns, and ``margin = |row| * margin_factor + max(margin_offset, 1e-30)``."""
     assert src.is_cuda and src.dtype == torch.float32 and src.dim() == 2
     if src.stride(1) != 1:
         src = src.contiguous()
@@ -648,7 +649,7 @@ def split_rows(src: torch.Tensor, d_pad: int, want_copy: bool = False, margin_fa
     copy = torch.empty(n, d_pad, dtype=torch.float32, device=src.device) if want_copy else None
     margin = None if margin_factor is None else torch.empty(n, dtype=torch.float32, device=src.device)
     _call("dice_split_rows", src, _ptr(src), src.stride(0), n, d, int(d_pad), _ptr(hi), _ptr(lo), _ptr(copy), _ptr(margin),
-          0.0 if margin_factor is None else float(margin_factor))
+          0.0 if margin_factor is None else float(margin_factor), max(float(margin_offset), 1e-30))
     return hi, lo, copy, margin
 
 

@@ -355,3 +355,23 @@ def test_a_target_of_minus_zero():
         greater = torch.zeros(5, dtype=torch.int32, device=DEV)
         K.rank_count(x, y, torch.full((5,), -0.0, device=DEV), None, greater, status, col_bias=bias, **kw)
         assert greater.tolist() == [1] * 5 and int(status) == 0 and (not band or int(count) == 0)
+
+
+@pytest.mark.parametrize("D", [64, 256])
+@pytest.mark.parametrize("size", [1e-2, 30.0, 1000.0])
+def test_exact_ranks_with_a_bias_far_above_the_scores(D, size):
+    """A bias that rounds most of the score away leaves few different sums; the ranks are still those of the fp32 sums, which
+    the gather-dots give with the same order of additions as the second pass."""
+    torch.manual_seed(0)
+    n, B = 3000, 300
+    x, y = torch.randn(B, D, device=DEV) * 1e-4, torch.randn(n, D, device=DEV)
+    bias = torch.full((n,), size, device=DEV)
+    bias[::7] = float("-inf")
+    tgt = 1 + 7 * torch.randint(0, n // 7, (B,), device=DEV, dtype=torch.int32)
+    r = FusedRanker(y, col_bias=bias, exact=True)
+    got = r.ranks(x, tgt)
+    r.check()
+    ts, above = torch.zeros(B, device=DEV), torch.zeros(B, dtype=torch.int32, device=DEV)
+    K.eval_sparse(x, y, tgt, ts, above, torch.arange(B + 1, device=DEV) * n, torch.arange(n, device=DEV, dtype=torch.int32).repeat(B),
+                  col_bias=bias)
+    assert torch.equal(got, 1 + above.long())
