@@ -77,6 +77,7 @@ class FusedRanker:
         self.status = self._flags[0:1]      # kernel status word
         self.overflow = self._flags[1:2]    # set when a top-k candidate list ran full
         self._scan_done = {}
+        self._whole_table = False           # top-k thresholds from the whole table: set once a list of the two-stage search ran full
         self.W, self.rank = 1, 0
         self._heap = None
         if group is not None:
@@ -127,8 +128,9 @@ class FusedRanker:
             raise kernels.KernelError(f"kernel status {code} ({kernels.STATUS_TEXT.get(code, '?')}) in the fused ranker"
                                       " (band list full: raise band_capacity or use smaller batches)")
         if over != 0:
-            raise kernels.KernelError("a top-k candidate list ran full: the table prefix used for the threshold was "
-                                      "not representative; call topk again with a smaller batch")
+            self._whole_table = True
+            raise kernels.KernelError("a top-k candidate list ran full (the sample of the table gave too low a threshold); call "
+                                      "topk again: this ranker takes its thresholds from the whole table from here on")
 
     #: relative error of a split score for each padded width: the terms left out of (hi + lo)(hi + lo) are at most
     #: 3 · 2^-16, the accumulation of 3 d products and of the fp32 reference at most 4 d · 2^-23
@@ -241,12 +243,29 @@ class FusedRanker:
         kernels.merge_ranks(self._tab["greater"], self._tab["filtered"], self.W, out, B, self.status)
         return out
 
-    #: tables with more rows than this are searched in two stages (threshold from a prefix, then one collecting pass)
+    #: tables with more rows than this are searched in two stages (threshold from a sample, then one collecting pass)
     TWO_STAGE_ROWS = 131072
     SAMPLE_ROWS = 32768
 
-    #: queries per pass: bounds the group maxima (16 KB per query at 131 072 rows)
+    #: queries per pass, and what the group maxima of a pass may take (16 KB per query at 131 072 rows)
     TOPK_QUERIES = 8192
+    GROUP_MAX_BYTES = 1 << 30
+
+    def _sample_rows(self) -> torch.Tensor:
+        """One row out of each of ``SAMPLE_ROWS`` equally long ranges of the table, at a place a hash of the range's number
+        gives: the whole table is covered, and no order of the rows (sorted, periodic) can keep a class of them out."""
+        n, S = self.table.shape[0], self.SAMPLE_ROWS
+        i = torch.arange(S + 1, dtype=torch.int64, device=self.device)
+        edge = i * n // S
+        h = (i[:S] + 1) * 0x9E3779B97F4A7C1            # odd multipliers and shifts: Fibonacci hashing, twice
+        h = (h ^ (h >> 29)) * 0x5851F42D4C957F2D
+        return edge[:S] + ((h >> 33) & 0x7fffffff) % (edge[1:] - edge[:S])
+
+    def _list_capacity(self, kk: int) -> int:
+        """Room for the scores above the ``kk``-th best of the sample.  In units of ``n / S`` their number follows a gamma
+        distribution of order ``kk`` (exponential for 1); it is above ``kk + 6 sqrt(kk) + 24`` of them with probability 6e-13
+        or less for every ``kk`` up to 32, so that a call of 8192 queries meets a full list once in 200 million calls."""
+        return int((kk + 6 * kk ** 0.5 + 24) * (self.table.shape[0] / self.SAMPLE_ROWS)) + 64
 
     def _done(self) -> torch.Tensor:
         """Block counter of the scan: calls on one stream follow one another, so there is one per stream."""
@@ -266,28 +285,28 @@ class FusedRanker:
         # tensor cores, where a tile costs the same for 1 query as for 128.
         if kk and B and q.dtype in (torch.float32, torch.bfloat16) and q.stride(1) == 1 and kernels.topk_scan_blocks(B, n_local):
             return kernels.topk_scan(q, self.table, kk, self._done(), **kw)
-        if B > self.TOPK_QUERIES:
-            parts = [self._topk_local(q[i:i + self.TOPK_QUERIES], kk) for i in range(0, B, self.TOPK_QUERIES)]
-            return torch.cat([p[0] for p in parts]), torch.cat([p[1] for p in parts])
         if kk == 0 or B == 0:
             return (torch.empty(B, kk, dtype=torch.float32, device=self.device),
                     torch.empty(B, kk, dtype=torch.int64, device=self.device))
+        two_stage = n_local > self.TWO_STAGE_ROWS and not self._whole_table
+        most = self.TOPK_QUERIES if two_stage else max(1, min(self.TOPK_QUERIES, self.GROUP_MAX_BYTES // (16 * ((n_local + 127) // 128))))
+        if B > most:
+            parts = [self._topk_local(q[i:i + most], kk) for i in range(0, B, most)]
+            return torch.cat([p[0] for p in parts]), torch.cat([p[1] for p in parts])
         qk = to_kernel_operand(q, self.d_pad)
-        if n_local <= self.TWO_STAGE_ROWS:
+        if not two_stage:
             return kernels.topk_bounded(qk, self.table, kk, self.status, self.overflow, **kw)
-        # stage 1: the k-th best score over a sample of the table is a lower bound of the k-th best overall.  The
-        # sample takes every (n / S)-th row, so it is representative whatever the order of the rows (a prefix of a
-        # table sorted by norm would not be); it is copied once per ranker.
-        S = self.SAMPLE_ROWS
+        # stage 1: the k-th best score over a sample of the table (copied once per ranker) is a lower bound of the k-th best
+        # overall
         if getattr(self, "_sample", None) is None:
-            step = max(n_local // S, 1)
-            self._sample_bias = None if self.col_bias is None else self.col_bias[::step][:S].contiguous()
-            self._sample = self.table[::step][:S].contiguous()
+            rows = self._sample_rows()
+            self._sample_bias = None if self.col_bias is None else self.col_bias[rows]
+            self._sample = self.table[rows]
         floor = kernels.topk_bounded(qk, self._sample, kk, self.status, self.overflow, col_bias=self._sample_bias, kth_only=True)
-        # stage 2: one pass over the whole table that collects what reaches the bound (few per row).  A list that ran full
-        # (sample not representative of the table) is recorded on the device and reported by check()
+        # stage 2: one pass over the whole table that collects what reaches the bound (few per row).  A list that ran full is
+        # recorded on the device and reported by check()
         return kernels.topk_bounded(qk, self.table, kk, self.status, self.overflow, floor=floor,
-                                    cand_cap=int(8 * kk * (n_local / S) + 64), **kw)
+                                    cand_cap=self._list_capacity(kk), **kw)
 
     @torch.no_grad()
     def topk(self, q: torch.Tensor, k: int) -> Tuple[torch.Tensor, torch.Tensor]:
