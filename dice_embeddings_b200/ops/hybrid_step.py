@@ -30,12 +30,19 @@ The reference runs these models as ``conv2d`` / ``Linear`` / four to eight ``tor
 from __future__ import annotations
 
 import os
+import types
 from typing import Optional
 
 import torch
 
 from . import kernels as K
 from .fused_step import SUPPORTED_DIMS, SUPPORTED_SCORING, _EngineOptimizer, fused_model_code
+
+
+#: attribute types of a module that its forward may read and a captured step therefore has fixed (momentum, eps, probabilities,
+#: modes, replaced functions ...)
+_PLAIN = frozenset((bool, int, float, str, tuple, type(None), torch.dtype, types.FunctionType, types.BuiltinFunctionType,
+                    types.MethodType))
 
 
 def hybrid_supported(model) -> bool:
@@ -213,17 +220,23 @@ class ExternalQueryEngine:
         if nn_module._global_forward_hooks or nn_module._global_forward_pre_hooks or nn_module._global_backward_hooks \
                 or nn_module._global_backward_pre_hooks:
             return None
-        mods = []
-        for m in self.model.modules():
+        # one walk over the modules (half the time of modules(), parameters() and buffers() one after the other)
+        kinds, tensors, todo = [], [], [self.model]
+        while todo:
+            m = todo.pop()
+            if m is None:
+                continue
             if m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks:
                 return None
-            mods.append((m.training, getattr(m, "p", None)))
-        params = []
-        for p in self.model.parameters():
-            if p._backward_hooks or p._post_accumulate_grad_hooks:
-                return None
-            params.append((p.data_ptr(), p.requires_grad))
-        params += [t.data_ptr() for t in self.model.buffers()]
+            kinds.append(type(m))
+            kinds += [kv for kv in m.__dict__.items() if type(kv[1]) in _PLAIN]
+            for p in m._parameters.values():
+                if p is not None:
+                    if p._backward_hooks or p._post_accumulate_grad_hooks:
+                        return None
+                    tensors += (p.data_ptr(), p.requires_grad)
+            tensors += [t.data_ptr() for t in m._buffers.values() if t is not None]
+            todo += m._modules.values()
         opt = []
         if self.rest_optimizer is not None:
             o = self.rest_optimizer
@@ -234,9 +247,17 @@ class ExternalQueryEngine:
                 if any(isinstance(v, torch.Tensor) for k, v in g.items() if k != "params"):
                     return None
                 opt += [t.data_ptr() for p in g["params"] for t in o.state.get(p, {}).values() if isinstance(t, torch.Tensor)]
-        flags = (torch.backends.cuda.matmul.allow_tf32, torch.backends.cudnn.allow_tf32, torch.backends.cudnn.deterministic,
-                 torch.are_deterministic_algorithms_enabled())
-        return (x.shape[0], self.lr, self.weight_decay, tuple(mods), tuple(params), tuple(opt), flags)
+        mm, cudnn = torch.backends.cuda.matmul, torch.backends.cudnn
+        flags = (mm.allow_tf32, mm.allow_fp16_reduced_precision_reduction, mm.allow_bf16_reduced_precision_reduction, cudnn.enabled,
+                 cudnn.benchmark, cudnn.allow_tf32, cudnn.deterministic, torch.are_deterministic_algorithms_enabled(),
+                 torch.get_default_dtype())
+        mine = (self.lr, self.weight_decay, self.betas, self.eps, self.opt_kind, self.margin, self.pos_weight, self.base)
+        key = (x.shape[0], mine, tuple(kinds), tuple(tensors), tuple(opt), flags)
+        try:
+            hash(key)
+        except TypeError:       # a tuple of lists or the like: nothing to recognise a step by
+            return None
+        return key
 
     def _capture(self, n: int, key):
         b = self._buffers(n)

@@ -268,3 +268,41 @@ def test_external_query_step_with_hooks_runs_as_plain_launches():
     with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(1) or t, lambda t: t):
         eng.step(ds.make_batch(idx)[:1] + (idx,))
     assert len(calls) == 1 and packed
+
+
+@pytest.mark.parametrize("what", ["momentum", "eps", "dropout", "margin", "function", "betas"])
+def test_host_values_changed_after_a_capture_take_effect(what):
+    """Replay fixes what a step reads on the host: a change of such a value gives the same state as plain launches do (atomics in
+    another order: 1e-3), here far from the state without the change."""
+    out = []
+    for use_graph, change in ((True, True), (False, True), (False, False)):
+        torch.manual_seed(0)
+        name = "TransE" if what == "margin" else "ConEx"
+        ds = KvsAll(zipf_kg(300, 9, 3000, seed=1), 300, 9, label_smoothing_rate=0.1).to(DEV)
+        model, _ = initialize_model(dict(model=name, embedding_dim=64, num_entities=300, num_relations=9, optim="SGD",
+                                         learning_rate=0.01, scoring_technique="KvsAll", num_of_output_channels=4, kernel_size=3))
+        model = model.to(DEV).train()
+        eng = ExternalQueryEngine(model, ds, batch_size=128, lr=0.05, device=DEV, use_graph=use_graph)
+        idx = torch.arange(128, device=DEV)
+        batch = (ds.make_batch(idx)[0], idx)
+        for _ in range(3):
+            eng.step(batch)
+        if change:
+            if what == "momentum":
+                model.bn_conv2d.momentum = 0.9
+            elif what == "eps":
+                model.bn_conv2d.eps = 0.5
+            elif what == "dropout":
+                model.input_dp_ent_real.p = 1.0
+            elif what == "margin":
+                eng.margin += 2.0
+            elif what == "function":
+                model.fc1.forward = lambda x, fc=model.fc1: torch.nn.functional.linear(x, fc.weight, fc.bias) + 1.0
+            else:
+                eng.weight_decay, eng.betas = 0.3, (0.5, 0.9)
+        for _ in range(3):
+            loss = eng.step(batch)
+        out.append(torch.cat([loss.reshape(1), eng.E.flatten()] + [b.float().flatten() for b in model.buffers()]))
+        assert len(eng._graphs) == ((2 if change else 1) if use_graph else 0)
+    size = (out[1] - out[2]).norm()
+    assert (out[0] - out[1]).norm() < 1e-3 * out[1].norm() and (out[0] - out[1]).norm() < 0.1 * size, (what, size)
