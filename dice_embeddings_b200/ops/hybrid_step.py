@@ -29,8 +29,10 @@ The reference runs these models as ``conv2d`` / ``Linear`` / four to eight ``tor
 """
 from __future__ import annotations
 
+import logging
 import os
 import types
+from collections import OrderedDict
 from typing import Optional
 
 import torch
@@ -107,8 +109,12 @@ class FusedScoring(torch.autograd.Function):
 
 
 class ExternalQueryEngine:
-    #: captured steps kept (one per batch size as a rule); a program that needs more runs the further ones as plain launches
+    #: captured steps kept (one per batch size as a rule); the least recently used one makes room for another
     MAX_GRAPHS = 4
+    #: plain steps of a kind before it takes the place of another: a capture takes 2 to 13 ms, a replay saves 0.35 to 1.2 ms
+    STEPS_BEFORE_REPLACING = 16
+    #: kinds of steps whose number is remembered
+    MAX_KINDS = 64
 
     def __init__(self, model, dataset, batch_size: int, lr: float, weight_decay: float = 0.0, device=None,
                  use_graph: bool = True):
@@ -145,8 +151,8 @@ class ExternalQueryEngine:
                 g["capturable"], g["fused"], g["foreach"] = True, True, False
         elif self.rest_optimizer is not None and type(self.rest_optimizer) is not torch.optim.SGD:
             self.use_graph = False
-        self._graphs = {}
-        self._seen = set()
+        self._graphs = OrderedDict()
+        self._seen = OrderedDict()      # kind of step: plain launches so far
         self.dataset = dataset
         dataset.sparse_labels = True
         if hasattr(dataset, "offsets"):
@@ -191,14 +197,14 @@ class ExternalQueryEngine:
             return self._step(x, dp)
         entry = self._graphs.get(key)
         if entry is None:
-            if key not in self._seen or len(self._graphs) >= self.MAX_GRAPHS:
+            if self._seen.get(key, 0) < (1 if len(self._graphs) < self.MAX_GRAPHS else self.STEPS_BEFORE_REPLACING):
                 loss = self._step(x, dp)   # the first step of a kind sets up libraries and the optimiser's state
-                if len(self._seen) < 64:
-                    self._seen.add(self._graph_key(x))
+                self._count(self._graph_key(x))
                 return loss
             entry = self._capture(x.shape[0], key)
             if entry is None:
                 return self._step(x, dp)
+        self._graphs.move_to_end(key)
         graph, loss, grads = entry
         b = self._buffers(x.shape[0])
         K.stage((b.x_in, x[:, :2]), (b.dp, dp))
@@ -206,6 +212,11 @@ class ExternalQueryEngine:
         for p, g in grads:
             p.grad = g
         return loss.clone()
+
+    def _count(self, key) -> None:
+        self._seen[key] = self._seen.pop(key, 0) + 1
+        if len(self._seen) > self.MAX_KINDS:
+            self._seen.popitem(last=False)
 
     def _graph_key(self, x):
         """Everything a captured step has fixed, or ``None`` where the step has to run as plain launches: hooks, autocast,
@@ -261,13 +272,19 @@ class ExternalQueryEngine:
 
     def _capture(self, n: int, key):
         b = self._buffers(n)
+        if len(self._graphs) >= self.MAX_GRAPHS:
+            torch.cuda.synchronize(self.device)      # no replay is under way when its memory is given back
+            self._graphs.popitem(last=False)
         graph = torch.cuda.CUDAGraph()
         try:
             with torch.cuda.graph(graph, capture_error_mode="thread_local"):
                 loss = self._step(b.x_in, b.dp)
-        except RuntimeError:
-            # something in the model cannot be captured (nothing has run): plain launches from here on
+        except RuntimeError as err:
+            # the step cannot be captured, or there is no memory for a graph's own pool (nothing has run): plain launches from
+            # here on, which raise what is wrong with the step itself
+            logging.getLogger(__name__).warning("training step runs as plain launches, its capture failed: %s", err)
             self.use_graph = False
+            self._graphs.clear()
             return None
         grads = [(p, p.grad) for p in self.model.parameters() if p.grad is not None]
         self._graphs[key] = (graph, loss, grads)

@@ -306,3 +306,56 @@ def test_host_values_changed_after_a_capture_take_effect(what):
         assert len(eng._graphs) == ((2 if change else 1) if use_graph else 0)
     size = (out[1] - out[2]).norm()
     assert (out[0] - out[1]).norm() < 1e-3 * out[1].norm() and (out[0] - out[1]).norm() < 0.1 * size, (what, size)
+
+
+def _small_engine(**kw):
+    ds = KvsAll(zipf_kg(300, 9, 3000, seed=1), 300, 9, label_smoothing_rate=0.1).to(DEV)
+    model, _ = initialize_model(dict(model="ConEx", embedding_dim=64, num_entities=300, num_relations=9, optim="Adam",
+                                     learning_rate=0.01, scoring_technique="KvsAll", num_of_output_channels=4, kernel_size=3))
+    eng = ExternalQueryEngine(model.to(DEV).train(), ds, batch_size=128, lr=0.05, device=DEV, **kw)
+    idx = torch.arange(128, device=DEV)
+    eng.plain, step = 0, eng._step
+
+    def counted(*a):
+        eng.plain += 1
+        return step(*a)
+    eng._step = counted
+    return eng, (ds.make_batch(idx)[0], idx)
+
+
+def test_replay_follows_a_learning_rate_schedule():
+    """More rates than graphs are kept: every rate is replayed in the end, the oldest graphs go, and a rate that stays for a
+    few steps only does not push out one in use."""
+    eng, batch = _small_engine()
+    view = eng.optimizer_view().param_groups[0]
+    late = eng.STEPS_BEFORE_REPLACING
+    for epoch in range(eng.MAX_GRAPHS + 3):
+        view["lr"] = 0.05 / (epoch + 1)
+        eng.plain = 0
+        for _ in range(late + 10):
+            assert torch.isfinite(eng.step(batch))
+        assert eng.plain == (2 if epoch < eng.MAX_GRAPHS else late + 1), epoch      # the capture runs the step's host side once
+        assert len(eng._graphs) == min(epoch + 1, eng.MAX_GRAPHS)
+    kept = list(eng._graphs)
+    for i in range(2 * eng.MAX_KINDS):                  # a rate of its own for every step
+        view["lr"] = 1e-3 / (i + 1)
+        eng.step(batch)
+    assert list(eng._graphs) == kept and len(eng._seen) == eng.MAX_KINDS
+    view["lr"] = 0.05 / (eng.MAX_GRAPHS + 3)
+    eng.plain = 0
+    eng.step(batch)
+    assert eng.plain == 0
+
+
+def test_a_failed_capture_is_reported_and_the_step_goes_on(caplog):
+    eng, batch = _small_engine()
+    eng.step(batch)
+    forward = eng.model.fc1.forward
+
+    def waits(x):
+        float(x.sum())                                  # a copy to the host: not allowed in a capture
+        return forward(x)
+    eng.model.fc1.forward = waits
+    for _ in range(4):
+        assert torch.isfinite(eng.step(batch))
+    assert not eng._graphs and not eng.use_graph and sum("capture failed" in r.message for r in caplog.records) == 1
