@@ -215,14 +215,18 @@ def test_fused_entity_update_equals_scoring_then_optimizer(kind, nx, ny, D, ctas
             K.kvsall_fused(Xi, y, gi, loss, status, 0.01, 1.0 / 64, True, num_ctas=ctas, mask=mask, pos_delta=0.9,
                            opt=opt)
             if not fused:
+                gmax = float(gi.abs().max()) + wd * float(Pi.abs().max())
                 K.optimizer_step(kind, Pi, gi, mi, vi, Xi, step, lr, b1, b2, eps, wd)
             torch.cuda.synchronize()
             K.check_status(status)
             assert float(gi.abs().max()) == 0.0 and int(count.abs().max()) == 0
             assert torch.equal(Xi, Pi.to(torch.bfloat16))
             res.append((Pi, mi, vi, loss))
+        # ADOPT divides by max(sqrt(v), eps), so the rounding of the gradient sums reaches the moment as (1 - b1) / eps times
+        # itself: about ny / 96 + 2 partial sums that none exceeds gmax, added in any order, differ by 2^-24 gmax per addition
+        noise = 0.1 / eps * 2.0 ** -24 * (ny // 96 + 2) * gmax if kind == 3 else 0.0
         for a, b in zip(*res):
-            assert (a - b).abs().max() <= 2e-5 * a.abs().max().clamp_min(1e-6) + 1e-7
+            assert (a - b).abs().max() <= 2e-5 * a.abs().max().clamp_min(1e-6) + 1e-7 + noise
         P, m, v = res[0][:3]
         step += 1
 
