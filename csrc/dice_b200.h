@@ -52,6 +52,7 @@ int dice_kvsall_fused(const void* x, int x_rows, const void* y, int y_rows, int 
                       const float* y_bias, float* x_dsum, float margin, const DiceFusedOptimizer* opt, void* stream);
 // CTA-pair variant (tcgen05.mma.cta_group::2), D = 256.  loss_share -1 / 0 / 1: all / even / odd 256 x 256 blocks add
 // their loss terms in this launch.  trace: optional int64[64][8] pipeline stamps.
+int dice_kvsall_fused_resources(int D, int with_loss, int masked, int* threads, int* registers, int* shared_bytes);
 int dice_kvsall_pair(const void* x, int x_rows, const void* y, int y_rows, int D, float* out, double* loss, float base,
                      float scale, int with_loss, int* status, int num_pairs, const unsigned int* mask,
                      int mask_stride, float pos_delta, int loss_share, long long* trace, void* stream);

@@ -64,9 +64,7 @@ struct Cfg {
 };
 
 template <int D, bool LOSS, bool MASK, int SCORE>
-__global__ void __launch_bounds__(Cfg<D>::THREADS, 1)
-kvsall_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_y,
-                    const KvsAllParams p) {
+__device__ __forceinline__ void kvsall_fused_body(const CUtensorMap& tmap_x, const CUtensorMap& tmap_y, const KvsAllParams& p) {
   using C = Cfg<D>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -451,11 +449,38 @@ kvsall_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
   }
 }
 
+template <int D, bool LOSS, bool MASK, int SCORE>
+__global__ void __launch_bounds__(Cfg<D>::THREADS, 1)
+kvsall_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_y,
+                    const KvsAllParams p) {
+  kvsall_fused_body<D, LOSS, MASK, SCORE>(tmap_x, tmap_y, p);
+}
+
+// The same compiled to a number of registers that leaves a warp of 32 in each of the SM's four register partitions (16 384
+// each) for the kernels of the sharded step's side branch: of 14 warps at D = 256 a partition holds four at most, hence 120.
+// The occupancy bound alone gives 128 with loss and label masks; at 120 nothing spills and the time is the same (14 541 x 4096
+// 63.5 / 63.5 us, 4096 x 14 541 62.0 / 61.8 us).  Not taken where it costs time: without masks (122 registers; 62.0 -> 63.0 us,
+// and the steps that use it are too long for the side branch to matter), for distances (39.0 -> 41.0 us, single GPU only).
+constexpr int SIDE_REGS = 120;
+template <int D, bool LOSS, bool MASK, int SCORE>
+__global__ void __maxnreg__(SIDE_REGS)
+kvsall_fused_side_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_y,
+                         const KvsAllParams p) {
+  static_assert((Cfg<D>::THREADS / 32 + 3) / 4 * 32 * SIDE_REGS + 32 * 32 <= 16384, "register partition");
+  kvsall_fused_body<D, LOSS, MASK, SCORE>(tmap_x, tmap_y, p);
+}
+
 // ------------------------------------------------------------------------------------ host side
+template <int D, bool LOSS, bool MASK, int SCORE>
+static auto kernel_of() {
+  if constexpr (D == 256 && LOSS && MASK && SCORE == 0) return kvsall_fused_side_kernel<D, LOSS, MASK, SCORE>;
+  else return kvsall_fused_kernel<D, LOSS, MASK, SCORE>;
+}
+
 template <int D, bool LOSS, bool MASK, int SCORE>
 static int launch(const CUtensorMap& tx, const CUtensorMap& ty, const KvsAllParams& p, int num_ctas,
                   cudaStream_t stream) {
-  auto kern = kvsall_fused_kernel<D, LOSS, MASK, SCORE>;
+  auto kern = kernel_of<D, LOSS, MASK, SCORE>();
   static bool configured[64] = {false};   // the attribute is per device: one flag per device ordinal
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -3;
@@ -465,6 +490,16 @@ static int launch(const CUtensorMap& tx, const CUtensorMap& ty, const KvsAllPara
     configured[dev] = true;
   }
   return launch_pdl(kern, dim3(num_ctas), dim3(Cfg<D>::THREADS), Cfg<D>::SMEM_BYTES, stream, tx, ty, p) == cudaSuccess ? 0 : -4;
+}
+
+template <int D, bool LOSS, bool MASK>
+static int resources(int* threads, int* registers, int* shared_bytes) {
+  cudaFuncAttributes a;
+  if (cudaFuncGetAttributes(&a, kernel_of<D, LOSS, MASK, 0>()) != cudaSuccess) return -4;
+  *threads = Cfg<D>::THREADS;
+  *registers = a.numRegs;
+  *shared_bytes = Cfg<D>::SMEM_BYTES + static_cast<int>(a.sharedSizeBytes);
+  return 0;
 }
 
 }  // namespace dice
@@ -548,6 +583,24 @@ extern "C" int dice_kvsall_fused(const void* x, int x_rows, const void* y, int y
       return wl ? launch<DD, true, true, 2>(tx, ty, p, num_ctas, s) : launch<DD, false, true, 2>(tx, ty, p, num_ctas, s); \
     if (wl) return mk ? launch<DD, true, true, 0>(tx, ty, p, num_ctas, s) : launch<DD, true, false, 0>(tx, ty, p, num_ctas, s); \
     return mk ? launch<DD, false, true, 0>(tx, ty, p, num_ctas, s) : launch<DD, false, false, 0>(tx, ty, p, num_ctas, s);
+  switch (D) {
+    DICE_DISPATCH(256)
+    DICE_DISPATCH(128)
+    DICE_DISPATCH(64)
+    default: return -6;
+  }
+#undef DICE_DISPATCH
+}
+
+// What a CTA of the dot-product form takes of its SM: threads, registers per thread, bytes of shared memory.
+extern "C" int dice_kvsall_fused_resources(int D, int with_loss, int masked, int* threads, int* registers, int* shared_bytes) {
+  using namespace dice;
+#define DICE_DISPATCH(DD)                                                                                          \
+  case DD:                                                                                                         \
+    if (with_loss) return masked ? resources<DD, true, true>(threads, registers, shared_bytes)                     \
+                                 : resources<DD, true, false>(threads, registers, shared_bytes);                   \
+    return masked ? resources<DD, false, true>(threads, registers, shared_bytes)                                   \
+                  : resources<DD, false, false>(threads, registers, shared_bytes);
   switch (D) {
     DICE_DISPATCH(256)
     DICE_DISPATCH(128)

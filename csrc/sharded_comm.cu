@@ -521,12 +521,13 @@ extern "C" int dice_compose_backward_owner(int model, int normalize, const long 
 //   dice_dq_pull_owner sums, for every listed row, the W partial rows (one per rank, in dq_table) by peer loads and puts
 //                      the sum in place of this rank's own partial row in dq_local.  Nobody else reads those rows (a
 //                      peer pulls only the rows IT owns), so the update is in place.
-// Both run on a graph branch beside the entity-role scoring launch, whose one CTA per SM (18 warps of 96 registers)
-// leaves room for ONE more warp of at most 32 registers in each of the SM's four register partitions (measured: blocks
-// of 256 threads do not start until the scoring CTA has left, a one-warp kernel does).  Hence blocks of 128 threads
-// capped at 32 registers.  The pull is a persistent grid (16 bytes per work item, W independent loads in flight per
-// thread); because the list holds owned rows only, every thread has loads in flight, which is what keeps NVLink busy
-// at one resident block per SM.  The backward of the composition afterwards reads local memory only.
+// Both run on a graph branch beside the entity-role scoring launch, whose one CTA per SM (18 warps of 96 registers, at
+// D = 256 with label masks 14 warps of 120) leaves room for ONE more warp of at most 32 registers in each of the SM's four
+// register partitions (measured with the 18-warp CTA: blocks of 256 threads do not start until it has left the SM, a
+// one-warp kernel does).  Hence blocks of 128 threads capped at 32 registers.  The pull is a persistent grid (16 bytes per
+// work item, W independent loads in flight per thread); because the list holds owned rows only, every thread has loads in
+// flight, which is what keeps NVLink busy at one resident block per SM.  The backward of the composition afterwards reads
+// local memory only.
 namespace dice {
 // Kernels meant to run beside a scoring launch ask for the same shared-memory carveout as that launch (the maximum):
 // an SM is not shared between kernels that want different carveouts.

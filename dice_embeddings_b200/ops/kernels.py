@@ -159,6 +159,15 @@ def kvsall_fused(x: torch.Tensor, y: torch.Tensor, out: torch.Tensor, loss_acc: 
           others=(y, out, loss_acc, status, mask, trace, x_bias, y_bias, x_dsum))
 
 
+def kvsall_fused_resources(D: int, with_loss: bool, masked: bool):
+    """``(threads, registers per thread, bytes of shared memory)`` of a CTA of :func:`kvsall_fused`: what it leaves of an SM
+    decides which kernels can run beside it."""
+    out = (ctypes.c_int * 3)()
+    _check(_lib.lib().dice_kvsall_fused_resources(int(D), int(with_loss), int(masked), *[ctypes.byref(out, 4 * i) for i in range(3)]),
+           "dice_kvsall_fused_resources")
+    return tuple(out)
+
+
 def padded_rows(n: int) -> int:
     """Length the per-row scalar vectors of :func:`kvsall_fused` need for ``n`` rows (whole 128-row tiles)."""
     return (int(n) + 127) // 128 * 128

@@ -586,3 +586,14 @@ def test_stage_copies_every_array(sizes):
     a, b = torch.zeros(20, dtype=torch.int64, device=DEV), torch.zeros(20, dtype=torch.int64, device=DEV)
     K.stage((a, strided), (b, strided.to(torch.int32)))
     assert torch.equal(a, strided) and torch.equal(b, strided)
+
+
+@pytest.mark.parametrize("D", [64, 128, 256])
+@pytest.mark.parametrize("with_loss,masked", [(False, False), (False, True), (True, True)])
+def test_scoring_cta_leaves_room_for_the_side_branch(D, with_loss, masked):
+    """The launches with label masks: the kernels of the sharded step's side branch come in blocks of four warps of 32 registers, one per register partition of
+    16 384: the scoring CTA's warps (a quarter of them per partition, registers in units of eight) must leave that much."""
+    threads, regs, shared = K.kvsall_fused_resources(D, with_loss, masked)
+    per_partition = (threads // 32 + 3) // 4
+    assert per_partition * 32 * ((regs + 7) // 8 * 8) + 32 * 32 <= 16384, (threads, regs)
+    assert shared + 1024 + 1024 <= 228 * 1024            # and the shared memory every resident block costs
