@@ -436,12 +436,16 @@ extern "C" int dice_eval_rank(const void* x, int x_rows, const void* y, int y_ro
   if (k != 0 && (cand_score == nullptr || cand_idx == nullptr || cand_count == nullptr || cand_cap < k)) return -7;
   if (k == -1 && row_floor == nullptr) return -7;
   if (margin != nullptr && (k > 0 || band_rows == nullptr || band_cols == nullptr || band_count == nullptr)) return -7;
-  if (k == -1)
-    return dice_rank_collect(x, x_rows, y, y_rows, D, col_bias, y_offset, y_stride, row_floor, cand_cap, 0, cand_score, cand_idx,
-                             cand_count, status, num_ctas, stream);
+  if (k == -1) {
+    const int rc = dice_rank_collect(x, x_rows, y, y_rows, D, col_bias, y_offset, y_stride, row_floor, cand_cap, 0, cand_score,
+                                     cand_idx, cand_count, status, num_ctas, stream);
+    if (rc != 0 || target == nullptr || greater == nullptr) return rc;
+    return dice_rank_count(x, nullptr, x_rows, y, nullptr, y_rows, D, target, target_idx, col_bias, y_offset, y_stride, nullptr, 0,
+                           greater, nullptr, nullptr, nullptr, nullptr, 0, status, num_ctas, stream);
+  }
   if (k == 0) {
     if (D != 64 && D != 128 && D != 256) return -6;
-    if (target == nullptr || greater == nullptr) return 0;   // nothing can be counted
+    if (target == nullptr || (greater == nullptr && margin == nullptr)) return 0;   // nothing to count or to list
     return dice_rank_count(x, nullptr, x_rows, y, nullptr, y_rows, D, target, target_idx, col_bias, y_offset, y_stride, nullptr, 0,
                            greater, margin, band_rows, band_cols, band_count, band_cap, status, num_ctas, stream);
   }

@@ -435,7 +435,7 @@ rank_tiles_kernel(const __grid_constant__ CUtensorMap tmap_y, const __grid_const
       if constexpr (MODE == COUNT || MODE == BAND) {
 #pragma unroll
         for (int u = 0; u < UN; ++u)
-          if (valid[u] && cnt[u] != 0) atomicAdd(p.greater + x_global[u], cnt[u]);
+          if (valid[u] && cnt[u] != 0 && p.greater != nullptr) atomicAdd(p.greater + x_global[u], cnt[u]);
       }
       w += n;
       ++seg;
@@ -603,7 +603,7 @@ extern "C" int dice_rank_count(const void* x, const void* x_lo, int x_rows, cons
                                int* status, int num_ctas, void* stream) {
   using namespace dice::rankk;
   if (x_rows <= 0 || y_rows <= 0) return 0;
-  if (target == nullptr || greater == nullptr) return -7;
+  if (target == nullptr || (greater == nullptr && margin == nullptr)) return -7;   // a band may be listed without counts
   if (margin != nullptr ? (band_rows == nullptr || band_cols == nullptr || band_count == nullptr) : x_lo != nullptr) return -7;
   RankParams p{};
   p.x = static_cast<const __nv_bfloat16*>(x);

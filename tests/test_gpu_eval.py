@@ -436,3 +436,26 @@ def _check_topk_close(sc, ix, x, y, k):
     scores = x.float() @ y.float().t()
     assert torch.allclose(sc, torch.topk(scores, k, dim=1).values, atol=1e-3)
     assert torch.allclose(torch.gather(scores, 1, ix), sc, atol=1e-3)
+
+
+def test_collecting_with_counts_and_a_band_without():
+    """``eval_rank`` counts beside collecting when it is given a target and a count buffer, and lists a band without one."""
+    nx, ny, D = 150, 2000, 64
+    x, y = _operands(nx, ny, D, 21)
+    scores = x.float() @ y.float().t()
+    tgt = torch.randint(0, ny, (nx,), device=DEV, dtype=torch.int32)
+    ts = scores[torch.arange(nx, device=DEV), tgt.long()].contiguous()
+    want = torch.zeros(nx, dtype=torch.int32, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    K.eval_rank(x, y, ts, tgt, want, status)
+    greater, count = torch.zeros(nx, dtype=torch.int32, device=DEV), torch.zeros(nx, dtype=torch.int32, device=DEV)
+    lists = torch.full((nx, 100), float("-inf"), device=DEV), torch.full((nx, 100), -1, dtype=torch.int32, device=DEV)
+    floor = torch.topk(scores, 20, dim=1).values[:, -1].contiguous() - 1e-3
+    K.eval_rank(x, y, ts, tgt, greater, status, k=-1, cand_score=lists[0], cand_idx=lists[1], cand_count=count, row_floor=floor)
+    assert torch.equal(greater, want) and int(want.sum()) > 0 and ((count >= 20) & (count < 25)).all()
+    rows, cols = (torch.zeros(nx * ny, dtype=torch.int32, device=DEV) for _ in range(2))
+    n = torch.zeros(2, dtype=torch.int64, device=DEV)
+    for i, g in enumerate((torch.zeros(nx, dtype=torch.int32, device=DEV), None)):
+        K.eval_rank(x, y, ts, tgt, g, status, margin=torch.full((nx,), 0.05, device=DEV), band_rows=rows, band_cols=cols,
+                    band_count=n[i:i + 1])
+    assert int(status) == 0 and int(n[0]) > 0 and int(n[0]) == int(n[1])
