@@ -50,8 +50,9 @@ class FusedRanker:
                  y_stride: int = 1, group=None, exact: bool = False, band_capacity: int = 1 << 24):
         """``exact``: ranks equal those of an fp32 scoring of the same operands.  The tensor cores still do the bulk of the
         work, on operands split into two bf16 terms each; such a score differs from its fp32 value by at most
-        ``MARGIN[d] · ‖q‖ · ‖e‖`` (plus the rounding of the bias), so only entities within that margin of the target are undecided, and exactly those
-        (well below a tenth of a percent) are re-scored in fp32 by a second, sparse pass."""
+        ``MARGIN[d] · ‖q‖ · ‖e‖`` (plus the rounding of the bias), so only entities within that margin of the target are
+        undecided, and exactly those (0.2 percent for targets in the middle of a random table, far fewer near its top) are
+        re-scored in fp32 by a second, sparse pass."""
         assert table.is_cuda, "the fused ranker runs on a CUDA device"
         self.d = table.shape[1]
         self.d_pad = pad_dim(self.d)
@@ -165,19 +166,19 @@ class FusedRanker:
             filt_ptr = filt_ptr.to(torch.int64).contiguous()
             filt_cols = filt_cols.to(torch.int32).contiguous()
             if self.y_offset == 0 and self.y_stride == 1 and self._mask_pays(B, filt_cols.numel()):
-                cleared, mask, repeated = self._cleared(B, self._mask_words())
+                cleared, mask, buf = self._cleared(B, self._mask_words())
+                repeated = buf[-B:]
                 kernels.filter_mask(mask, self.table.shape[0], ptr=filt_ptr, cols=filt_cols, repeated=repeated)
                 return self._ranks(q, target, filt_ptr, filt_cols, mask, cleared, repeated=repeated)
         return self._ranks(q, target, filt_ptr, filt_cols, None)
 
     def _cleared(self, B: int, words: int):
-        """Zeros for one batch in one fill: target scores and counts (and the band's counter), the mask ``[B, words]`` and the
-        flags of lists that repeat an answer."""
+        """Zeros for one batch in one fill: target scores and counts (and the band's counter), the mask ``[B, words]``, and behind
+        them ``B`` more."""
         rows = (B + 3) // 4 * 4
-        buf = torch.zeros(3 * rows + 4 + B * words, dtype=torch.int32, device=self.device)
-        small, mask = buf[:3 * rows + 4], buf[3 * rows + 4:].view(B, words)
-        return (small[:B].view(torch.float32), small[rows:rows + B], small[2 * rows:2 * rows + 2].view(torch.int64)), mask, \
-            small[2 * rows + 4:2 * rows + 4 + B]
+        buf = torch.zeros(2 * rows + 4 + B * words + B, dtype=torch.int32, device=self.device)
+        mask = buf[2 * rows + 4:-B].view(B, words) if words else None
+        return (buf[:B].view(torch.float32), buf[rows:rows + B], buf[2 * rows:2 * rows + 2].view(torch.int64)), mask, buf
 
     @torch.no_grad()
     def ranks_of_pairs(self, q: torch.Tensor, target: torch.Tensor, ab: torch.Tensor, num_b: int, keys: torch.Tensor,
