@@ -69,7 +69,8 @@ int dice_rank_collect(const void* x, int x_rows, const void* y, int y_rows, int 
                       int* cand_count, int* status, int num_ctas, void* stream);
 int dice_filter_mask(int n, const long long* ptr, const int* cols, const long long* ab, long long ab_stride, long long num_b,
                      const long long* keys, long long num_keys, const long long* offsets, const long long* values,
-                     unsigned int* mask, long long mask_stride, int y_rows, int* repeated, void* stream);
+                     unsigned int* mask, long long mask_stride, int y_rows, unsigned int* repeated,
+                     void* stream);
 int dice_split_rows(const float* src, long long src_stride, long long n, int d, int d_pad, void* hi, void* lo, float* copy,
                     float* margin, float factor, float offset, void* stream);
 int dice_topk_floor(const float* gmax, int rows, int groups, int k, float* floor, int* cand_count, void* stream);
@@ -87,7 +88,7 @@ int dice_eval_rank(const void* x, int x_rows, const void* y, int y_rows, int D, 
 int dice_eval_rank_cand_cap(int x_rows, int y_rows, int D, int k, int num_ctas);
 int dice_eval_sparse(const void* q, const void* y, int n, int D, int y_rows, int y_offset, int y_stride,
                      const int* target, const float* col_bias, const float* target_in, const long long* filt_ptr,
-                     const int* filt_cols, const int* repeated, float* target_score, int* filtered_greater,
+                     const int* filt_cols, const unsigned int* repeated, float* target_score, int* filtered_greater,
                      int fp32_operands, void* stream);
 int dice_eval_band_exact(const float* q, const float* y, int D, int y_rows, int y_offset, int y_stride,
                          const float* col_bias, const int* band_rows, const int* band_cols,

@@ -332,7 +332,7 @@ __global__ void eval_sparse_kernel(const T* __restrict__ q, const T* __restrict_
                                    int D, int y_rows, int y_offset, int y_stride, const int* __restrict__ target,
                                    const float* __restrict__ col_bias, const float* __restrict__ target_in,
                                    const long long* __restrict__ filt_ptr, const int* __restrict__ filt_cols,
-                                   const int* __restrict__ repeated, float* __restrict__ target_score,
+                                   const uint32_t* __restrict__ repeated, float* __restrict__ target_score,
                                    int* __restrict__ filtered_greater) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -369,21 +369,22 @@ __global__ void eval_sparse_kernel(const T* __restrict__ q, const T* __restrict_
     if (lane == 0 && target_score != nullptr) target_score[warp] = ts;
   }
   if (filt_ptr == nullptr || filtered_greater == nullptr) return;
-  if (repeated != nullptr && repeated[warp] == 0) return;
   int cnt = 0;
   const long long beg = filt_ptr[warp], end = filt_ptr[warp + 1];
-  for (long long e = beg; e < end; ++e) {
+  auto beats = [&](long long e) -> int {
     const int j = filt_cols[e];
     const int jl = local_row(j);
-    if (j == tg || jl < 0) continue;
-    if (repeated != nullptr) {   // the first mention is in the mask: count the further ones
-      bool seen = false;
-      for (long long f = beg + lane; f < e; f += 32) seen |= filt_cols[f] == j;
-      if (!__any_sync(0xffffffffu, seen)) continue;
-    }
-    cnt += dot(jl) > ts ? 1 : 0;
+    return j != tg && jl >= 0 && dot(jl) > ts ? 1 : 0;
+  };
+  if (repeated != nullptr) {   // the first mention of an answer is in the mask: count the further ones
+    const uint32_t* rep = repeated + beg / 32 + warp;
+    for (long long e = beg; e < end; e += 32)
+      for (uint32_t bits = rep[(e - beg) / 32]; bits != 0u; bits &= bits - 1) cnt += beats(e + __ffs(bits) - 1);
+    if (lane == 0 && cnt != 0) filtered_greater[warp] = -cnt;
+    return;
   }
-  if (lane == 0) filtered_greater[warp] = repeated != nullptr ? -cnt : cnt;
+  for (long long e = beg; e < end; ++e) cnt += beats(e);
+  if (lane == 0) filtered_greater[warp] = cnt;
 }
 
 // Exact second pass of the band mode: one warp per undecided (query, entity) pair, fp32 operands; the pair counts
@@ -523,11 +524,11 @@ extern "C" int dice_eval_rank_cand_cap(int x_rows, int y_rows, int D, int k, int
 }
 
 // Target scores, and per query the number of listed entities that beat the target, as often as they are listed.  With
-// repeated [n] (see dice_filter_mask) only second and further mentions in the flagged lists count, and
-// filtered_greater[i] is set to minus their number (left alone where the flag is zero).
+// repeated (see dice_filter_mask) only second and further mentions count, and filtered_greater[i] is set to minus their number
+// (left alone where there are none).
 extern "C" int dice_eval_sparse(const void* q, const void* y, int n, int D, int y_rows, int y_offset, int y_stride,
                                 const int* target, const float* col_bias, const float* target_in,
-                                const long long* filt_ptr, const int* filt_cols, const int* repeated, float* target_score,
+                                const long long* filt_ptr, const int* filt_cols, const unsigned int* repeated, float* target_score,
                                 int* filtered_greater, int fp32_operands, void* stream) {
   using namespace dice::evalk;
   if (n <= 0) return 0;

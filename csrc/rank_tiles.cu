@@ -520,7 +520,8 @@ struct MaskParams {
   uint32_t* mask;
   long long stride;
   int y_rows;
-  int* repeated;               // [n] set where a list names an answer more than once; may be null
+  uint32_t* repeated;          // bits of the entries whose answer their list has named before, list i from word
+                               // ptr[i] / 32 + i on; may be null
 };
 
 __global__ void __launch_bounds__(256) filter_mask_kernel(const MaskParams p) {
@@ -550,19 +551,31 @@ __global__ void __launch_bounds__(256) filter_mask_kernel(const MaskParams p) {
     end = p.offsets[lo + 1];
   }
   uint32_t* row = p.mask + i * p.stride;
-  for (long long e0 = beg + lane; e0 < end; e0 += 128) {   // four loads in flight: popular pairs have thousands of answers
+  uint32_t* rep = p.repeated != nullptr ? p.repeated + beg / 32 + i : nullptr;
+  for (long long b0 = beg; b0 < end; b0 += 128) {   // four loads in flight: popular pairs have thousands of answers
     long long c[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const long long e = e0 + 32 * j;
+      const long long e = b0 + 32 * j + lane;
       c[j] = e >= end ? -1 : p.ptr != nullptr ? static_cast<long long>(p.cols[e]) : p.values[e];
     }
+    bool again[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < 4; ++j) {
+      again[j] = false;
       if (c[j] >= 0 && c[j] < p.y_rows) {
-        const uint32_t bit = 1u << (c[j] & 31), before = atomicOr(row + (c[j] >> 5), bit);
-        if (p.repeated != nullptr && (before & bit)) p.repeated[i] = 1;
+        const uint32_t bit = 1u << (c[j] & 31);
+        if (rep == nullptr) atomicOr(row + (c[j] >> 5), bit);   // no value to wait for (8 us a batch of 4096 popular pairs)
+        else again[j] = (atomicOr(row + (c[j] >> 5), bit) & bit) != 0u;
       }
+    }
+    if (rep != nullptr) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t bits = __ballot_sync(0xffffffffu, again[j]);
+        if (lane == 0 && b0 + 32 * j < end) rep[(b0 - beg) / 32 + j] = bits;
+      }
+    }
   }
 }
 
@@ -672,14 +685,16 @@ extern "C" int dice_rank_collect(const void* x, int x_rows, const void* y, int y
 }
 
 // Sets the mask bits of the known answers of n queries: of (ptr [n + 1], cols), or with ptr == null of the pairs ab (two
-// leading columns, row stride ab_stride) found in keys / offsets / values.  With repeated [n], entries of lists that name an
-// answer more than once are set to one.  Mask and flags are cleared by the caller.
+// leading columns, row stride ab_stride) found in keys / offsets / values.  The mask is cleared by the caller.  repeated (with
+// ptr, optional): one bit per entry of cols, set where its list has named the answer before (dice_eval_sparse reads it); the
+// words of list i start at ptr[i] / 32 + i, which no two lists share; ptr[n] / 32 + n words, need not be cleared.
 extern "C" int dice_filter_mask(int n, const long long* ptr, const int* cols, const long long* ab, long long ab_stride,
                                 long long num_b, const long long* keys, long long num_keys, const long long* offsets,
-                                const long long* values, unsigned int* mask, long long mask_stride, int y_rows, int* repeated, void* stream) {
+                                const long long* values, unsigned int* mask, long long mask_stride, int y_rows, unsigned int* repeated,
+                                void* stream) {
   using namespace dice::rankk;
   if (n <= 0) return 0;
-  if (mask == nullptr || mask_stride * 32 < y_rows) return -7;
+  if (mask == nullptr || mask_stride * 32 < y_rows || (repeated != nullptr && ptr == nullptr)) return -7;
   if (ptr == nullptr ? (ab == nullptr || (num_keys > 0 && (keys == nullptr || offsets == nullptr || values == nullptr))) : cols == nullptr)
     return -7;
   const MaskParams p{n, ptr, cols, ab, ab_stride, num_b, keys, num_keys, offsets, values, mask, mask_stride, y_rows, repeated};

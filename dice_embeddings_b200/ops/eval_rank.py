@@ -166,19 +166,18 @@ class FusedRanker:
             filt_ptr = filt_ptr.to(torch.int64).contiguous()
             filt_cols = filt_cols.to(torch.int32).contiguous()
             if self.y_offset == 0 and self.y_stride == 1 and self._mask_pays(B, filt_cols.numel()):
-                cleared, mask, buf = self._cleared(B, self._mask_words())
-                repeated = buf[-B:]
+                cleared, mask = self._cleared(B, self._mask_words())
+                repeated = torch.empty(filt_cols.numel() // 32 + B, dtype=torch.int32, device=self.device)
                 kernels.filter_mask(mask, self.table.shape[0], ptr=filt_ptr, cols=filt_cols, repeated=repeated)
                 return self._ranks(q, target, filt_ptr, filt_cols, mask, cleared, repeated=repeated)
         return self._ranks(q, target, filt_ptr, filt_cols, None)
 
     def _cleared(self, B: int, words: int):
-        """Zeros for one batch in one fill: target scores and counts (and the band's counter), the mask ``[B, words]``, and behind
-        them ``B`` more."""
+        """Zeros for one batch in one fill: target scores and counts (and the band's counter) and the mask ``[B, words]``."""
         rows = (B + 3) // 4 * 4
-        buf = torch.zeros(2 * rows + 4 + B * words + B, dtype=torch.int32, device=self.device)
-        mask = buf[2 * rows + 4:-B].view(B, words) if words else None
-        return (buf[:B].view(torch.float32), buf[rows:rows + B], buf[2 * rows:2 * rows + 2].view(torch.int64)), mask, buf
+        buf = torch.zeros(2 * rows + 4 + B * words, dtype=torch.int32, device=self.device)
+        small, mask = buf[:2 * rows + 4], buf[2 * rows + 4:].view(B, words)
+        return (small[:B].view(torch.float32), small[rows:rows + B], small[2 * rows:2 * rows + 2].view(torch.int64)), mask
 
     @torch.no_grad()
     def ranks_of_pairs(self, q: torch.Tensor, target: torch.Tensor, ab: torch.Tensor, num_b: int, keys: torch.Tensor,
@@ -186,7 +185,7 @@ class FusedRanker:
         """:meth:`ranks` with the filter of query ``i`` given as the pair in the first two columns of ``ab[i]``, looked up on
         the device in a CSR over sorted keys ``a * num_b + b`` (whole table on this device)."""
         assert self.group is None and self.y_offset == 0 and self.y_stride == 1
-        cleared, mask, _ = self._cleared(q.shape[0], self._mask_words())
+        cleared, mask = self._cleared(q.shape[0], self._mask_words())
         kernels.filter_mask(mask, self.table.shape[0], ab=ab, num_b=num_b, keys=keys, offsets=offsets, values=values)
         return self._ranks(q, target, None, None, mask, cleared, out)
 

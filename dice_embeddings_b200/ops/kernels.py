@@ -622,8 +622,8 @@ def filter_mask(mask: torch.Tensor, y_rows: int, ptr: Optional[torch.Tensor] = N
                 repeated: Optional[torch.Tensor] = None) -> None:
     """Set the bits of the known answers of every query in ``mask`` (cleared by the caller): of the CSR ``ptr`` / ``cols``
     over the batch, or of the pairs in the first two columns of ``ab`` looked up in ``keys`` / ``offsets`` / ``values``
-    (``key = a * num_b + b``, ascending).  ``repeated`` (int32 per query, zeros before) is set to one where a list names an
-    answer more than once."""
+    (``key = a * num_b + b``, ascending).  ``repeated`` (with ``ptr``; int32 ``[len(cols) // 32 + queries]``) receives a
+    bit per entry, set where its list has named the answer before."""
     _req(mask, torch.int32, "mask")
     if ptr is not None:
         _req(ptr, torch.int64, "ptr")
@@ -639,7 +639,7 @@ def filter_mask(mask: torch.Tensor, y_rows: int, ptr: Optional[torch.Tensor] = N
     assert mask.shape[0] >= n
     if repeated is not None:
         _req(repeated, torch.int32, "repeated")
-        assert repeated.numel() >= n
+        assert ptr is not None and repeated.numel() >= cols.numel() // 32 + n
     _call("dice_filter_mask", mask, n, _ptr(ptr), _ptr(cols), _ptr(ab), 0 if ab is None else ab.stride(0), int(num_b),
           _ptr(keys), 0 if keys is None else keys.numel(), _ptr(offsets), _ptr(values), _ptr(mask), mask.shape[1], int(y_rows),
           _ptr(repeated), others=(ptr, cols, ab, keys, offsets, values, repeated))
@@ -756,8 +756,8 @@ def eval_sparse(q: torch.Tensor, y: torch.Tensor, target_idx: torch.Tensor, targ
                 target_in: Optional[torch.Tensor] = None, y_offset: int = 0, y_stride: int = 1,
                 repeated: Optional[torch.Tensor] = None) -> None:
     """Gather-dots of the ranking protocol: the target score of each query and the number of filtered entities (CSR
-    ``filt_ptr`` int64 / ``filt_cols`` int32) that beat it.  With the ``repeated`` flags of :func:`filter_mask` only second
-    and further mentions in the flagged lists count, and ``filtered_greater`` (zeros before) receives minus their number."""
+    ``filt_ptr`` int64 / ``filt_cols`` int32) that beat it.  With the ``repeated`` bits of :func:`filter_mask` only second
+    and further mentions count, and ``filtered_greater`` (zeros before) receives minus their number."""
     fp32 = q.dtype == torch.float32
     _req(q, torch.float32 if fp32 else torch.bfloat16, "q")
     _req(y, q.dtype, "y")
@@ -767,7 +767,7 @@ def eval_sparse(q: torch.Tensor, y: torch.Tensor, target_idx: torch.Tensor, targ
         _req(filt_cols, torch.int32, "filt_cols")
     if repeated is not None:
         _req(repeated, torch.int32, "repeated")
-        assert repeated.numel() >= q.shape[0]
+        assert repeated.numel() >= filt_cols.numel() // 32 + q.shape[0]
     _call("dice_eval_sparse", q, _ptr(q), _ptr(y), q.shape[0], q.shape[1], y.shape[0], int(y_offset), int(y_stride),
           _ptr(target_idx), _ptr(col_bias), _ptr(target_in), _ptr(filt_ptr), _ptr(filt_cols), _ptr(repeated),
           _ptr(target_score), _ptr(filtered_greater), int(fp32),

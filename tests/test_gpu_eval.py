@@ -330,6 +330,7 @@ def test_repeated_answers_in_a_filter(exact, masked):
     tgt = torch.randint(0, ny, (nx,), device=DEV)
     lists = [torch.randint(0, 25, (90,)) if i % 3 == 0 else torch.randperm(ny)[:40] if i % 3 == 1 else torch.zeros(0).long() for i in range(nx)]
     lists[0][7:9] = int(tgt[0])
+    lists[1] = torch.arange(129) // 2 * 3           # more than one round of the mask kernel, repeats across its words
     ptr = torch.zeros(nx + 1, dtype=torch.int64)
     ptr[1:] = torch.tensor([len(a) for a in lists]).cumsum(0)
     rows, cols = torch.repeat_interleave(torch.arange(nx), ptr[1:] - ptr[:-1]).to(DEV), torch.cat(lists).to(DEV)
