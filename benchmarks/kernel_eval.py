@@ -1,10 +1,10 @@
-"""Stand-alone timing of the ranking kernel: ``python benchmarks/kernel_eval.py``.
+"""Stand-alone timing of the ranking kernels: ``python benchmarks/kernel_eval.py``.
 
-Times ``eval_rank`` (counting mode and top-k mode) with CUDA events after warm-up, flushing L2 between launches, and
-reports the achieved tensor throughput (one GEMM of ``2·B·|E|·D`` FLOP per launch) as a fraction of the cuBLAS bf16
-figure in ``MEASURED_PEAKS.json``.  With ``--compare`` it also times the PyTorch formulation of the same counts
-(``torch.mm`` per 1024 queries + comparison + row sum).  It is the small, self-terminating program used for ``ncu``
-captures of this kernel."""
+Times the counting kernel that ``FusedRanker`` launches (``rank_count``, and with ``--band`` its form on split operands with
+an undecided band, three GEMMs) and the top-k search with CUDA events after warm-up, flushing L2 between launches, and
+reports the achieved tensor throughput (``2·B·|E|·D`` FLOP per GEMM) as a fraction of the cuBLAS bf16 figure in
+``MEASURED_PEAKS.json``.  With ``--compare`` it also times the PyTorch formulation of the same counts (``torch.mm`` per 1024
+queries + comparison + row sum).  It is the small, self-terminating program used for ``ncu`` captures of these kernels."""
 from __future__ import annotations
 
 import argparse
@@ -28,6 +28,7 @@ def main():
     ap.add_argument("--iters", type=int, default=10)
     ap.add_argument("--warmup", type=int, default=3)
     ap.add_argument("--topk", type=int, default=0, help="also time top-k mode with this k on the first 256 queries")
+    ap.add_argument("--band", action="store_true", help="also time the counting kernel on split operands")
     ap.add_argument("--topk_queries", type=int, default=256)
     ap.add_argument("--compare", action="store_true")
     a = ap.parse_args()
@@ -58,31 +59,32 @@ def main():
             ms += e0.elapsed_time(e1)
         return ms / iters
 
-    ms = timed(lambda: K.eval_rank(q, y, ts, tgt, greater, status), a.iters)
-    tf = 2.0 * a.queries * a.entities * a.d / (ms * 1e-3) / 1e12
-    print(f"eval_rank  B={a.queries} E={a.entities} D={a.d}: {ms * 1e3:9.1f} us  {tf:7.1f} TFLOP/s  "
-          f"{tf / pk['bf16_tflops']:.2f} of {pk['source']} ({pk['bf16_tflops']:.0f})")
+    def report(name, ms, gemms):
+        tf = 2.0 * gemms * a.queries * a.entities * a.d / (ms * 1e-3) / 1e12
+        print(f"{name}  B={a.queries} E={a.entities} D={a.d}: {ms * 1e3:9.1f} us  {tf:7.1f} TFLOP/s  "
+              f"{tf / pk['bf16_tflops']:.2f} of {pk['source']} ({pk['bf16_tflops']:.0f})")
+
+    report("rank_count", timed(lambda: K.rank_count(q, y, ts, tgt, greater, status), a.iters), 1)
+    if a.band:
+        q32, y32 = q.float() + 1e-3 * torch.randn_like(q.float()), y.float() + 1e-3 * torch.randn_like(y.float())
+        yh, yl, _, _ = K.split_rows(y32, a.d)
+        qh, ql, _, margin = K.split_rows(q32, a.d, margin_factor=float(y32.norm(dim=1).max()) * FusedRanker.MARGIN[a.d])
+        K.eval_sparse(q32, y32, tgt, ts, None)
+        rows, cols = (torch.empty(1 << 24, dtype=torch.int32, device=dev) for _ in range(2))
+        count = torch.zeros(1, dtype=torch.int64, device=dev)
+
+        def banded():
+            count.zero_()
+            K.rank_count(qh, yh, ts, tgt, greater, status, x_lo=ql, y_lo=yl, margin=margin, band_rows=rows, band_cols=cols,
+                         band_count=count)
+        report("rank_count, split operands", timed(banded, a.iters), 3)
+        print(f"   undecided: {int(count) / (a.queries * a.entities):.1e} of the pairs")
     if a.topk:
         r = FusedRanker(y)
         n = min(a.topk_queries, a.queries)
         ms = timed(lambda: r.topk(q[:n], a.topk), max(a.iters // 2, 1))
-        print(f"top-{a.topk} of {n} queries over {a.entities} entities: {ms * 1e3:9.1f} us (with candidate merge)")
-        cap = K.eval_rank_cand_cap(n, a.entities, a.d, a.topk)
-        cs = torch.full((n, cap), float("-inf"), device=dev)
-        ci = torch.full((n, cap), -1, dtype=torch.int32, device=dev)
-        cc = torch.zeros(n, dtype=torch.int32, device=dev)
-        qn = q[:n].contiguous()
-
-        fl = torch.empty(n, device=dev)
-
-        def kernel_only():
-            cc.zero_()
-            fl.fill_(float("-inf"))
-            K.eval_rank(qn, y, None, None, None, status, k=a.topk, cand_score=cs, cand_idx=ci, cand_count=cc,
-                        row_floor=fl)
-        ms = timed(kernel_only, max(a.iters // 2, 1))
-        tfk = 2.0 * n * a.entities * a.d / (ms * 1e-3) / 1e12
-        print(f"   kernel alone: {ms * 1e3:9.1f} us  {tfk:7.1f} TFLOP/s  (candidate capacity {cap} per row)")
+        r.check()
+        print(f"top-{a.topk} of {n} queries over {a.entities} entities: {ms * 1e3:9.1f} us")
     if a.compare:
         def torch_counts():
             out = []

@@ -17,12 +17,12 @@ struct KvsAllParams {
   float base;           // label value outside the positives (smoothing term)
   float scale;          // factor applied to out (1 / (B * |E|) for a mean-reduced loss)
   const uint32_t* mask; // MASK: bit y of row x set where (x, y) is a positive label; row stride mask_stride words
-  int mask_stride;      // (a multiple of 4, so the two words a thread needs per tile are one aligned 8-byte load)
+  int mask_stride;      // (a multiple of 4; a thread reads one word per tile)
   float pos_delta;      // label(positive) - base
   long long* trace;     // optional [64 tiles][8] clock64 stamps written by CTA 0 (pipeline diagnostics), else null
   // SCORE != 0: the logit is a function of the dot product and one scalar per row of X and of Y
-  const float* x_bias;  // [nx_tiles * 128] or null (= 0): SCORE 1 bias of row x; SCORE 2 squared norm of row x
-  const float* y_bias;  // [ny_tiles * 128] or null (= 0), padded to whole tiles: the same for the rows of Y
+  const float* x_bias;  // [x_rows] or null (= 0): SCORE 1 bias of row x; SCORE 2 squared norm of row x
+  const float* y_bias;  // the same for the rows of Y, or null (= 0); readable up to the next multiple of 128 rows
   float* x_dsum;        // optional [x_rows]: += scale * sum over y of the value fed to the second GEMM
   float margin;         // SCORE 2: logit = margin - sqrt(|x|^2 + |y|^2 - 2 x.y)
   // Optimiser fused into the drain (opt.param != null): out is then the gradient buffer of the rows of X, and the CTA
@@ -41,7 +41,6 @@ __device__ __forceinline__ float fast_tanh(float x) {
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-
 
 // Position of one GEMM stream inside this CTA's range of flattened (x tile, y tile) pairs; a segment is a run of
 // tiles sharing the x tile.

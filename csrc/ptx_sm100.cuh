@@ -129,20 +129,10 @@ __device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
       : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem desc]
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                       uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
-      : "memory");
-}
 
-// The same three for a warp whose lanes all take part (same operands in every lane): one elected lane issues.  The operands
-// stay warp-uniform values, which the instruction needs; from inside a branch that one lane took, each MMA first had to move
-// its descriptors over, about 95 cycles per MMA whatever its width.
+// Commit and MMA for a warp whose lanes all take part (same operands in every lane): one elected lane issues.  The operands stay
+// warp-uniform values, which the instruction needs; from inside a branch that one lane took, each MMA first had to move its
+// descriptors over, about 95 cycles per MMA whatever its width.
 __device__ __forceinline__ void tc_commit_warp(uint64_t* bar) {
   asm volatile(
       "{\n\t.reg .pred q;\n\t"
@@ -161,6 +151,7 @@ __device__ __forceinline__ void mma_ss_warp(uint32_t d_tmem, uint64_t a_desc, ui
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
       : "memory");
 }
+// D[tmem] (+)= A[tmem] * B[smem desc]
 __device__ __forceinline__ void mma_ts_warp(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
                                             uint32_t accumulate) {
   asm volatile(

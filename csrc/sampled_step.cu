@@ -18,9 +18,9 @@
 // entities are chained, so a chain has a Poisson length; the positives' entities, whose degrees are heavy-tailed, and
 // candidates given by the caller go through red.add into the gradient table and a flag per row.
 //
-// Measured against the launch sequence lookup / score / backward / sweeps (one triple per query, scalar atomics): 10 000
-// positives x 11, D = 128, 123 182 rows, 37 relations 640 -> 128 us; 1024 x 100 given candidates, D = 256, 14 541 rows
-// 131 -> 85 us; 32 768 x 129, D = 128, 5 million rows, sparse 5207 -> 2530 us (the update of 2.9 million rows moves 8.7 GB
+// Measured against the launch sequence lookup / score / backward / sweeps (one triple per query, scalar atomics), whole step:
+// 10 000 positives x 11, D = 128, 123 182 rows, 37 relations 655 -> 123 us; 1024 x 100 given candidates, D = 256, 14 541 rows
+// 132 -> 74 us; 32 768 x 129, D = 128, 5 million rows, sparse 5280 -> 2730 us (the update of 2.9 million rows moves 8.7 GB
 // in 1.9 ms).
 #include "algebra.cuh"
 #include "dice_b200.h"
@@ -258,7 +258,9 @@ __device__ __forceinline__ float transpose_sum(float (&a)[CH], int lane) {
 
 constexpr int GRAD_THREADS = 256;
 // Candidate rows in flight (of up to 128 floats) and resident blocks per SM.  Measured (4, 4) / (8, 2): 32 768 x 129 on 5
-// million rows, D = 128: 609 / 660 us, 10 000 x 11: 30 / 39 us.
+// million rows, D = 128: 609 / 660 us, 10 000 x 11: 30 / 39 us.  Measured at D = 128 only: four blocks leave 64 registers, at
+// which most widths spill (116 to 144 bytes of stores per thread at D = 128, 320 to 400 at 256, up to 830 at 512), and two
+// blocks would leave room for all but the widest.
 constexpr int GRAD_CH = 4;
 constexpr int GRAD_B = 4;
 
