@@ -275,13 +275,14 @@ class ExternalQueryEngine:
         if len(self._graphs) >= self.MAX_GRAPHS:
             torch.cuda.synchronize(self.device)      # no replay is under way when its memory is given back
             self._graphs.popitem(last=False)
-        graph = torch.cuda.CUDAGraph()
+        graph, pool, stream = torch.cuda.CUDAGraph(), torch.cuda.graph_pool_handle(), torch.cuda.current_stream(self.device)
         try:
-            with torch.cuda.graph(graph, capture_error_mode="thread_local"):
+            with torch.cuda.graph(graph, pool=pool, capture_error_mode="thread_local"):
                 loss = self._step(b.x_in, b.dp)
         except RuntimeError as err:
             # the step cannot be captured, or there is no memory for a graph's own pool (nothing has run): plain launches from
             # here on, which raise what is wrong with the step itself
+            self._leave_failed_capture(pool, stream)
             logging.getLogger(__name__).warning("training step runs as plain launches, its capture failed: %s", err)
             self.use_graph = False
             self._graphs.clear()
@@ -289,6 +290,18 @@ class ExternalQueryEngine:
         grads = [(p, p.grad) for p in self.model.parameters() if p.grad is not None]
         self._graphs[key] = (graph, loss, grads)
         return self._graphs[key]
+
+    def _leave_failed_capture(self, pool, stream) -> None:
+        """What the end of a capture does and an invalidated one leaves undone: the caller's stream is current again, the
+        allocator no longer waits for the capture's end, and the random generator (whose mark only the end of a whole capture
+        takes off) gives numbers outside of captures."""
+        torch.cuda.set_stream(stream)
+        try:
+            torch._C._cuda_endAllocateToPool(self.device.index, pool)
+        except RuntimeError:
+            pass        # it was ended
+        with torch.cuda.graph(torch.cuda.CUDAGraph(), capture_error_mode="thread_local"):
+            self.loss_acc.add_(0.0)     # recorded, never run
 
     def _step(self, x: torch.Tensor, dp: torch.Tensor) -> torch.Tensor:
         m = self.model

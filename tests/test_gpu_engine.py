@@ -348,14 +348,32 @@ def test_replay_follows_a_learning_rate_schedule():
 
 
 def test_a_failed_capture_is_reported_and_the_step_goes_on(caplog):
+    """The process is as it was before: the caller's stream is current, random numbers (here of a dropout) can be drawn and follow
+    the seed, memory can be had and given back, and another engine captures and replays its steps."""
     eng, batch = _small_engine()
     eng.step(batch)
     forward = eng.model.fc1.forward
+    eng.model.input_dp_ent_real.p = 0.3
 
     def waits(x):
-        float(x.sum())                                  # a copy to the host: not allowed in a capture
+        float(x.detach().sum())                         # a copy to the host: not allowed in a capture
         return forward(x)
     eng.model.fc1.forward = waits
+    stream = torch.cuda.current_stream()
     for _ in range(4):
         assert torch.isfinite(eng.step(batch))
+        assert torch.cuda.current_stream() == stream
     assert not eng._graphs and not eng.use_graph and sum("capture failed" in r.message for r in caplog.records) == 1
+    draws = []
+    for _ in range(2):
+        torch.manual_seed(5)
+        draws.append(torch.rand(1000, device=DEV))
+    assert torch.equal(*draws) and 0.4 < float(draws[0].mean()) < 0.6
+    del draws
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    other, batch = _small_engine()
+    other.model.input_dp_ent_real.p = 0.3
+    other.optimizer_view().param_groups[0]["lr"] = 0.0      # the same weights throughout: only the dropout differs
+    losses = [float(other.step(batch)) for _ in range(5)]
+    assert len(other._graphs) == 1 and len(set(losses)) == 5 and all(x == x for x in losses)
