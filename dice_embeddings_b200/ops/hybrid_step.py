@@ -283,7 +283,9 @@ class ExternalQueryEngine:
             # the step cannot be captured, or there is no memory for a graph's own pool (nothing has run): plain launches from
             # here on, which raise what is wrong with the step itself
             self._leave_failed_capture(pool, stream)
-            logging.getLogger(__name__).warning("training step runs as plain launches, its capture failed: %s", err)
+            # the text alone: the exception holds the frames of the step, and they its tensors
+            logging.getLogger(__name__).warning("training step runs as plain launches, its capture failed: %s",
+                                                (str(err) or type(err).__name__).splitlines()[0])
             self.use_graph = False
             self._graphs.clear()
             return None
@@ -297,7 +299,7 @@ class ExternalQueryEngine:
         takes off) gives numbers outside of captures."""
         torch.cuda.set_stream(stream)
         try:
-            torch._C._cuda_endAllocateToPool(self.device.index, pool)
+            torch._C._cuda_endAllocateToPool(self.E.device.index, pool)
         except RuntimeError:
             pass        # it was ended
         with torch.cuda.graph(torch.cuda.CUDAGraph(), capture_error_mode="thread_local"):
